@@ -62,3 +62,29 @@ def test_activation_view_with_row_stride(wrk, ctx):
     want = np.zeros((N, M), dtype=np.float32)
     oracle.matmul(okind, om, oscale, np.ascontiguousarray(x3[2]), want, mode=1)
     assert_close(y.numpy().reshape(N, M), want, "z-slice input")
+
+
+@pytest.mark.parametrize("kind", KINDS)
+@pytest.mark.parametrize("k,m,n", [(128, 128, 9), (384, 200, 15), (2688, 768, 33), (8064, 100, 17), (1152, 130, 250), (640, 129, 512)])
+def test_odd_numbers_of_k_blocks_and_few_tokens(wrk, ctx, kind, k, m, n):
+    # 1, 3, 21, 63, 9, 5 blocks of 128: the two dequantizing groups get unequal shares, K splits into unequal parts (4 CTAs of
+    # 5 or 6 blocks, 8 of 7 or 8), fewer blocks than ring stages; 9 tokens are the fewest the kernel takes
+    got, want = _run(wrk, ctx, kind, k, m, n, turbo=True, seed=k + n)
+    assert_close(got, want, f"{kind} {k}x{m} n={n}")
+    assert ctx.device_status() == 0
+
+
+def test_a_matmul_waits_for_the_op_that_writes_its_weights(wrk, ctx):
+    # in a list a matmul starts before the ops in front of it have finished and fetches its weights at once, unless one of
+    # them writes the weights: here the matrix is copied into place by the list itself
+    rng = np.random.default_rng(13)
+    K, M, N = 4096, 2048, 64
+    w = (rng.standard_normal((M, K), dtype=np.float32) * 0.02).astype(np.float16)
+    x = rng.standard_normal((N, K), dtype=np.float32).astype(np.float16)
+    source, matrix, t_x = ctx.from_numpy(w), ctx.tensor(wrk.F16, [K, M], zeros=True), ctx.from_numpy(x)
+    y = ctx.tensor(wrk.F32, [M, N])
+    ops = wrk.op_list([wrk.blit(source, matrix), wrk.Matrix.fp16(matrix).matmul_op(t_x, y, turbo=True)])
+    for graph in (False, True):
+        matrix.load(np.zeros((M, K), dtype=np.float16))
+        ctx.encode(ops, use_graph=graph).submit()
+        assert_close(y.numpy().reshape(N, M), x.astype(np.float32) @ w.astype(np.float32).T, f"graph={graph}")

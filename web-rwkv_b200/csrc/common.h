@@ -121,12 +121,14 @@ struct wrk_op {
     wrk::Launch launch;                              // Atom
     uint32_t num_kernels = 1;                        // kernels one launch() issues
     std::vector<std::shared_ptr<wrk::Buffer>> keep;  // buffers the atom touches
+    std::vector<const wrk::Buffer*> early;           // of those: read before the kernels in front of it have finished (weights)
     std::vector<wrk_op*> children;                   // List (retained)
     ~wrk_op();
 };
 
 struct wrk_commands {
     std::vector<wrk_op*> atoms;  // retained, in order
+    std::vector<char> chained;   // per atom: launched as a programmatic dependent of the one before it
     uint64_t num_kernels = 0;
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;

@@ -4,9 +4,12 @@
 // `Context::encode` (src/tensor/ops.rs:78-144) of the reference: one CUDA stream per context,
 // device buffers from cudaMallocAsync's pool, pinned staging buffers for uploads and read-backs,
 // and command lists that can be replayed as CUDA graphs.
+#include <algorithm>
 #include <cstring>
+#include <unordered_set>
 
 #include "common.h"
+#include "kernels/kernels.h"
 
 namespace wrk {
 
@@ -21,6 +24,13 @@ int32_t set_error(int32_t code, const char* fmt, ...) {
     g_last_error = buf;
     return code;
 }
+
+namespace k {
+static thread_local bool tl_chained = false;
+bool chained_launches() { return tl_chained; }
+ChainedLaunches::ChainedLaunches(bool on) : before(tl_chained) { tl_chained = on; }
+ChainedLaunches::~ChainedLaunches() { tl_chained = before; }
+}  // namespace k
 
 // Tears the context down when its last reference (owner or buffer) goes.
 static void context_unref(wrk_context* ctx) {
@@ -460,11 +470,28 @@ int32_t wrk_op_num_atoms(const wrk_op* op, uint64_t* count) {
     return WRK_OK;
 }
 
-static int32_t launch_all(wrk_context* ctx, const std::vector<wrk_op*>& atoms, cudaStream_t stream) {
-    for (auto a : atoms) {
-        cudaError_t e = a->launch(stream);
+// Which atoms of a list may be launched while the one before them still runs.  Every kernel waits for its predecessors
+// before it touches what they wrote, except that a matmul fetches its first weights (`early`) at once: an atom is chained
+// unless an earlier atom of the list touches one of its weights other than as a weight.  The first atom is not: what
+// precedes it on the stream is not known here.
+static std::vector<char> chain_of(const std::vector<wrk_op*>& atoms) {
+    std::vector<char> chained(atoms.size(), 0);
+    std::unordered_set<const Buffer*> touched;
+    for (size_t i = 0; i < atoms.size(); ++i) {
+        const auto& early = atoms[i]->early;
+        chained[i] = i > 0 && std::none_of(early.begin(), early.end(), [&](const Buffer* b) { return touched.count(b) != 0; });
+        for (const auto& b : atoms[i]->keep)
+            if (std::find(early.begin(), early.end(), b.get()) == early.end()) touched.insert(b.get());
+    }
+    return chained;
+}
+
+static int32_t launch_all(wrk_context* ctx, const std::vector<wrk_op*>& atoms, const std::vector<char>& chained, cudaStream_t stream) {
+    for (size_t i = 0; i < atoms.size(); ++i) {
+        const k::ChainedLaunches scope(chained[i] != 0);
+        cudaError_t e = atoms[i]->launch(stream);
         if (e != cudaSuccess)
-            return set_error(WRK_ERR_CUDA, "launch of %s failed: %s", a->name.c_str(), cudaGetErrorString(e));
+            return set_error(WRK_ERR_CUDA, "launch of %s failed: %s", atoms[i]->name.c_str(), cudaGetErrorString(e));
     }
     return WRK_OK;
 }
@@ -477,6 +504,7 @@ int32_t wrk_encode(wrk_context* ctx, wrk_op* op, int32_t use_graph, wrk_commands
         a->refs.fetch_add(1);
         cmd->num_kernels += a->num_kernels;
     }
+    cmd->chained = chain_of(cmd->atoms);
     if (use_graph && !cmd->atoms.empty()) {
         std::lock_guard<std::mutex> lock(ctx->mutex);
         cudaSetDevice(ctx->device);
@@ -485,7 +513,7 @@ int32_t wrk_encode(wrk_context* ctx, wrk_op* op, int32_t use_graph, wrk_commands
             delete cmd;
             return set_error(WRK_ERR_CUDA, "cudaStreamBeginCapture failed: %s", cudaGetErrorString(e));
         }
-        int32_t s = launch_all(ctx, cmd->atoms, ctx->stream);
+        int32_t s = launch_all(ctx, cmd->atoms, cmd->chained, ctx->stream);
         e = cudaStreamEndCapture(ctx->stream, &cmd->graph);
         if (s != WRK_OK || e != cudaSuccess) {
             delete cmd;
@@ -508,7 +536,7 @@ int32_t wrk_submit(wrk_context* ctx, wrk_commands* commands) {
     if (commands->exec) {
         WRK_CUDA(cudaGraphLaunch(commands->exec, ctx->stream));
     } else {
-        WRK_TRY(launch_all(ctx, commands->atoms, ctx->stream));
+        WRK_TRY(launch_all(ctx, commands->atoms, commands->chained, ctx->stream));
     }
     ctx->launches.fetch_add(commands->num_kernels);
     return WRK_OK;
@@ -524,7 +552,7 @@ int32_t wrk_run(wrk_context* ctx, wrk_op* op) {
     WRK_CUDA(cudaSetDevice(ctx->device));
     std::vector<wrk_op*> atoms;
     flatten(op, atoms);
-    WRK_TRY(launch_all(ctx, atoms, ctx->stream));
+    WRK_TRY(launch_all(ctx, atoms, chain_of(atoms), ctx->stream));
     uint64_t n = 0;
     for (auto a : atoms) n += a->num_kernels;
     ctx->launches.fetch_add(n);

@@ -21,6 +21,7 @@
 // accumulate, Int8 affine term through per-block activation sums).  Every tensor the reference stores as
 // fp16 is rounded to fp16 here at the same point.
 #include "gemv_device.cuh"
+#include "launch.cuh"
 
 #include <mutex>
 
@@ -436,21 +437,6 @@ __global__ void __launch_bounds__(4 * S) wkv56_fused_kernel(const Wkv6Args a) {
     for (int i = 0; i < SI; ++i) static_cast<float*>(a.state.base)[a.state.index(c, 1 + q * SI + i, slot)] = st[i];
 }
 
-template <typename Kernel, typename Args>
-cudaError_t launch_pdl(Kernel kernel, dim3 grid, dim3 block, size_t smem, cudaStream_t stream, const Args& args) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = grid;
-    cfg.blockDim = block;
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, kernel, args);
-}
-
 }  // namespace
 
 // Cuts the concatenated rows of the launch's matrices into one contiguous range per CTA, balanced by
@@ -583,23 +569,21 @@ size_t fused_gemv_prepare(FusedGemvArgs& a) {
 }
 
 template <int PRO, int EPI>
-cudaError_t launch_fused_gemv(const FusedGemvArgs& a, int grid, size_t smem, cudaStream_t stream, bool pdl) {
+cudaError_t launch_fused_gemv(const FusedGemvArgs& a, int grid, size_t smem, cudaStream_t stream) {
     static SmemOptIn opt_in;  // one per instantiation
     if (cudaError_t e = opt_in.ensure(fused_gemv_kernel<PRO, EPI>, 200 * 1024); e != cudaSuccess) return e;
-    if (pdl) return launch_pdl(fused_gemv_kernel<PRO, EPI>, dim3(grid), dim3(kThreads), smem, stream, a);
-    fused_gemv_kernel<PRO, EPI><<<grid, kThreads, smem, stream>>>(a);
-    return cudaGetLastError();
+    return launch(fused_gemv_kernel<PRO, EPI>, dim3(grid), dim3(kThreads), smem, stream, a);
 }
 
-cudaError_t dispatch_fused_gemv(const FusedGemvArgs& a, int grid, size_t smem, cudaStream_t stream, bool pdl) {
+cudaError_t dispatch_fused_gemv(const FusedGemvArgs& a, int grid, size_t smem, cudaStream_t stream) {
     if (a.prologue == PRO_NONE) {
-        if (a.epilogue == EPI_STORE) return launch_fused_gemv<PRO_NONE, EPI_STORE>(a, grid, smem, stream, pdl);
-        if (a.epilogue == EPI_RESIDUAL) return launch_fused_gemv<PRO_NONE, EPI_RESIDUAL>(a, grid, smem, stream, pdl);
-        if (a.epilogue == EPI_CHANNEL_MIX) return launch_fused_gemv<PRO_NONE, EPI_CHANNEL_MIX>(a, grid, smem, stream, pdl);
+        if (a.epilogue == EPI_STORE) return launch_fused_gemv<PRO_NONE, EPI_STORE>(a, grid, smem, stream);
+        if (a.epilogue == EPI_RESIDUAL) return launch_fused_gemv<PRO_NONE, EPI_RESIDUAL>(a, grid, smem, stream);
+        if (a.epilogue == EPI_CHANNEL_MIX) return launch_fused_gemv<PRO_NONE, EPI_CHANNEL_MIX>(a, grid, smem, stream);
     } else if (a.epilogue == EPI_STORE) {
-        if (a.prologue == PRO_LN) return launch_fused_gemv<PRO_LN, EPI_STORE>(a, grid, smem, stream, pdl);
-        if (a.prologue == PRO_LN_SHIFT1) return launch_fused_gemv<PRO_LN_SHIFT1, EPI_STORE>(a, grid, smem, stream, pdl);
-        if (a.prologue == PRO_LN_SHIFT2) return launch_fused_gemv<PRO_LN_SHIFT2, EPI_STORE>(a, grid, smem, stream, pdl);
+        if (a.prologue == PRO_LN) return launch_fused_gemv<PRO_LN, EPI_STORE>(a, grid, smem, stream);
+        if (a.prologue == PRO_LN_SHIFT1) return launch_fused_gemv<PRO_LN_SHIFT1, EPI_STORE>(a, grid, smem, stream);
+        if (a.prologue == PRO_LN_SHIFT2) return launch_fused_gemv<PRO_LN_SHIFT2, EPI_STORE>(a, grid, smem, stream);
     }
     return cudaErrorInvalidValue;  // a prologue with a residual epilogue is not instantiated
 }
@@ -609,17 +593,17 @@ cudaError_t dispatch_fused_gemv(const FusedGemvArgs& a, int grid, size_t smem, c
 cudaError_t fused_gemv(const FusedGemvArgs& a_in, int grid, cudaStream_t stream) {
     FusedGemvArgs a = a_in;
     const size_t smem = fused_gemv_prepare(a);
-    return dispatch_fused_gemv(a, grid, smem, stream, true);
+    return dispatch_fused_gemv(a, grid, smem, stream);
 }
 
 cudaError_t tmix_shift_v6(const TmixArgs& a, cudaStream_t stream) {
     const uint32_t threads = 5 * a.C;
     const size_t smem = (size_t)a.T * 5 * a.D * sizeof(__half);
-    return launch_pdl(tmix_shift_kernel, dim3((threads + 255) / 256), dim3(256), smem, stream, a);
+    return launch(tmix_shift_kernel, dim3((threads + 255) / 256), dim3(256), smem, stream, a);
 }
 
 cudaError_t wkv56_fused(const Wkv6Args& a, cudaStream_t stream) {
-    return launch_pdl(wkv56_fused_kernel<64>, dim3(a.H, a.B), dim3(256), 0, stream, a);
+    return launch(wkv56_fused_kernel<64>, dim3(a.H, a.B), dim3(256), 0, stream, a);
 }
 
 // ---- Int8 GEMV with its row-range table in static device memory -------------------------------------
@@ -715,8 +699,9 @@ int gemv_int8_static(int device, cudaStream_t stream, const uint8_t* w, const __
     const size_t smem = fused_gemv_prepare(a);
     static_partition_kernel<<<1, 32, 0, stream>>>(su.table, K, M, grid);
     if ((*cuda_error = cudaGetLastError()) != cudaSuccess) return SG_CUDA;
-    // a plain launch: the multiply reads the table at once, so it must not start before the fill kernel ends
-    if ((*cuda_error = dispatch_fused_gemv(a, grid, smem, stream, false)) != cudaSuccess) return SG_CUDA;
+    // not chained: the multiply reads the table at once, so it must not start before the fill kernel ends
+    const ChainedLaunches plain(false);
+    if ((*cuda_error = dispatch_fused_gemv(a, grid, smem, stream)) != cudaSuccess) return SG_CUDA;
     return SG_OK;
 }
 

@@ -9,6 +9,7 @@
 // blit.wgsl, channel_mix.wgsl / channel_mix_v7.wgsl, layer_norm.wgsl (src/tensor/ops.rs:1393-1462, 1656-1795, 1566-1650,
 // 2015-2060, 407-470).
 #include "device.cuh"
+#include "launch.cuh"
 
 namespace wrk {
 namespace k {
@@ -78,6 +79,8 @@ bool fits32(size_t elements) { return elements / 8 < 0x7fffffffull; }
 template <typename In, typename Out>
 __global__ void binary_vec_kernel(int is_mul, const In* in, Out* out, uint32_t c8, uint32_t total8, int in_row, uint32_t plane8,
                                   int act_x, int act_y, int act_out) {
+    pdl_launch_dependents();
+    pdl_wait();
     for (uint32_t o = blockIdx.x * blockDim.x + threadIdx.x; o < total8; o += gridDim.x * blockDim.x) {
         float x[8], y[8];
         load8(in + (size_t)(in_row ? (plane8 ? o / plane8 * c8 : 0u) + o % c8 : o) * 8, x);
@@ -103,14 +106,15 @@ bool binary_typed(int is_mul, const DView& input, const DView& output, int act_x
     const size_t total = (size_t)output.shape[0] * output.shape[1] * output.shape[2];
     if (!fits32(total)) return false;
     const uint32_t c8 = output.shape[0] / 8;
-    binary_vec_kernel<In, Out><<<vec_grid(total / 8), kVecThreads, 0, stream>>>(
-        is_mul, in, out, c8, (uint32_t)(total / 8), same ? 0 : 1, same || row ? 0u : c8 * output.shape[1], act_x, act_y, act_out);
+    launch(binary_vec_kernel<In, Out>, dim3(vec_grid(total / 8)), dim3(kVecThreads), 0, stream, is_mul, in, out, c8, (uint32_t)(total / 8), same ? 0 : 1, same || row ? 0u : c8 * output.shape[1], act_x, act_y, act_out);
     return true;
 }
 
 // ---- activation.wgsl ---------------------------------------------------------------------------------------------------
 template <typename T>
 __global__ void activate_vec_kernel(T* x, uint32_t total8, int act) {
+    pdl_launch_dependents();
+    pdl_wait();
     for (uint32_t o = blockIdx.x * blockDim.x + threadIdx.x; o < total8; o += gridDim.x * blockDim.x) {
         float v[8];
         load8(x + (size_t)o * 8, v);
@@ -123,6 +127,8 @@ __global__ void activate_vec_kernel(T* x, uint32_t total8, int act) {
 // ---- blit.wgsl without a transpose (the data types may differ) --------------------------------------------------
 template <typename In, typename Out>
 __global__ void blit_vec_kernel(const In* in, Out* out, uint32_t total8) {
+    pdl_launch_dependents();
+    pdl_wait();
     for (uint32_t o = blockIdx.x * blockDim.x + threadIdx.x; o < total8; o += gridDim.x * blockDim.x) {
         float v[8];
         load8(in + (size_t)o * 8, v);
@@ -137,7 +143,7 @@ bool blit_typed(const DView& input, const DView& output, cudaStream_t stream) {
     if (!dense_as<In>(input, &in) || !dense_as<Out>(output, &out)) return false;
     const size_t total = (size_t)input.shape[0] * input.shape[1] * input.shape[2];
     if (!fits32(total)) return false;
-    blit_vec_kernel<In, Out><<<vec_grid(total / 8), kVecThreads, 0, stream>>>(in, out, (uint32_t)(total / 8));
+    launch(blit_vec_kernel<In, Out>, dim3(vec_grid(total / 8)), dim3(kVecThreads), 0, stream, in, out, (uint32_t)(total / 8));
     return true;
 }
 
@@ -156,6 +162,8 @@ struct ShiftVecArgs {
 };
 
 __global__ void token_shift_vec_kernel(const ShiftVecArgs a) {
+    pdl_launch_dependents();
+    pdl_wait();
     const uint32_t total8 = a.c8 * a.T;
     for (uint32_t o = blockIdx.x * blockDim.x + threadIdx.x; o < total8; o += gridDim.x * blockDim.x) {
         const uint32_t c = (o % a.c8) * 8, t = o / a.c8;
@@ -191,6 +199,8 @@ __global__ void token_shift_vec_kernel(const ShiftVecArgs a) {
 template <typename T>
 __global__ void channel_mix_vec_kernel(const uint32_t* cursors, int wide, DView state, const T* r, const T* v, T* x, T* xres,
                                        uint32_t c8, uint32_t total8, int v7) {
+    pdl_launch_dependents();
+    pdl_wait();
     for (uint32_t o = blockIdx.x * blockDim.x + threadIdx.x; o < total8; o += gridDim.x * blockDim.x) {
         const uint32_t c = (o % c8) * 8, t = o / c8;
         const CursorD cu = cursor_at(cursors, wide, t);
@@ -251,6 +261,8 @@ __device__ __forceinline__ void norm_store(const __half* w, const __half* b, siz
 template <typename T>
 __global__ void layer_norm_rows_kernel(const __half* w, const __half* b, const T* delta, T* src, T* x, uint32_t C, uint32_t rows,
                                        uint32_t wrows, float eps, const __half* gate, __half* gated, int gate_act) {
+    pdl_launch_dependents();
+    pdl_wait();
     const uint32_t lanes = C / 8;
     const uint32_t per_block = blockDim.x / lanes;
     for (uint32_t row0 = blockIdx.x * per_block; row0 < rows; row0 += gridDim.x * per_block) {  // uniform trip count per warp
@@ -287,6 +299,8 @@ constexpr int kNormIters = 4;
 template <typename T>
 __global__ void __launch_bounds__(256) layer_norm_wide_kernel(const __half* w, const __half* b, const T* delta, T* src, T* x,
                                                               uint32_t C, uint32_t rows, uint32_t wrows, float eps) {
+    pdl_launch_dependents();
+    pdl_wait();
     __shared__ float scratch[2][8];
     const uint32_t c8 = C / 8, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     auto block_total = [&](float s, int which) {
@@ -340,12 +354,11 @@ bool layer_norm_typed(const __half* w, const __half* b, const void* delta, void*
     const uint32_t lanes = C / 8;
     if (C <= 256 && (lanes & (lanes - 1)) == 0) {
         const uint32_t per_block = 256 / lanes, blocks = (rows + per_block - 1) / per_block;
-        layer_norm_rows_kernel<T><<<blocks < 148u * 16u ? blocks : 148u * 16u, 256, 0, stream>>>(w, b, dp, sp, xp, C, rows, wrows, eps,
-                                                                                                   nullptr, nullptr, 0);
+        launch(layer_norm_rows_kernel<T>, dim3(blocks < 148u * 16u ? blocks : 148u * 16u), dim3(256), 0, stream, w, b, dp, sp, xp, C, rows, wrows, eps, nullptr, nullptr, 0);
         return true;
     }
     if (lanes <= (uint32_t)kNormIters * 256) {
-        layer_norm_wide_kernel<T><<<rows < 148u * 8u ? rows : 148u * 8u, 256, 0, stream>>>(w, b, dp, sp, xp, C, rows, wrows, eps);
+        launch(layer_norm_wide_kernel<T>, dim3(rows < 148u * 8u ? rows : 148u * 8u), dim3(256), 0, stream, w, b, dp, sp, xp, C, rows, wrows, eps);
         return true;
     }
     return false;
@@ -366,11 +379,9 @@ cudaError_t group_norm_gate(const __half* w, const __half* b, int dtype, void* x
     const uint32_t per_block = 256 / (C / 8), blocks = (rows + per_block - 1) / per_block;
     const uint32_t grid = blocks < 148u * 16u ? blocks : 148u * 16u;
     if (dtype == WRK_F16)
-        layer_norm_rows_kernel<__half><<<grid, 256, 0, stream>>>(w, b, nullptr, static_cast<__half*>(x), static_cast<__half*>(x), C, rows,
-                                                                 wrows, eps, gate, out, gate_act);
+        launch(layer_norm_rows_kernel<__half>, grid, dim3(256), 0, stream, w, b, nullptr, static_cast<__half*>(x), static_cast<__half*>(x), C, rows, wrows, eps, gate, out, gate_act);
     else
-        layer_norm_rows_kernel<float><<<grid, 256, 0, stream>>>(w, b, nullptr, static_cast<float*>(x), static_cast<float*>(x), C, rows,
-                                                                wrows, eps, gate, out, gate_act);
+        launch(layer_norm_rows_kernel<float>, grid, dim3(256), 0, stream, w, b, nullptr, static_cast<float*>(x), static_cast<float*>(x), C, rows, wrows, eps, gate, out, gate_act);
     return cudaGetLastError();
 }
 
@@ -397,11 +408,11 @@ bool activate_vec(const DView& x, int act, cudaStream_t stream) {
     __half* h;
     float* f;
     if (dense_as<__half>(x, &h)) {
-        activate_vec_kernel<__half><<<vec_grid(total / 8), kVecThreads, 0, stream>>>(h, (uint32_t)(total / 8), act);
+        launch(activate_vec_kernel<__half>, dim3(vec_grid(total / 8)), dim3(kVecThreads), 0, stream, h, (uint32_t)(total / 8), act);
         return true;
     }
     if (dense_as<float>(x, &f)) {
-        activate_vec_kernel<float><<<vec_grid(total / 8), kVecThreads, 0, stream>>>(f, (uint32_t)(total / 8), act);
+        launch(activate_vec_kernel<float>, dim3(vec_grid(total / 8)), dim3(kVecThreads), 0, stream, f, (uint32_t)(total / 8), act);
         return true;
     }
     return false;
@@ -459,7 +470,7 @@ bool token_shift_vec(const uint32_t* cursors, int wide, const DView& time_mix, c
                      const DView& input, const DView& output, int reversed, cudaStream_t stream) {
     ShiftVecArgs a;
     if (!shift_vec_args(cursors, wide, time_mix, bias, state, input, output, reversed, &a)) return false;
-    token_shift_vec_kernel<<<vec_grid((size_t)a.c8 * a.T), kVecThreads, 0, stream>>>(a);
+    launch(token_shift_vec_kernel, dim3(vec_grid((size_t)a.c8 * a.T)), dim3(kVecThreads), 0, stream, a);
     return true;
 }
 
@@ -480,7 +491,7 @@ bool token_shift_multi_vec(const ShiftMultiArgs& m, cudaStream_t stream) {
         a.mix[i] = m.mix[i];
         a.out[i] = m.out[i];
     }
-    token_shift_vec_kernel<<<vec_grid((size_t)a.c8 * m.T), kVecThreads, 0, stream>>>(a);
+    launch(token_shift_vec_kernel, dim3(vec_grid((size_t)a.c8 * m.T)), dim3(kVecThreads), 0, stream, a);
     return true;
 }
 
@@ -490,13 +501,9 @@ bool channel_mix_vec(const uint32_t* cursors, int wide, const DView& state, int 
         return false;
     const uint32_t total8 = C / 8 * T;
     if (dtype == WRK_F16)
-        channel_mix_vec_kernel<__half><<<vec_grid(total8), kVecThreads, 0, stream>>>(
-            cursors, wide, state, static_cast<const __half*>(r), static_cast<const __half*>(v), static_cast<__half*>(x),
-            static_cast<__half*>(xres), C / 8, total8, v7);
+        launch(channel_mix_vec_kernel<__half>, dim3(vec_grid(total8)), dim3(kVecThreads), 0, stream, cursors, wide, state, static_cast<const __half*>(r), static_cast<const __half*>(v), static_cast<__half*>(x), static_cast<__half*>(xres), C / 8, total8, v7);
     else
-        channel_mix_vec_kernel<float><<<vec_grid(total8), kVecThreads, 0, stream>>>(
-            cursors, wide, state, static_cast<const float*>(r), static_cast<const float*>(v), static_cast<float*>(x),
-            static_cast<float*>(xres), C / 8, total8, v7);
+        launch(channel_mix_vec_kernel<float>, dim3(vec_grid(total8)), dim3(kVecThreads), 0, stream, cursors, wide, state, static_cast<const float*>(r), static_cast<const float*>(v), static_cast<float*>(x), static_cast<float*>(xres), C / 8, total8, v7);
     return true;
 }
 

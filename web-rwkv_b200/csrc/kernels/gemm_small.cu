@@ -14,6 +14,7 @@
 #include <algorithm>
 
 #include "device.cuh"
+#include "launch.cuh"
 #include "kernels.h"
 
 namespace wrk {
@@ -37,6 +38,8 @@ __device__ __forceinline__ void mma16816(float c[4], const uint32_t a[4], const 
 }
 
 __global__ void __launch_bounds__(kSmallThreads) matmul_small_kernel(const SmallParams p) {
+    pdl_launch_dependents();
+    pdl_wait();
     __shared__ __align__(16) __half sw[kTileM][kChunk + kPad];
     __shared__ __align__(16) __half sx[kTileN][kChunk + kPad];
     const uint32_t m0 = blockIdx.x * kTileM, n0 = blockIdx.y * kTileN;
@@ -130,7 +133,7 @@ cudaError_t matmul_small(const MatmulArgs& a, int num_sms, cudaStream_t stream) 
     p.act = a.act;
     (void)num_sms;
     dim3 grid((a.M + kTileM - 1) / kTileM, (a.N + kTileN - 1) / kTileN, a.B);
-    matmul_small_kernel<<<grid, kSmallThreads, 0, stream>>>(p);
+    launch(matmul_small_kernel, grid, dim3(kSmallThreads), 0, stream, p);
     return cudaGetLastError();
 }
 

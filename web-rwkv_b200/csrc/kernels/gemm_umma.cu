@@ -1,37 +1,41 @@
-// Tensor-memory GEMM for the prefill / batched path (matmul_mat_fp16 / int8 / nf4 with 16 or more tokens):
+// Tensor-memory GEMM for the prefill / batched path (matmul_mat_fp16 / int8 / nf4 with more than 8 tokens):
 // out[n][m] = act(sum_k W[m][k] * x[n][k]).
 //
 // One CTA owns a 128-row slice of W and up to 256 tokens and walks K in steps of 64.  Warp roles:
-//   * warp 9 (one lane) streams the packed weight tiles with TMA (cp.async.bulk.tensor.2d): 128 rows x 64
-//     (Int8) or 32 (NF4) bytes per step into a ring of raw stages several steps ahead of their use; fp16
-//     weights go straight into the A operand stage through a 128-byte-swizzled tensor map;
-//   * warp 10 (one lane) streams the fp16 activations of the step, [tokens x 64] through a 128-byte-swizzled
-//     tensor map, into the B operand stage (rows past the last token are zero-filled by the TMA unit);
-//   * warps 0-7 dequantize as two groups of four warps on alternate pairs of steps: a thread turns the 64
-//     weights of one row and step into fp16 (f32 math, one rounding) and stores them in the K-major
-//     128-byte-swizzled layout tcgen05 reads; the (min, max) / absmax values of the next 256 columns are
-//     fetched with cp.async while the current ones are in use;
-//   * warp 8 (one lane) issues tcgen05.mma.cta_group::1.kind::f16 (M = 128, N = token tile, K = 16, four per
-//     step) into a TMEM accumulator of 128 lanes x N fp32 columns and releases the stage with tcgen05.commit;
-//   * after the last step warps 0-7 read the accumulator back with tcgen05.ld (warp w reads lanes
-//     32 (w % 4) ..), apply the activation and put the tile, in the output's type, into shared memory (the operand
-//     stages are free by then), from where it goes to global memory in 16-byte pieces: the 128 rows of a token are
-//     adjacent elements of the output.
+//   * warp 9 (one thread) streams the packed weight tiles with TMA: 128 rows x 128 (Int8) or 64 (NF4) bytes per pair of
+//     steps into a swizzled ring of raw stages; fp16 weights go straight into the A operand stage;
+//   * warp 10 (one thread) streams the fp16 activations, [steps][tokens][64] per copy, into the B operand stages (rows
+//     past the last token are zero-filled by the TMA unit);
+//   * warps 0-7 dequantize as two groups of four warps on alternate pairs of steps: a thread owns a row of the tile, turns
+//     its 64 weights of a step into fp16 (f32 math, one rounding) and stores them in TENSOR MEMORY, 32 columns per step:
+//     the A operand of the MMA, row m in lane m;
+//   * warp 8 (one thread) issues tcgen05.mma.cta_group::1.kind::f16 (M = 128, N = token tile, K = 16, four per step) into
+//     an accumulator of 128 lanes x N fp32 columns and releases the stages with tcgen05.commit;
+//   * after the last step warps 0-7 bring the accumulator to shared memory (the operand stages are free by then), and all
+//     warps write it out, four rows of a token per thread.
 // A launch takes up to four matrices of one format, K and token count (UmmaGroup): their row tiles share grid.x, so
 // key / value / receptance / gate of a layer fill the SMs together and none has to split K.
-// At 256 tokens the K walk is paced by the L2: every CTA re-reads the whole [tokens x K] activation tile next to its
-// own 128 rows of weights (40 KB per step and CTA; four 4096 x 4096 matrices at 256 tokens: 335 MB in 43 us, 7.7 TB/s),
-// which neither fewer dequantizing instructions (packed add.f32x2 / fma.rn.f32x2) nor a fourth operand stage change much.
 // Where the output tiles alone leave SMs idle, the CTAs of a thread-block cluster (up to 8, along grid.z) split the
-// K range of one tile: each writes its partial accumulator to its own shared memory and, after a cluster barrier,
-// adds its share of the columns over all peers through distributed shared memory.
+// K range of one tile; after a cluster barrier CTA r finishes its share of the columns, adding its peers' partial tiles
+// through distributed shared memory.
 // Weights enter the MMA as fp16(fma(q, (max - min) / 255, min)) resp. fp16(table[nib] * absmax), computed in
 // f32 and rounded once; the accumulation is fp32.  Every wait on an mbarrier is bounded: on a timeout the
 // kernel records WRK_ERR_TIMEOUT in the context's status word, stops waiting and still frees its TMEM.
+//
+// What bounds it: at 256 tokens a step is 512 cycles of MMA; it takes about 850, most of it shared-memory and L2 traffic of the
+// activation tile (32 KB per step and CTA).  At 64 tokens and below the dequantizers' instructions (about 250 cycles per
+// step) and the HBM stream of the weights are of one size, and a launch has about 5 us of fixed work.  An operand A that
+// went through shared memory cost 32 KB of its traffic per step and a proxy fence; what cost more was the issuing
+// threads: per step, divisions by ring sizes, parameters read again from memory, barrier answers waited for one after
+// the other and `lane == 0` branches around tensor-core instructions took 1100 cycles.  Measured with and without all of
+// these (us; Int8 unless noted): four 4096 x 4096 at 256 tokens 57 -> 35, 4096 x 14336 at 256 tokens 54 -> 34, 16384 x 4096
+// at 64 tokens 44 -> 23, 768 x 768 at 32 tokens 12 -> 5; NF4 four 2560 x 2560 at 256 tokens 47 -> 23; fp16 65536 x 2048 at
+// 16 tokens 71 -> 48 (5.6 TB/s), 14336 x 4096 at 1024 tokens 158 -> 139.
 #include <cuda.h>
 
 #include "device.cuh"
 #include "kernels.h"
+#include "launch.cuh"
 
 namespace wrk {
 namespace k {
@@ -39,42 +43,45 @@ namespace k {
 namespace {
 
 constexpr int BM = 128;             // weight rows per CTA (UMMA M)
-constexpr int BK = 64;              // K per stage: one 128-byte swizzle atom of fp16
+constexpr int BK = 64;              // K per step: one 128-byte swizzle atom of fp16 activations
 constexpr int kDequantWarps = 8;
 constexpr int kMmaWarp = 8, kWeightTmaWarp = 9;  // warp 10 streams the activations
 constexpr int kUmmaThreads = 11 * 32;
-constexpr int kMaxStages = 6;       // operand stages
+constexpr int kMaxStages = 8;       // operand stages
 constexpr int kMaxRaw = 8;          // raw weight stages
+constexpr uint32_t kScaleSlots = 8, kScaleAhead = 6;
+constexpr uint32_t SCALE_BYTES = 2 * kScaleSlots * BM * 4;  // two groups of dequantizing warps
 constexpr uint32_t kSpinLimit = 1u << 22;
-constexpr uint32_t A_STAGE_BYTES = BM * BK * 2;  // 16 KB
-constexpr uint32_t SCALE_SLOT_BYTES = BM * 8;    // 8 bytes of scales per row and 256 columns
-
-struct UmmaParams {
-    const uint8_t* w;
-    const __half* scale;
-    const float* table;
-    int kind;
-    uint32_t K, M, N;
-    DView out;
-    int act;
-    uint32_t n_tile;    // tokens per CTA: multiple of 16, <= 256
-    uint32_t tmem_cols; // power of two >= max(32, n_tile)
-    uint32_t stages;    // operand stages
-    uint32_t raw;       // raw weight stages (quantized kinds)
-    uint32_t splits;    // CTAs along K per output tile (grid.z = the cluster's size)
-    int32_t* status;
-};
+constexpr uint32_t A_STEP_BYTES = BM * BK * 2;  // fp16 weights: 16 KB of shared memory per step
+constexpr uint32_t A_STEP_COLS = BK / 2;        // quantized weights: 32 TMEM columns of fp16 pairs per step
 
 // Up to kMaxGroup problems of one weight format, K, token count and tiling in one launch: the row tiles of problem i
 // are CTAs tile_start[i] .. tile_start[i + 1] - 1 along grid.x.  Matrices that read different activations at the same
 // point of a layer (key / value / receptance / gate) fill the SMs together, where each alone would have to split K
 // and pay for the exchange of partial tiles.
 constexpr int kMaxGroup = 4;
+struct UmmaProblem {
+    const __half* scale;
+    const float* table;
+    uint32_t M;
+    int act;
+    DView out;
+};
 struct alignas(64) UmmaGroup {
     CUtensorMap map_w[kMaxGroup], map_x[kMaxGroup];
-    UmmaParams p[kMaxGroup];
+    UmmaProblem p[kMaxGroup];
     uint32_t tile_start[kMaxGroup + 1];
     uint32_t count;
+    uint32_t K, N;
+    uint32_t n_tile;     // tokens per CTA: multiple of 16, <= 256
+    uint32_t acc_cols;   // accumulator columns: n_tile rounded up to 32
+    uint32_t tmem_cols;  // power of two: the accumulator and, for quantized weights, the A stages
+    uint32_t bu;         // steps per stage of the activation operand (and of fp16 weights): 1 or 2
+    uint32_t a_stages;   // quantized weights: A stages in tensor memory, a pair of steps each
+    uint32_t b_stages;   // activation stages (fp16 weights: of both operands)
+    uint32_t raw;        // raw weight stages (quantized kinds), a pair of steps each
+    uint32_t splits;     // CTAs along K per output tile (grid.z = the cluster's size)
+    int32_t* status;
 };
 
 __device__ __forceinline__ uint32_t smem_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -88,46 +95,91 @@ __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
 __device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, uint32_t bytes) {
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(smem_addr(bar)), "r"(bytes) : "memory");
 }
-// 2-D tiled TMA load of the box at (x, y) into this CTA's shared memory at dst, completing on bar.
+// A position in a ring of stages: the stage and the parity of its current use.  Counted, not divided: a division by the
+// number of stages in every step cost the issuing thread more than the tensor core's work.
+struct Ring {
+    uint32_t stage = 0, phase = 0;
+    __device__ __forceinline__ void next(uint32_t stages) {
+        if (++stage == stages) stage = 0, phase ^= 1;
+    }
+    __device__ __forceinline__ void skip(uint32_t n, uint32_t stages) {  // n <= stages
+        stage += n;
+        if (stage >= stages) stage -= stages, phase ^= 1;
+    }
+};
+
+// True in one lane of the (converged) warp.  The compiler knows the branch is taken by one thread, which keeps the operands
+// of the tensor-core instructions in uniform registers; behind `lane == 0` each tcgen05.mma cost its thread 0.1 us.
+__device__ __forceinline__ bool elect_one() {
+    uint32_t pred;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "elect.sync _|p, 0xffffffff;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}\n"
+        : "=r"(pred));
+    return pred != 0;
+}
+// Tiled TMA load of the box at (x, y (, z)) into this CTA's shared memory at dst, completing on bar.
 __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, uint32_t x, uint32_t y, uint64_t* bar) {
     asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];\n" ::"r"(
                      smem_addr(dst)),
                  "l"(reinterpret_cast<uint64_t>(map)), "r"(smem_addr(bar)), "r"(x), "r"(y)
                  : "memory");
 }
-__device__ __forceinline__ void cp_async8z(void* dst, const void* src, bool valid) {
-    const uint32_t n = valid ? 8u : 0u;
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(smem_addr(dst)), "l"(src), "r"(n) : "memory");
+__device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* map, uint32_t x, uint32_t y, uint32_t z, uint64_t* bar) {
+    asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];\n" ::"r"(
+                     smem_addr(dst)),
+                 "l"(reinterpret_cast<uint64_t>(map)), "r"(smem_addr(bar)), "r"(x), "r"(y), "r"(z)
+                 : "memory");
 }
-// Waits for the phase with the given parity; gives up after kSpinLimit polls (or at once when another
-// wait of this CTA has already given up) and reports it.
-__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int32_t* status) {
+__device__ __forceinline__ void prefetch_map(const CUtensorMap* map) {
+    asm volatile("prefetch.tensormap [%0];\n" ::"l"(reinterpret_cast<uint64_t>(map)) : "memory");
+}
+__device__ __forceinline__ void cp_async4z(void* dst, const void* src, bool valid) {
+    const uint32_t n = valid ? 4u : 0u;  // src-size 0: zero-filled, nothing is read
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;\n" ::"r"(smem_addr(dst)), "l"(src), "r"(n) : "memory");
+}
+// Whether the phase with the given parity has completed, now (test) or within a short time (try, which may suspend the
+// thread).  The answer takes some 60 cycles: a thread that tests the next stage before it works on this one does not wait
+// for it.
+__device__ __forceinline__ bool mbar_test(uint64_t* bar, uint32_t parity) {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}\n"
+        : "=r"(ok)
+        : "r"(smem_addr(bar)), "r"(parity)
+        : "memory");
+    return ok != 0;
+}
+__device__ __forceinline__ bool mbar_try(uint64_t* bar, uint32_t parity) {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}\n"
+        : "=r"(ok)
+        : "r"(smem_addr(bar)), "r"(parity)
+        : "memory");
+    return ok != 0;
+}
+// Waits for it; gives up after kSpinLimit polls (or at once when another wait of this CTA has already given up) and
+// reports it.
+__device__ __forceinline__ void mbar_wait(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int32_t* status) {
+#pragma unroll 1
     for (uint32_t i = 0; i < kSpinLimit; ++i) {
-        uint32_t ok;
-        asm volatile(
-            "{\n\t.reg .pred p;\n\t"
-            "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-            "selp.u32 %0, 1, 0, p;\n\t}\n"
-            : "=r"(ok)
-            : "r"(smem_addr(bar)), "r"(parity)
-            : "memory");
-        if (ok) return true;
-        if (*abort_flag) return false;
+        if (mbar_try(bar, parity)) return;
+        if (*abort_flag) return;
     }
     *abort_flag = 1;
     if (status != nullptr) atomicExch(status, (int32_t)WRK_ERR_TIMEOUT);
-    return false;
 }
 
-__device__ __forceinline__ void fence_async_smem() { asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory"); }
 
-// K-major, 128-byte swizzle: rows of 128 bytes, groups of 8 rows 1024 bytes apart, 16-byte chunk index XOR row % 8.
-__device__ __forceinline__ uint32_t sw128_offset(uint32_t row, uint32_t chunk) {
-    return (row >> 3) * 1024 + (row & 7) * 128 + ((chunk ^ (row & 7)) << 4);
-}
-// Shared-memory matrix descriptor of such a tile (start address, LBO = 1, SBO = 1024 bytes, version 1, SWIZZLE_128B).
+// Shared-memory matrix descriptor of a K-major tile with 128-byte swizzle (start address, LBO = 1, SBO = 1024 bytes, version 1, SWIZZLE_128B).
 __device__ __forceinline__ uint64_t sw128_desc(uint32_t saddr) {
     uint64_t d = 0;
     d |= (uint64_t)((saddr & 0x3FFFF) >> 4);
@@ -150,6 +202,16 @@ __device__ __forceinline__ void umma_f16(uint32_t tmem_d, uint64_t desc_a, uint6
         : "r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
         : "memory");
 }
+// The same with the A operand in tensor memory: row m in lane m, two consecutive K elements per 32-bit column.
+__device__ __forceinline__ void umma_f16_ta(uint32_t tmem_d, uint32_t tmem_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}\n"
+        :
+        : "r"(tmem_d), "r"(tmem_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
+        : "memory");
+}
 __device__ __forceinline__ void umma_commit(uint64_t* bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(smem_addr(bar)) : "memory");
 }
@@ -158,6 +220,21 @@ __device__ __forceinline__ void tmem_ld8(uint32_t taddr, uint32_t v[8]) {
                  : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
                  : "r"(taddr)
                  : "memory");
+}
+// Four activations, out of line: the copy-out loop stays short.
+__device__ __noinline__ float4 activate4(int act, float4 v) {
+    return make_float4(activate_f(act, v.x), activate_f(act, v.y), activate_f(act, v.z), activate_f(act, v.w));
+}
+// 32 columns of this warp's 32 lanes; waits until the store has been performed.
+__device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t v[32]) {
+    asm volatile(
+        "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, "
+        "%17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31, %32};\n"
+        "tcgen05.wait::st.sync.aligned;\n" ::"r"(taddr),
+        "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]), "r"(v[9]), "r"(v[10]), "r"(v[11]),
+        "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15]), "r"(v[16]), "r"(v[17]), "r"(v[18]), "r"(v[19]), "r"(v[20]), "r"(v[21]), "r"(v[22]),
+        "r"(v[23]), "r"(v[24]), "r"(v[25]), "r"(v[26]), "r"(v[27]), "r"(v[28]), "r"(v[29]), "r"(v[30]), "r"(v[31])
+        : "memory");
 }
 __device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory"); }
 
@@ -185,22 +262,13 @@ __device__ __forceinline__ float4 ld_peer_smem(uint32_t local_addr, uint32_t ran
 
 __device__ __forceinline__ uint32_t pack_half2(__half2 v) { return *reinterpret_cast<uint32_t*>(&v); }
 
-// Two variations measured the same as this arrangement and were dropped: sixteen dequantizing warps, each taking half of
-// a step's columns (Int8 4096 x 4096 at 64 / 1024 tokens: 19.3 / 72.5 us against 19.1 / 74.4 us), and four MMA issuer
-// warps with an accumulator each (19.2 us at 64 tokens, slower at 256).  Neither the convert chain's latency nor the
-// single issuing thread paces the kernel at few tokens; its fixed work per launch does (set-up, pipeline fill,
-// epilogue, cluster reduction: about 10 of the 19 us).
-// 32 (Int8) weights of one row, raw bytes in `q0, q1`, block scale (min, max) -> four 16-byte groups of fp16.
-__device__ __forceinline__ void dequant_int8(uint4 q0, uint4 q1, uint32_t minmax, uint4 out[4]) {
-    // f32 dequantization, one rounding to fp16 per weight: the errors of a row are independent, none is
-    // shared by a whole block
-    const float2 mm = __half22float2(*reinterpret_cast<const __half2*>(&minmax));
-    const float sc = (mm.y - mm.x) * (1.0f / 255.0f), mn = mm.x;
-    const uint32_t words[8] = {q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, q1.z, q1.w};
+// 16 Int8 weights of one row (16 raw bytes), slope and minimum of their block -> 8 fp16 pairs.  f32 arithmetic, one
+// rounding to fp16 per weight: the errors of a row are independent, none is shared by a whole block.
+__device__ __forceinline__ void dequant_int8(uint4 q, float sc, float mn, uint32_t* h) {
+    const uint32_t words[4] = {q.x, q.y, q.z, q.w};
     const float2 sc2 = make_float2(sc, sc), mn2 = make_float2(mn, mn), bias2 = make_float2(-8388608.0f, -8388608.0f);
-    uint32_t h[16];
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
+    for (int i = 0; i < 4; ++i) {
         // byte b -> float 8388608 + b (0x4B000000 | b), minus 8388608: b exactly; two weights per instruction from
         // there on (add.f32x2, fma.rn.f32x2: the same roundings as the scalar forms)
         const float2 f01 = make_float2(__uint_as_float(__byte_perm(words[i], 0x4B000000u, 0x7650)),
@@ -210,22 +278,35 @@ __device__ __forceinline__ void dequant_int8(uint4 q0, uint4 q1, uint32_t minmax
         h[2 * i] = pack_half2(__float22half2_rn(__ffma2_rn(__fadd2_rn(f01, bias2), sc2, mn2)));
         h[2 * i + 1] = pack_half2(__float22half2_rn(__ffma2_rn(__fadd2_rn(f23, bias2), sc2, mn2)));
     }
-#pragma unroll
-    for (int j = 0; j < 4; ++j) out[j] = make_uint4(h[4 * j], h[4 * j + 1], h[4 * j + 2], h[4 * j + 3]);
 }
-// 32 NF4 weights (16 bytes, low nibble first) of one 64-weight block with absmax `am`.
-__device__ __forceinline__ void dequant_nf4(uint4 q, float am, const float2* lut2, uint4 out[4]) {
-    const uint32_t words[4] = {q.x, q.y, q.z, q.w};
-    uint32_t h[16];
+
+// The 16 weights a row's 64-weight NF4 block can hold, fp16(table[i] * absmax), as registers that byte permutes can index:
+// lo[j] / hi[j] hold the low / high bytes of entries 4 j .. 4 j + 3.
+struct Nf4Book {
+    uint32_t lo[4], hi[4];
+};
+__device__ __forceinline__ void nf4_book(const float* table, float am, Nf4Book& b) {
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
+    for (int j = 0; j < 4; ++j) {
+        const uint32_t e01 = pack_half2(__floats2half2_rn(table[4 * j] * am, table[4 * j + 1] * am));
+        const uint32_t e23 = pack_half2(__floats2half2_rn(table[4 * j + 2] * am, table[4 * j + 3] * am));
+        b.lo[j] = __byte_perm(e01, e23, 0x6420);
+        b.hi[j] = __byte_perm(e01, e23, 0x7531);
+    }
+}
+// Eight NF4 weights (one word, low nibble first) -> 4 fp16 pairs.  A byte permute looks up four nibbles' low three bits
+// in eight entries; the nibbles' top bits choose between the results for entries 0-7 and 8-15.  No shared memory: a
+// table there costs a data-dependent bank conflict per lookup (this loop took 1.2 us per step with one).
+__device__ __forceinline__ void dequant_nf4(uint32_t w, const Nf4Book& b, uint32_t* h) {
+    const uint32_t low3 = w & 0x77777777u, top = (w >> 3) & 0x11111111u;
 #pragma unroll
-        for (int b = 0; b < 4; ++b) {
-            const float2 pair = lut2[(words[i] >> (8 * b)) & 0xffu];  // (table[lo nibble], table[hi nibble])
-            h[4 * i + b] = pack_half2(__float22half2_rn(__fmul2_rn(pair, make_float2(am, am))));
-        }
-#pragma unroll
-    for (int j = 0; j < 4; ++j) out[j] = make_uint4(h[4 * j], h[4 * j + 1], h[4 * j + 2], h[4 * j + 3]);
+    for (int half = 0; half < 2; ++half) {
+        const uint32_t sel = low3 >> (16 * half), m = __byte_perm(0x0000ff00u, 0u, top >> (16 * half));  // 0xff where the top bit is set
+        const uint32_t lo = (__byte_perm(b.lo[0], b.lo[1], sel) & ~m) | (__byte_perm(b.lo[2], b.lo[3], sel) & m);
+        const uint32_t hi = (__byte_perm(b.hi[0], b.hi[1], sel) & ~m) | (__byte_perm(b.hi[2], b.hi[3], sel) & m);
+        h[2 * half] = __byte_perm(lo, hi, 0x5140);
+        h[2 * half + 1] = __byte_perm(lo, hi, 0x7362);
+    }
 }
 
 // One instantiation per weight format: the dequantizing loop holds only its own format's code.
@@ -237,308 +318,322 @@ matmul_umma_kernel(const __grid_constant__ UmmaGroup grp) {
 #pragma unroll
     for (uint32_t i = 1; i < (uint32_t)kMaxGroup; ++i)
         if (i < grp.count && blockIdx.x >= grp.tile_start[i]) gi = i;
-    const UmmaParams& p = grp.p[gi];
+    const UmmaProblem& p = grp.p[gi];
     const CUtensorMap& map_w = grp.map_w[gi];
     const CUtensorMap& map_x = grp.map_x[gi];
-    __shared__ uint64_t ab_full[kMaxStages], ab_empty[kMaxStages], raw_full[kMaxRaw], raw_empty[kMaxRaw], done_bar;
+    // full / empty of the A stages in tensor memory (quantized weights), of the operand stages in shared memory and of the
+    // raw weight stages
+    __shared__ uint64_t a_full[kMaxStages], a_empty[kMaxStages], b_full[kMaxStages], b_empty[kMaxStages], raw_full[kMaxRaw],
+        raw_empty[kMaxRaw], done_bar;
     __shared__ uint32_t tmem_base_slot;
-    __shared__ float2 lut2[256];
+    __shared__ __align__(16) float code_book[16];
     __shared__ int abort_flag;
 
-    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const uint32_t warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
     constexpr bool quantized = KIND != MAT_FP16;
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
-    const uint32_t b_bytes = p.n_tile * BK * 2;
-    const uint32_t stage_bytes = A_STAGE_BYTES + b_bytes;                   // [A | B], both 1024-byte aligned
-    constexpr uint32_t raw_row = KIND == MAT_INT8 ? 64u : 32u;              // raw bytes per row and step
-    const uint32_t raw_bytes = BM * raw_row;
-    uint8_t* raw_base = smem + (size_t)p.stages * stage_bytes;              // raw weight stages
-    uint8_t* scale_base = raw_base + (size_t)p.raw * raw_bytes;             // [2 groups][2 slots][BM][8 bytes]
-    const uint32_t m0 = (blockIdx.x - grp.tile_start[gi]) * BM, n0 = blockIdx.y * p.n_tile;
-    // this CTA's share of the K steps (split-K: grid.z CTAs per output tile)
-    const uint32_t nk_all = p.K / BK;
-    const uint32_t k_begin = (uint32_t)((uint64_t)nk_all * blockIdx.z / p.splits);
-    const uint32_t nk = (uint32_t)((uint64_t)nk_all * (blockIdx.z + 1) / p.splits) - k_begin;
-
-    if (threadIdx.x == 0) {
-        for (uint32_t s = 0; s < p.stages; ++s) {
-            mbar_init(&ab_full[s], quantized ? kDequantWarps / 2 + 1 : 2);  // one dequant group (or the weight TMA) + activation TMA
-            mbar_init(&ab_empty[s], 1);
+    // what the loops below use, in registers: read from the parameters, each would be fetched again after every asm
+    // statement (several memory round trips per step)
+    const uint32_t n_tile = grp.n_tile, bu = grp.bu, a_stages = grp.a_stages, b_stages = grp.b_stages, n_raw = grp.raw, splits = grp.splits;
+    const uint32_t M = p.M;
+    int32_t* const status = grp.status;
+    const uint32_t b_step = n_tile * BK * 2, b_bytes = bu * b_step;
+    constexpr uint32_t raw_row = KIND == MAT_INT8 ? 128u : 64u;  // raw bytes per row and pair of steps
+    constexpr uint32_t raw_bytes = BM * raw_row;
+    uint8_t* b_base = smem;                           // [b_stages] activation stages
+    uint8_t* w_base = smem + b_stages * b_bytes;      // fp16: [b_stages] weight stages; else [raw] raw stages and the scales
+    const uint32_t m0 = (blockIdx.x - grp.tile_start[gi]) * BM, n0 = blockIdx.y * n_tile;
+    // this CTA's share of K (split-K: grid.z CTAs per output tile) in units: a pair of steps for quantized weights, a
+    // stage for fp16 ones
+    const uint32_t unit = quantized ? 2u : bu, units = (grp.K / BK + unit - 1) / unit;
+    const uint32_t u_begin = units * blockIdx.z / splits, nu = units * (blockIdx.z + 1) / splits - u_begin;
+    // the first weights are on their way before anything else is set up
+    auto load_raw = [&](uint32_t u, uint32_t stage) {
+        mbar_expect_tx(&raw_full[stage], raw_bytes);
+        tma_load_2d(w_base + stage * raw_bytes, &map_w, (u_begin + u) * raw_row, m0, &raw_full[stage]);
+    };
+    auto load_weights = [&](uint32_t u, uint32_t stage) {
+        mbar_expect_tx(&b_full[stage], bu * A_STEP_BYTES);
+        tma_load_3d(w_base + stage * bu * A_STEP_BYTES, &map_w, 0, m0, (u_begin + u) * bu, &b_full[stage]);
+    };
+    const uint32_t ahead = min(nu, quantized ? n_raw : b_stages);
+    if (warp == kWeightTmaWarp) {
+        if (elect_one()) {
+            if (quantized) {
+                for (uint32_t r = 0; r < n_raw; ++r) {
+                    mbar_init(&raw_full[r], 1);
+                    mbar_init(&raw_empty[r], kDequantWarps / 2);  // the four warps of a dequantizing group
+                }
+            } else {
+                for (uint32_t r = 0; r < b_stages; ++r) mbar_init(&b_full[r], 2);  // both TMA threads
+            }
+            asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+#pragma unroll 1
+            for (uint32_t u = 0; u < ahead; ++u) {
+                if (quantized) load_raw(u, u);
+                else load_weights(u, u);
+            }
         }
-        for (uint32_t r = 0; r < p.raw; ++r) {
-            mbar_init(&raw_full[r], 1);
-            mbar_init(&raw_empty[r], kDequantWarps / 2);
-        }
-        mbar_init(&done_bar, 1);
-        abort_flag = 0;
-        asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
-    }
-    if (KIND == MAT_NF4 && threadIdx.x < 256) lut2[threadIdx.x] = make_float2(p.table[threadIdx.x & 15], p.table[threadIdx.x >> 4]);
-    if (warp == kMmaWarp) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(smem_addr(&tmem_base_slot)), "r"(p.tmem_cols)
+        __syncwarp();
+    } else if (warp == kMmaWarp) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(smem_addr(&tmem_base_slot)), "r"(grp.tmem_cols)
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
+    } else if (warp == kMmaWarp + 2) {
+        if (elect_one()) {
+            prefetch_map(&map_x);
+            for (uint32_t s = 0; s < b_stages; ++s) {
+                if (quantized) mbar_init(&b_full[s], 1);
+                mbar_init(&b_empty[s], 1);
+            }
+            for (uint32_t s = 0; s < a_stages; ++s) {
+                mbar_init(&a_full[s], kDequantWarps / 2);
+                mbar_init(&a_empty[s], 1);
+            }
+            mbar_init(&done_bar, 1);
+            abort_flag = 0;
+            asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+        }
+        __syncwarp();
+    } else if (KIND == MAT_NF4 && threadIdx.x < 16) {
+        code_book[threadIdx.x] = p.table[threadIdx.x];
     }
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tmem_d = tmem_base_slot;
+    const uint32_t tmem_d = tmem_base_slot, tmem_a = tmem_d + grp.acc_cols;
+    // the next kernel of a job may start from here on: this CTA has its tensor memory, so neither can wait for the other's
+    pdl_launch_dependents();
 
     if (warp < kDequantWarps) {
         if (quantized) {
-            // ---- dequantizers: two groups of four warps take alternate pairs of steps (group g: steps 4j + 2g and
-            // 4j + 2g + 1), so one group computes while the other sits in its fence and barriers; a thread owns a
-            // row: 64 weights per step, one proxy fence and one round of arrivals per pair ----
-            const uint32_t group = warp >> 2, row = threadIdx.x & (BM - 1);
-            const uint32_t m = m0 + row;
-            // scale slots cover 256 columns = four steps; the walk starts at a multiple of four steps
-            const uint32_t nsuper = (nk + 3) / 4;
-            const uint8_t* srow = reinterpret_cast<const uint8_t*>(p.scale) + ((size_t)m * (p.K / 256) + k_begin / 4) * 8;
-            uint8_t* my_scale = scale_base + group * 2 * SCALE_SLOT_BYTES + row * 8;  // [group][2 slots][BM][8 bytes]
-            cp_async8z(my_scale, srow, m < p.M);
-            asm volatile("cp.async.commit_group;\n" ::: "memory");
-            for (uint32_t j = 0; j < nsuper; ++j) {
-                if (j + 1 < nsuper) cp_async8z(my_scale + ((j + 1) & 1) * SCALE_SLOT_BYTES, srow + (size_t)(j + 1) * 8, m < p.M);
+            // ---- dequantizers: two groups of four warps take alternate pairs of steps (an Int8 block of 128 columns, two
+            // NF4 blocks), so one group computes while the other waits; a thread owns a row, i.e. a lane of tensor memory,
+            // and writes each step's 64 weights there as fp16 pairs ----
+            const uint32_t group = warp >> 2, row = threadIdx.x & (BM - 1), m = m0 + row;
+            const uint32_t lanes = ((warp & 3) * 32) << 16;
+            // one word of scales per row and pair (Int8 (min, max), NF4 two absmax): a thread copies its own row's words into
+            // its own slots of shared memory, kScaleAhead of the group's pairs before their use (a memory round trip lasts
+            // longer than a pair)
+            const uint32_t* srow = reinterpret_cast<const uint32_t*>(p.scale) + (size_t)(m < M ? m : 0) * (grp.K / (2 * BK));
+            uint32_t* my_scale = reinterpret_cast<uint32_t*>(w_base + n_raw * raw_bytes) + group * kScaleSlots * BM + row;
+            auto fetch_scale = [&](uint32_t i) {  // the group's i-th pair
+                const uint32_t u = group + 2 * i;
+                if (u < nu) cp_async4z(my_scale + (i % kScaleSlots) * BM, srow + u_begin + u, m < M);
                 asm volatile("cp.async.commit_group;\n" ::: "memory");
-                asm volatile("cp.async.wait_group 1;\n" ::: "memory");
-                const uint8_t* ss = my_scale + (j & 1) * SCALE_SLOT_BYTES;
-                const uint32_t kt0 = 4 * j + 2 * group;
+            };
+#pragma unroll 1
+            for (uint32_t i = 0; i < kScaleAhead; ++i) fetch_scale(i);
+            Ring raw, a;  // of this group's next pair
+            raw.skip(group, n_raw);
+            a.skip(group, a_stages);
+            const uint32_t swz = KIND == MAT_INT8 ? (row & 7) : ((row >> 1) & 3);  // the TMA unit's swizzle of this row
+#pragma unroll 1
+            for (uint32_t u = group, i = 0; u < nu; u += 2, ++i) {
+                fetch_scale(i + kScaleAhead);
+                asm volatile("cp.async.wait_group %0;\n" ::"n"(kScaleAhead) : "memory");
+                const uint32_t sc_word = my_scale[(i % kScaleSlots) * BM];
+                const float2 mm = __half22float2(*reinterpret_cast<const __half2*>(&sc_word));
+                mbar_wait(&raw_full[raw.stage], raw.phase, &abort_flag, status);
+                constexpr int kVecs = raw_row / 32;  // 16-byte pieces of a step
+                const uint8_t* rs = w_base + raw.stage * raw_bytes + row * raw_row;
+                // not unrolled: the warps of the kernel run four different loops, which together have to stay in the
+                // instruction caches of their schedulers (unrolled, a fifth of all stalls waited for instructions)
 #pragma unroll 1
                 for (uint32_t d = 0; d < 2; ++d) {
-                    const uint32_t kt = kt0 + d;
-                    if (kt >= nk) break;
-                    const uint32_t r = kt % p.raw;
-                    mbar_wait(&raw_full[r], (kt / p.raw) & 1, &abort_flag, p.status);
-                    const uint4* rs = reinterpret_cast<const uint4*>(raw_base + (size_t)r * raw_bytes + row * raw_row);
-                    const uint32_t s = kt % p.stages, use = kt / p.stages;
-                    if (use > 0) mbar_wait(&ab_empty[s], (use - 1) & 1, &abort_flag, p.status);
-                    uint8_t* sa = smem + (size_t)s * stage_bytes;
-                    uint4 wv[4];
+                    uint4 q[kVecs];
 #pragma unroll
-                    for (uint32_t h = 0; h < 2; ++h) {  // columns 32 h .. 32 h + 31 of the step
-                        if (KIND == MAT_INT8)  // a 128-column block is two steps: this group's pair shares (min, max)
-                            dequant_int8(rs[2 * h], rs[2 * h + 1], *reinterpret_cast<const uint32_t*>(ss + group * 4), wv);
-                        else
-                            dequant_nf4(rs[h], __half2float(*reinterpret_cast<const __half*>(ss + (kt & 3) * 2)), lut2, wv);
-#pragma unroll
-                        for (uint32_t c = 0; c < 4; ++c) *reinterpret_cast<uint4*>(sa + sw128_offset(row, h * 4 + c)) = wv[c];
+                    for (uint32_t c = 0; c < kVecs; ++c) q[c] = *reinterpret_cast<const uint4*>(rs + (((kVecs * d + c) ^ swz) << 4));
+                    if (d == 1) {
+                        __syncwarp();  // every lane has its raw bytes in registers
+                        if (lane == 0) mbar_arrive(&raw_empty[raw.stage]);
                     }
-                    __syncwarp();  // every lane has consumed its raw bytes
-                    if (lane == 0) mbar_arrive(&raw_empty[r]);  // the raw stage may be refilled
+                    uint32_t h[32];
+                    if (KIND == MAT_INT8) {
+                        const float sc = (mm.y - mm.x) * (1.0f / 255.0f);
+#pragma unroll
+                        for (int c = 0; c < kVecs; ++c) dequant_int8(q[c], sc, mm.x, h + (8 * c) % 32);
+                    } else {
+                        Nf4Book book;
+                        nf4_book(code_book, d == 0 ? mm.x : mm.y, book);
+#pragma unroll
+                        for (int c = 0; c < kVecs; ++c) {
+                            dequant_nf4(q[c].x, book, h + (16 * c) % 32);
+                            dequant_nf4(q[c].y, book, h + (16 * c) % 32 + 4);
+                            dequant_nf4(q[c].z, book, h + (16 * c) % 32 + 8);
+                            dequant_nf4(q[c].w, book, h + (16 * c) % 32 + 12);
+                        }
+                    }
+                    if (d == 0) {
+                        mbar_wait(&a_empty[a.stage], a.phase ^ 1, &abort_flag, status);  // at once in the stage's first use
+                        tc_fence_after();
+                    }
+                    tmem_st32(tmem_a + lanes + (2 * a.stage + d) * A_STEP_COLS, h);
                 }
-                fence_async_smem();  // generic-proxy stores -> visible to the tensor core's async proxy
+                tc_fence_before();
                 __syncwarp();
-                if (lane == 0) {
-                    if (kt0 < nk) mbar_arrive(&ab_full[kt0 % p.stages]);
-                    if (kt0 + 1 < nk) mbar_arrive(&ab_full[(kt0 + 1) % p.stages]);
-                }
+                if (lane == 0) mbar_arrive(&a_full[a.stage]);
+                raw.skip(2, n_raw);
+                a.skip(2, a_stages);  // past the other group's pair
             }
         }
-        // ---- epilogue: TMEM -> registers -> activation -> token-major rows ----
-        mbar_wait(&done_bar, 0, &abort_flag, p.status);
+        // ---- the accumulator to shared memory, [token][128 rows] in f32 (the operand stages are free once every MMA has
+        // completed): warp w holds lanes 32 (w % 4) .. and takes half of the columns ----
+        mbar_wait(&done_bar, 0, &abort_flag, status);
         tc_fence_after();
-        const uint32_t quad = warp & 3, side = warp >> 2;  // lanes 32 quad .., half of the columns each
-        const uint32_t m = m0 + quad * 32 + lane;
-        const uint32_t c_begin = side * (p.n_tile / 2), c_end = c_begin + p.n_tile / 2;
-        // split K: the partial tile goes to this CTA's own shared memory (the operand stages are free once every
-        // MMA has completed), column-major [n_tile][BM] floats, for the cluster-wide sum below
-        float* ws_mine = reinterpret_cast<float*>(smem);
-        const size_t col_stride = p.out.stride[0], out_row = p.out.index(m < p.M ? m : 0, n0, 0);
-        const bool act_none = p.act == WRK_ACT_NONE;
-        // one CTA per output tile: the tile goes through shared memory when 16-byte pieces of a column are aligned in
-        // the output (its first element of the tile 16-byte aligned, columns a multiple of 16 bytes apart)
-        const uint32_t osize = p.out.dtype == WRK_F16 ? 2u : 4u;
-        const bool staged = p.splits == 1 && (reinterpret_cast<uintptr_t>(p.out.base) + p.out.index(m0, n0, 0) * osize) % 16 == 0 &&
-                            (col_stride * osize) % 16 == 0;
-        // up to four 8-column accumulator loads are in flight before the single wait
+        const uint32_t quad = warp & 3, c_begin = (warp >> 2) * (n_tile / 2), c_end = c_begin + n_tile / 2;
+        float* tile = reinterpret_cast<float*>(smem) + quad * 32 + lane;
+#pragma unroll 1
         for (uint32_t c0 = c_begin; c0 < c_end; c0 += 32) {
             uint32_t v[4][8];
 #pragma unroll
             for (uint32_t q = 0; q < 4; ++q)
                 if (c0 + 8 * q < c_end) tmem_ld8(tmem_d + ((quad * 32) << 16) + c0 + 8 * q, v[q]);
             tmem_ld_wait();
-            if (!act_none && p.splits == 1) {  // the activation once, outside the store loops (which then hold no branch)
-#pragma unroll
-                for (uint32_t q = 0; q < 4; ++q)
-#pragma unroll
-                    for (int j = 0; j < 8; ++j) v[q][j] = __float_as_uint(activate_f(p.act, __uint_as_float(v[q][j])));
-            }
 #pragma unroll
             for (uint32_t q = 0; q < 4; ++q) {
-                const uint32_t c = c0 + 8 * q;
-                if (c >= c_end) continue;
-                if (p.splits > 1) {
+                if (c0 + 8 * q >= c_end) break;
 #pragma unroll
-                    for (int j = 0; j < 8; ++j) ws_mine[(size_t)(c + j) * BM + quad * 32 + lane] = __uint_as_float(v[q][j]);
-                } else if (staged) {
-                    // the finished values, in the output's type, into a [column][row] tile in shared memory
-                    if (p.out.dtype == WRK_F16) {
-                        __half* t = reinterpret_cast<__half*>(smem);
-#pragma unroll
-                        for (int j = 0; j < 8; ++j)
-                            t[(size_t)(c + j) * BM + quad * 32 + lane] =
-                                __float2half_rn(__uint_as_float(v[q][j]));
-                    } else {
-#pragma unroll
-                        for (int j = 0; j < 8; ++j)
-                            ws_mine[(size_t)(c + j) * BM + quad * 32 + lane] =
-                                __uint_as_float(v[q][j]);
-                    }
-                } else if (m < p.M) {
-                    // element (m, n) of the output lies col_stride elements after (m, n - 1): one address, then steps
-                    const size_t at = out_row + (size_t)c * col_stride;
-                    if (p.out.dtype == WRK_F16) {
-                        __half* o = static_cast<__half*>(p.out.base) + at;
-#pragma unroll
-                        for (int j = 0; j < 8; ++j)
-                            if (n0 + c + j < p.N) o[(size_t)j * col_stride] = __float2half_rn(__uint_as_float(v[q][j]));
-                    } else {
-                        float* o = static_cast<float*>(p.out.base) + at;
-#pragma unroll
-                        for (int j = 0; j < 8; ++j)
-                            if (n0 + c + j < p.N) o[(size_t)j * col_stride] = __uint_as_float(v[q][j]);
-                    }
-                }
-            }
-        }
-        if (staged) {
-            // ... and from there to global memory in 16-byte pieces: the 128 rows of a column are adjacent elements of
-            // the output, so a warp writes whole 256- or 512-byte runs instead of 64 bytes per instruction
-            asm volatile("bar.sync 1, %0;\n" ::"n"(kDequantWarps * 32) : "memory");
-            const uint32_t esize = p.out.dtype == WRK_F16 ? 2u : 4u, per_col = BM * esize / 16, per_vec = 16 / esize;
-            const uint32_t cols = min(p.n_tile, p.N - n0);
-            const size_t col0 = p.out.index(m0, n0, 0);
-            for (uint32_t i = threadIdx.x; i < cols * per_col; i += kDequantWarps * 32) {
-                const uint32_t c = i / per_col, r = (i % per_col) * per_vec;  // column, first row of the piece
-                if (m0 + r >= p.M) continue;
-                const uint4 piece = *reinterpret_cast<const uint4*>(smem + ((size_t)c * BM + r) * esize);
-                uint8_t* dst = static_cast<uint8_t*>(p.out.base) + (col0 + (size_t)c * col_stride + r) * esize;
-                if (m0 + r + per_vec <= p.M) {
-                    *reinterpret_cast<uint4*>(dst) = piece;
-                } else {  // the matrix ends inside the piece
-                    const uint8_t* src = reinterpret_cast<const uint8_t*>(&piece);
-                    for (uint32_t e = 0; e < (p.M - m0 - r) * esize; ++e) dst[e] = src[e];
-                }
+                for (int j = 0; j < 8; ++j) tile[(c0 + 8 * q + j) * BM] = __uint_as_float(v[q][j]);
             }
         }
     } else if (warp == kMmaWarp) {
-        // ---- MMA issuer ----
-        const uint32_t idesc = f16_idesc(BM, p.n_tile);
-        for (uint32_t kt = 0; kt < nk; ++kt) {
-            const uint32_t s = kt % p.stages, use = kt / p.stages;
-            mbar_wait(&ab_full[s], use & 1, &abort_flag, p.status);
-            tc_fence_after();
-            if (lane == 0) {
-                const uint32_t sa = smem_addr(smem + (size_t)s * stage_bytes);
-                const uint64_t da = sw128_desc(sa), db = sw128_desc(sa + A_STAGE_BYTES);
+        // ---- MMA issuer: one thread ----
+        if (elect_one()) {
+            const uint32_t idesc = f16_idesc(BM, n_tile);
+            Ring ra, rb;
+            bool have_a = quantized && mbar_test(&a_full[0], 0), have_b = mbar_test(&b_full[0], 0);
+            uint32_t accumulate = 0;
+            // the stage of shared memory that comes next: its `steps` steps, four MMAs of K = 16 each (32 bytes of K per
+            // instruction: + 2 in a descriptor's address field)
+            auto stage = [&](uint32_t ta) {
+                if (!have_b) mbar_wait(&b_full[rb.stage], rb.phase, &abort_flag, status);
+                tc_fence_after();
+                const uint64_t db = sw128_desc(smem_addr(b_base + rb.stage * b_bytes));
+                const uint64_t da = quantized ? 0 : sw128_desc(smem_addr(w_base + rb.stage * bu * A_STEP_BYTES));
+                uint64_t* done = &b_empty[rb.stage];
+                rb.next(b_stages);
+                have_b = mbar_test(&b_full[rb.stage], rb.phase);  // of the next stage: answered while this one is issued
+#pragma unroll 1
+                for (uint32_t d = 0; d < bu; ++d) {
 #pragma unroll
-                for (uint32_t kk = 0; kk < BK / 16; ++kk)  // 32 bytes of K per instruction: + 2 in the address field
-                    umma_f16(tmem_d, da + 2 * kk, db + 2 * kk, idesc, (kt | kk) != 0 ? 1u : 0u);
-                umma_commit(&ab_empty[s]);  // arrives when the MMAs above have read the stage
+                    for (uint32_t kk = 0; kk < BK / 16; ++kk) {
+                        if (quantized) umma_f16_ta(tmem_d, ta + d * A_STEP_COLS + 8 * kk, db + d * (b_step >> 4) + 2 * kk, idesc, accumulate);
+                        else umma_f16(tmem_d, da + d * (A_STEP_BYTES >> 4) + 2 * kk, db + d * (b_step >> 4) + 2 * kk, idesc, accumulate);
+                        accumulate = 1;
+                    }
+                }
+                umma_commit(done);  // arrives when the MMAs above have read the stage
+            };
+#pragma unroll 1
+            for (uint32_t u = 0; u < nu; ++u) {
+                if (quantized) {
+                    if (!have_a) mbar_wait(&a_full[ra.stage], ra.phase, &abort_flag, status);
+                    const uint32_t ta = tmem_a + 2 * ra.stage * A_STEP_COLS;
+                    uint64_t* done = &a_empty[ra.stage];
+                    ra.next(a_stages);
+                    have_a = mbar_test(&a_full[ra.stage], ra.phase);
+#pragma unroll 1
+                    for (uint32_t d = 0; d < 2; d += bu) stage(ta + d * A_STEP_COLS);
+                    umma_commit(done);
+                } else {
+                    stage(0);
+                }
             }
-            __syncwarp();
+            umma_commit(&done_bar);
         }
-        if (lane == 0) umma_commit(&done_bar);
         __syncwarp();
     } else if (warp == kWeightTmaWarp) {
-        if (lane == 0) {
-            if (quantized) {
-                for (uint32_t kt = 0; kt < nk; ++kt) {
-                    const uint32_t r = kt % p.raw, ruse = kt / p.raw;
-                    if (ruse > 0) mbar_wait(&raw_empty[r], (ruse - 1) & 1, &abort_flag, p.status);
-                    mbar_expect_tx(&raw_full[r], raw_bytes);
-                    tma_load_2d(raw_base + (size_t)r * raw_bytes, &map_w, (k_begin + kt) * raw_row, m0, &raw_full[r]);
-                }
-            } else {
-                for (uint32_t kt = 0; kt < nk; ++kt) {
-                    const uint32_t s = kt % p.stages, use = kt / p.stages;
-                    if (use > 0) mbar_wait(&ab_empty[s], (use - 1) & 1, &abort_flag, p.status);
-                    mbar_expect_tx(&ab_full[s], A_STAGE_BYTES);
-                    tma_load_2d(smem + (size_t)s * stage_bytes, &map_w, (k_begin + kt) * BK, m0, &ab_full[s]);
+        if (elect_one()) {
+            Ring ring;
+            ring.skip(ahead, quantized ? n_raw : b_stages);
+#pragma unroll 1
+            for (uint32_t u = ahead; u < nu; ++u) {
+                if (quantized) {
+                    mbar_wait(&raw_empty[ring.stage], ring.phase ^ 1, &abort_flag, status);
+                    load_raw(u, ring.stage);
+                    ring.next(n_raw);
+                } else {
+                    mbar_wait(&b_empty[ring.stage], ring.phase ^ 1, &abort_flag, status);
+                    load_weights(u, ring.stage);
+                    ring.next(b_stages);
                 }
             }
         }
+        __syncwarp();
     } else {
-        if (lane == 0) {
-            for (uint32_t kt = 0; kt < nk; ++kt) {
-                const uint32_t s = kt % p.stages, use = kt / p.stages;
-                if (use > 0) mbar_wait(&ab_empty[s], (use - 1) & 1, &abort_flag, p.status);
-                mbar_expect_tx(&ab_full[s], b_bytes);
-                tma_load_2d(smem + (size_t)s * stage_bytes + A_STAGE_BYTES, &map_x, (k_begin + kt) * BK, n0, &ab_full[s]);
+        if (elect_one()) {
+            pdl_wait();  // the only loads of what a kernel before this one wrote; the outputs are stored after they have arrived
+            Ring ring;
+#pragma unroll 1
+            for (uint32_t u = 0; u < nu; ++u) {
+                const uint32_t first = (u_begin + u) * unit;
+#pragma unroll 1
+                for (uint32_t d = 0; d < unit; d += bu) {
+                    mbar_wait(&b_empty[ring.stage], ring.phase ^ 1, &abort_flag, status);
+                    mbar_expect_tx(&b_full[ring.stage], b_bytes);
+                    tma_load_3d(b_base + ring.stage * b_bytes, &map_x, 0, n0, first + d, &b_full[ring.stage]);
+                    ring.next(b_stages);
+                }
             }
         }
+        __syncwarp();
     }
     tc_fence_before();
-    __syncthreads();
+    if (splits > 1) cluster_sync();  // a hardware barrier that every thread reaches, also after a wait above has given up
+    else __syncthreads();
     if (warp == kMmaWarp) {
         tc_fence_after();
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem_d), "r"(p.tmem_cols) : "memory");
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem_d), "r"(grp.tmem_cols) : "memory");
     }
-    if (p.splits > 1) {
-        // The CTAs of a cluster hold the partial tiles of one output tile.  After the cluster barrier CTA r adds
-        // its share of the columns over all peers (in rank order: the sum does not depend on timing), through
-        // distributed shared memory, and finishes those outputs.  The second barrier keeps every CTA's shared
-        // memory alive until its peers have read it.  Both are hardware barriers that every thread reaches, also
-        // after a wait above has given up.
-        cluster_sync();
-        const uint32_t rank = cluster_rank();
-        {
-            constexpr uint32_t kGroups = 4, kReduceThreads = kUmmaThreads;
-            const uint32_t c_lo = p.n_tile * rank / p.splits, c_hi = p.n_tile * (rank + 1) / p.splits;
-            const uint32_t v_lo = c_lo * (BM / 4), v_hi = c_hi * (BM / 4);  // groups of four rows
-            const uint32_t base_addr = smem_addr(smem);
-            const bool out_vec = reinterpret_cast<uintptr_t>(p.out.base) % 16 == 0;
-            for (uint32_t base = v_lo; base < v_hi; base += kGroups * kReduceThreads) {
-                float4 sum[kGroups];
+    // ---- from shared memory to the output, four rows of a token per thread and step (adjacent elements of the output).  With
+    // K split over a cluster, CTA r finishes its share of the columns: the sum over its peers' tiles, through distributed
+    // shared memory, in rank order (it does not depend on timing) ----
+    const uint32_t rank = splits > 1 ? cluster_rank() : 0;
+    const uint32_t v_lo = n_tile * rank / splits * (BM / 4), v_hi = min(n_tile * (rank + 1) / splits, grp.N - n0) * (BM / 4);
+    const uint32_t tile_addr = smem_addr(smem);
+    const bool out_vec = reinterpret_cast<uintptr_t>(p.out.base) % 16 == 0, f16 = p.out.dtype == WRK_F16;
+    const size_t col_stride = p.out.stride[0], at0 = p.out.index(m0, n0, 0);
+    const int act = p.act;
+    constexpr uint32_t kBatch = 4;  // positions whose loads are in flight together
+#pragma unroll 1
+    for (uint32_t base = v_lo + threadIdx.x; base < v_hi; base += kBatch * kUmmaThreads) {
+        float4 sum[kBatch];
 #pragma unroll
-                for (uint32_t u = 0; u < kGroups; ++u) sum[u] = make_float4(0.f, 0.f, 0.f, 0.f);
-                for (uint32_t z0 = 0; z0 < p.splits; z0 += 4) {
-                    float4 v[kGroups][4];
+        for (uint32_t i = 0; i < kBatch; ++i) sum[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 1
+        for (uint32_t z = 0; z < splits; ++z) {
+            float4 v[kBatch];
 #pragma unroll
-                    for (uint32_t u = 0; u < kGroups; ++u) {
-                        const uint32_t pos = base + u * kReduceThreads + threadIdx.x;
+            for (uint32_t i = 0; i < kBatch; ++i) {
+                const uint32_t pos = min(base + i * kUmmaThreads, v_hi - 1);
+                v[i] = splits > 1 ? ld_peer_smem(tile_addr + pos * 16, z) : *reinterpret_cast<const float4*>(smem + pos * 16);
+            }
 #pragma unroll
-                        for (uint32_t dz = 0; dz < 4; ++dz) {
-                            v[u][dz] = make_float4(0.f, 0.f, 0.f, 0.f);
-                            if (pos < v_hi && z0 + dz < p.splits) v[u][dz] = ld_peer_smem(base_addr + pos * 16, z0 + dz);
-                        }
-                    }
+            for (uint32_t i = 0; i < kBatch; ++i) sum[i].x += v[i].x, sum[i].y += v[i].y, sum[i].z += v[i].z, sum[i].w += v[i].w;
+        }
 #pragma unroll
-                    for (uint32_t u = 0; u < kGroups; ++u)
-#pragma unroll
-                        for (uint32_t dz = 0; dz < 4; ++dz)
-                            sum[u].x += v[u][dz].x, sum[u].y += v[u][dz].y, sum[u].z += v[u][dz].z, sum[u].w += v[u][dz].w;
+        for (uint32_t i = 0; i < kBatch; ++i) {
+            const uint32_t pos = base + i * kUmmaThreads, c = pos / (BM / 4), row = (pos % (BM / 4)) * 4;
+            if (pos >= v_hi || m0 + row >= M) continue;
+            const float4 r = act != WRK_ACT_NONE ? activate4(act, sum[i]) : sum[i];
+            const size_t at = at0 + c * col_stride + row;
+            if (m0 + row + 3 < M && (at & 3) == 0 && out_vec) {
+                if (f16) {
+                    const __half2 lo = __floats2half2_rn(r.x, r.y), hi = __floats2half2_rn(r.z, r.w);
+                    *reinterpret_cast<uint2*>(static_cast<__half*>(p.out.base) + at) = make_uint2(pack_half2(lo), pack_half2(hi));
+                } else {
+                    *reinterpret_cast<float4*>(static_cast<float*>(p.out.base) + at) = r;
                 }
-#pragma unroll
-                for (uint32_t u = 0; u < kGroups; ++u) {
-                    const uint32_t pos = base + u * kReduceThreads + threadIdx.x;
-                    if (pos >= v_hi) continue;
-                    const uint32_t c = pos / (BM / 4), row = (pos % (BM / 4)) * 4;
-                    const uint32_t n = n0 + c, m = m0 + row;
-                    if (n >= p.N) continue;
-                    float r4[4] = {sum[u].x, sum[u].y, sum[u].z, sum[u].w};
-                    if (p.act != WRK_ACT_NONE) {
-#pragma unroll
-                        for (int e = 0; e < 4; ++e) r4[e] = activate_f(p.act, r4[e]);
-                    }
-                    const size_t at = p.out.index(m, n, 0);  // rows m .. m + 3 of a column are adjacent elements
-                    if (m + 3 < p.M && (at & 3) == 0 && out_vec) {
-                        if (p.out.dtype == WRK_F16) {
-                            const __half2 lo = __floats2half2_rn(r4[0], r4[1]), hi = __floats2half2_rn(r4[2], r4[3]);
-                            *reinterpret_cast<uint2*>(static_cast<__half*>(p.out.base) + at) = make_uint2(pack_half2(lo), pack_half2(hi));
-                        } else {
-                            *reinterpret_cast<float4*>(static_cast<float*>(p.out.base) + at) = make_float4(r4[0], r4[1], r4[2], r4[3]);
-                        }
-                    } else {
-#pragma unroll
-                        for (int e = 0; e < 4; ++e)
-                            if (m + e < p.M) dstore(p.out.base, p.out.dtype, at + e, r4[e]);
-                    }
-                }
+            } else {
+                dstore(p.out.base, p.out.dtype, at, r.x);
+                if (m0 + row + 1 < M) dstore(p.out.base, p.out.dtype, at + 1, r.y);
+                if (m0 + row + 2 < M) dstore(p.out.base, p.out.dtype, at + 2, r.z);
+                if (m0 + row + 3 < M) dstore(p.out.base, p.out.dtype, at + 3, r.w);
             }
         }
-        cluster_sync();
     }
+    if (splits > 1) cluster_sync();  // the peers have read this CTA's shared memory
 }
 
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
@@ -558,25 +653,33 @@ EncodeTiledFn encode_tiled() {
     return fn;
 }
 
-bool make_map_2d(CUtensorMap* map, CUtensorMapDataType dt, const void* base, uint64_t inner, uint64_t rows, uint64_t row_bytes,
-                 uint32_t box_inner, uint32_t box_rows, CUtensorMapSwizzle swz) {
+bool make_map(CUtensorMap* map, CUtensorMapDataType dt, const void* base, std::initializer_list<uint64_t> dims,
+              std::initializer_list<uint64_t> strides, std::initializer_list<uint32_t> box, CUtensorMapSwizzle swz) {
     EncodeTiledFn fn = encode_tiled();
     if (fn == nullptr) return false;
-    const cuuint64_t gdim[2] = {inner, rows};
-    const cuuint64_t gstride[1] = {row_bytes};
-    const cuuint32_t box[2] = {box_inner, box_rows};
-    const cuuint32_t estr[2] = {1, 1};
-    return fn(map, dt, 2, const_cast<void*>(base), gdim, gstride, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, swz,
+    cuuint64_t gdim[3], gstride[2];
+    cuuint32_t gbox[3];
+    const cuuint32_t estr[3] = {1, 1, 1};
+    std::copy(dims.begin(), dims.end(), gdim);
+    std::copy(strides.begin(), strides.end(), gstride);
+    std::copy(box.begin(), box.end(), gbox);
+    return fn(map, dt, (cuuint32_t)dims.size(), const_cast<void*>(base), gdim, gstride, gbox, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, swz,
               CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+// fp16 [rows][K], rows row_bytes apart, as boxes of [steps][box_rows][64 values]: K in steps of 64 is the outermost dimension,
+// so one copy brings several steps, each a tile of its own in the 128-byte swizzle
+bool make_operand_map(CUtensorMap* map, const void* base, uint32_t K, uint32_t rows, uint64_t row_bytes, uint32_t box_rows, uint32_t steps) {
+    return make_map(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, base, {BK, rows, K / BK}, {row_bytes, BK * 2}, {BK, box_rows, steps},
+                    CU_TENSOR_MAP_SWIZZLE_128B);
 }
 
 }  // namespace
 
 bool matmul_umma_supported(const MatmulArgs& a) {
-    if (a.B != 1 || a.N < 16 || a.M == 0) return false;
-    if (a.K % BK != 0 || (a.kind != MAT_FP16 && a.K % 256 != 0)) return false;  // scale slots are fetched 8 bytes at a time
+    if (a.B != 1 || a.N <= 8 || a.M == 0) return false;
+    if (a.K % BK != 0 || (a.kind != MAT_FP16 && a.K % (2 * BK) != 0)) return false;  // quantized weights come in pairs of steps
     if (reinterpret_cast<uintptr_t>(a.matrix) % 16 != 0) return false;
-    if (a.scale != nullptr && reinterpret_cast<uintptr_t>(a.scale) % 8 != 0) return false;
+    if (a.scale != nullptr && reinterpret_cast<uintptr_t>(a.scale) % 4 != 0) return false;
     // activations go through a tensor map: fp16, rows 16-byte aligned
     if (a.in.dtype != WRK_F16 || a.in.stride[0] % 8 != 0) return false;
     const uintptr_t x0 = reinterpret_cast<uintptr_t>(a.in.base) + a.in.index(0, 0, 0) * 2;
@@ -604,18 +707,16 @@ cudaError_t matmul_umma_group(const MatmulArgs* args, int count, int32_t* status
         row_tiles += (args[i].M + BM - 1) / BM;
     }
     for (int i = count; i <= kMaxGroup; ++i) g.tile_start[i] = row_tiles;
-    UmmaParams p{};
-    p.kind = a.kind;
-    p.K = a.K;
-    p.N = a.N;
-    p.status = status;
+    g.K = a.K;
+    g.N = a.N;
+    g.status = status;
+    const bool quantized = a.kind != MAT_FP16;
     const uint32_t nk = a.K / BK;
     // Output tiles are 128 rows x n_tile tokens; K is split across the CTAs of a thread-block cluster while the
-    // tiles alone leave SMs idle: a split keeps at least eight steps (a multiple of four, so scale slots stay
-    // aligned), a cluster at most 8 CTAs.  Up to 512 tokens, 128-token tiles replace 256-token ones when that
-    // doubles the CTAs of the single wave without lengthening a CTA's K walk: smaller operand stages (a deeper
-    // ring) and smaller partial tiles.  (Measured: 2048x2048 Int8, 256 tokens: 22.8 -> 15.9 us; where the K walk
-    // would double instead, 31 -> 37 us, so those keep 256.)
+    // tiles alone leave SMs idle: a split keeps at least eight steps, a cluster at most 8 CTAs.  Up to 512 tokens,
+    // 128-token tiles replace 256-token ones when that doubles the CTAs of the single wave without lengthening a CTA's
+    // K walk: smaller operand stages (a deeper ring) and smaller partial tiles.  (Measured: 2048x2048 Int8, 256 tokens:
+    // 22.8 -> 15.9 us; where the K walk would double instead, 31 -> 37 us, so those keep 256.)
     int sms = 148, device = 0;
     if (cudaGetDevice(&device) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
     auto splits_for = [&](uint32_t n_tile) {
@@ -623,42 +724,56 @@ cudaError_t matmul_umma_group(const MatmulArgs* args, int count, int32_t* status
         uint32_t want = std::max<uint32_t>(1, (uint32_t)sms / tiles);
         want = std::min<uint32_t>(want, std::max<uint32_t>(1, nk / 8));
         want = std::min<uint32_t>(want, 8);
-        while (want > 1 && nk % (4 * want) != 0) --want;
+        while (nk % 4 == 0 && nk % (4 * want) != 0) --want;  // equal shares where K allows them
         return want;
     };
-    p.n_tile = std::min<uint32_t>(256, (a.N + 15) / 16 * 16);
-    p.splits = splits_for(p.n_tile);
-    if (p.n_tile > 128 && a.N <= 512) {
+    g.n_tile = std::min<uint32_t>(256, (a.N + 15) / 16 * 16);
+    g.splits = splits_for(g.n_tile);
+    if (g.n_tile > 128 && a.N <= 512) {
         const uint32_t s2 = splits_for(128);
-        if (s2 >= p.splits && row_tiles * ((a.N + 127) / 128) * s2 <= (uint32_t)sms) p.n_tile = 128, p.splits = s2;
+        if (s2 >= g.splits && row_tiles * ((a.N + 127) / 128) * s2 <= (uint32_t)sms) g.n_tile = 128, g.splits = s2;
     }
-    p.tmem_cols = 32;
-    while (p.tmem_cols < p.n_tile) p.tmem_cols *= 2;
-    const uint32_t stage_bytes = A_STAGE_BYTES + p.n_tile * BK * 2;
-    const uint32_t raw_bytes = a.kind == MAT_INT8 ? BM * 64 : a.kind == MAT_NF4 ? BM * 32 : 0;
-    // all of an SM's shared memory but the static part and the alignment slack: at 256-token tiles (48 KB operand
-    // stages) that is four stages, one pair for each group of dequantizing warps, instead of three
-    const uint32_t budget = 222u * 1024;
-    p.raw = a.kind == MAT_FP16 ? 0 : std::min<uint32_t>(kMaxRaw, std::max<uint32_t>(2, nk));
-    p.stages = std::min<uint32_t>(kMaxStages, std::max<uint32_t>(2, nk));
-    while (p.stages * stage_bytes + p.raw * raw_bytes + 4 * SCALE_SLOT_BYTES > budget) {
-        if (p.raw > 4) --p.raw;
-        else if (p.stages > 4) --p.stages;
-        else if (p.raw > 2) --p.raw;
-        else if (p.stages > 2) --p.stages;
-        else break;
+    // a copy of activations brings two steps unless a step's tile is large already; fewer, larger copies: issuing one costs
+    // its thread about 0.2 us, as much as the MMAs of a step of 64 tokens take
+    g.bu = g.n_tile <= 128 ? 2 : 1;
+    // tensor memory: the accumulator and (quantized weights) A stages of a pair of steps
+    g.acc_cols = (g.n_tile + 31) / 32 * 32;
+    g.tmem_cols = g.acc_cols;
+    if (quantized) {
+        g.tmem_cols = g.acc_cols <= 64 ? 256 : 512;
+        g.a_stages = std::min<uint32_t>(kMaxStages, (g.tmem_cols - g.acc_cols) / (2 * A_STEP_COLS));
     }
-    if (p.splits > 1) {
-        const uint32_t nk_split = nk / p.splits;
-        p.stages = std::min<uint32_t>(p.stages, std::max<uint32_t>(2, nk_split));
-        if (p.raw) p.raw = std::min<uint32_t>(p.raw, std::max<uint32_t>(2, nk_split));
+    for (uint32_t c = 32;; c *= 2)
+        if (c >= g.tmem_cols) {
+            g.tmem_cols = c;
+            break;
+        }
+    const uint32_t unit = quantized ? 2 : g.bu, walk = ((nk + unit - 1) / unit + g.splits - 1) / g.splits;  // most units of a CTA
+    const uint32_t b_bytes = g.bu * g.n_tile * BK * 2;
+    const uint32_t raw_bytes = a.kind == MAT_INT8 ? BM * 128 : a.kind == MAT_NF4 ? BM * 64 : 0;
+    const uint32_t budget = 222u * 1024;  // of an SM's shared memory: less the static part and the alignment slack
+    size_t smem = 0;
+    if (quantized) {
+        g.b_stages = std::min<uint32_t>(kMaxStages, std::max<uint32_t>(2, walk * (2 / g.bu)));
+        g.raw = std::min<uint32_t>(kMaxRaw, std::max<uint32_t>(2, walk));
+        auto bytes = [&] { return g.b_stages * b_bytes + g.raw * raw_bytes + SCALE_BYTES; };
+        while (bytes() > budget) {
+            if (g.raw > 4) --g.raw;
+            else if (g.b_stages > 4) --g.b_stages;
+            else if (g.raw > 2) --g.raw;
+            else --g.b_stages;
+        }
+        smem = bytes();
+    } else {
+        const uint32_t stage = b_bytes + g.bu * A_STEP_BYTES;
+        g.b_stages = std::min<uint32_t>(std::min<uint32_t>(kMaxStages, budget / stage), std::max<uint32_t>(2, walk));
+        smem = g.b_stages * stage;
     }
+    smem = std::max<size_t>(smem, (size_t)g.n_tile * BM * sizeof(float)) + 1024;  // at the end the f32 tile lies there
 
     for (int i = 0; i < count; ++i) {
         const MatmulArgs& ai = args[i];
-        UmmaParams& pi = g.p[i];
-        pi = p;
-        pi.w = static_cast<const uint8_t*>(ai.matrix);
+        UmmaProblem& pi = g.p[i];
         pi.scale = ai.scale;
         pi.table = ai.table;
         pi.M = ai.M;
@@ -666,37 +781,34 @@ cudaError_t matmul_umma_group(const MatmulArgs* args, int count, int32_t* status
         pi.act = ai.act;
         bool ok;
         if (a.kind == MAT_FP16)
-            ok = make_map_2d(&g.map_w[i], CU_TENSOR_MAP_DATA_TYPE_FLOAT16, ai.matrix, a.K, ai.M, (uint64_t)a.K * 2, BK, BM,
-                             CU_TENSOR_MAP_SWIZZLE_128B);
+            ok = make_operand_map(&g.map_w[i], ai.matrix, a.K, ai.M, (uint64_t)a.K * 2, BM, g.bu);
         else if (a.kind == MAT_INT8)
-            ok = make_map_2d(&g.map_w[i], CU_TENSOR_MAP_DATA_TYPE_UINT8, ai.matrix, a.K, ai.M, a.K, 64, BM, CU_TENSOR_MAP_SWIZZLE_NONE);
+            ok = make_map(&g.map_w[i], CU_TENSOR_MAP_DATA_TYPE_UINT8, ai.matrix, {a.K, ai.M}, {a.K}, {128, BM}, CU_TENSOR_MAP_SWIZZLE_128B);
         else
-            ok = make_map_2d(&g.map_w[i], CU_TENSOR_MAP_DATA_TYPE_UINT8, ai.matrix, a.K / 2, ai.M, a.K / 2, 32, BM,
-                             CU_TENSOR_MAP_SWIZZLE_NONE);
+            ok = make_map(&g.map_w[i], CU_TENSOR_MAP_DATA_TYPE_UINT8, ai.matrix, {a.K / 2, ai.M}, {a.K / 2}, {64, BM}, CU_TENSOR_MAP_SWIZZLE_64B);
         const __half* x0 = static_cast<const __half*>(ai.in.base) + ai.in.index(0, 0, 0);
-        ok = ok && make_map_2d(&g.map_x[i], CU_TENSOR_MAP_DATA_TYPE_FLOAT16, x0, a.K, a.N, (uint64_t)ai.in.stride[0] * 2, BK, p.n_tile,
-                               CU_TENSOR_MAP_SWIZZLE_128B);
+        ok = ok && make_operand_map(&g.map_x[i], x0, a.K, a.N, (uint64_t)ai.in.stride[0] * 2, g.n_tile, g.bu);
         if (!ok) return cudaErrorInvalidValue;
     }
 
     static SmemOptIn opt_in[3];
     auto kernel = a.kind == MAT_INT8 ? matmul_umma_kernel<MAT_INT8> : a.kind == MAT_NF4 ? matmul_umma_kernel<MAT_NF4> : matmul_umma_kernel<MAT_FP16>;
     if (cudaError_t e = opt_in[a.kind == MAT_INT8 ? 0 : a.kind == MAT_NF4 ? 1 : 2].ensure(kernel, 223 * 1024); e != cudaSuccess) return e;
-    dim3 grid(row_tiles, (a.N + p.n_tile - 1) / p.n_tile, p.splits);
-    size_t smem = (size_t)p.stages * stage_bytes + (size_t)p.raw * raw_bytes + 4 * SCALE_SLOT_BYTES + 1024;
-    smem = std::max<size_t>(smem, (size_t)p.n_tile * BM * sizeof(float) + 1024);  // the partial tile / the staged output tile
+    dim3 grid(row_tiles, (a.N + g.n_tile - 1) / g.n_tile, g.splits);
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = grid;
     cfg.blockDim = dim3(kUmmaThreads, 1, 1);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
+    cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = 1;
     attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = p.splits;
+    attr[0].val.clusterDim.z = g.splits;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = chained_launches() ? 2 : 1;
     return cudaLaunchKernelEx(&cfg, kernel, g);
 }
 

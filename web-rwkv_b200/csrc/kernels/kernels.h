@@ -26,6 +26,15 @@ struct SmemOptIn {
     }
 };
 
+// True while this thread issues the launches of a job (a chain whose every kernel waits for its predecessors before it
+// touches what they wrote): the launchers then ask for programmatic dependent launch.  launch.cuh has the rules.
+bool chained_launches();
+struct ChainedLaunches {  // scope guard
+    explicit ChainedLaunches(bool on);
+    ~ChainedLaunches();
+    const bool before;
+};
+
 // ---- quantizers (quant.cu) -------------------------------------------------------------
 cudaError_t quantize_int8(const __half* input, size_t len, __half* minmax, uint8_t* output, int num_sms,
                           cudaStream_t stream);
@@ -49,7 +58,7 @@ cudaError_t matmul(const MatmulArgs& a, int num_sms, cudaStream_t stream);
 // fp16 matrices with K <= 256 (the low-rank adapters' second matrices) at any token count (gemm_small.cu).
 bool matmul_small_supported(const MatmulArgs& a);
 cudaError_t matmul_small(const MatmulArgs& a, int num_sms, cudaStream_t stream);
-// Tensor-memory (tcgen05) GEMM for N >= 16 tokens (gemm_umma.cu).
+// Tensor-memory (tcgen05) GEMM for more than 8 tokens (gemm_umma.cu).
 bool matmul_umma_supported(const MatmulArgs& a);
 cudaError_t matmul_umma(const MatmulArgs& a, int32_t* status, cudaStream_t stream);
 // Up to four matrices of one weight format, K and token count (each with its own activations, output and activation

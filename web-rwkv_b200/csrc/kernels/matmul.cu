@@ -15,6 +15,7 @@
 // Fragment mapping (lane = 4*g + t): the MMA's k index is a permutation of the physical k, the same
 // for A and B: in k-step s lane t supplies physical elements 4s..4s+3 of its own 16-byte piece.
 #include "device.cuh"
+#include "launch.cuh"
 
 namespace wrk {
 namespace k {
@@ -112,6 +113,8 @@ __device__ __forceinline__ void stage_input(const MmParams& p, uint32_t n0, uint
 
 template <int KIND, int NT>
 __global__ void __launch_bounds__(kThreads) matmul_mma_kernel(const MmParams p) {
+    pdl_launch_dependents();
+    pdl_wait();
     extern __shared__ __align__(16) uint8_t smem[];
     __shared__ __half lut[16];
 
@@ -311,6 +314,8 @@ __global__ void __launch_bounds__(kThreads) matmul_mma_kernel(const MmParams p) 
 // per output element, the reference's arithmetic verbatim.  Correctness path only.
 __global__ void matmul_generic_kernel(int kind, const uint8_t* matrix, const __half* scale, const float* table,
                                       uint32_t K, uint32_t M, uint32_t N, uint32_t B, DView in, DView out, int act) {
+    pdl_launch_dependents();
+    pdl_wait();
     const size_t total = (size_t)M * N * B;
     for (size_t o = (size_t)blockIdx.x * blockDim.x + threadIdx.x; o < total; o += (size_t)gridDim.x * blockDim.x) {
         const uint32_t m = o % M, n = (o / M) % N, b = o / ((size_t)M * N);
@@ -341,7 +346,7 @@ cudaError_t launch_mma(const MmParams& p, uint32_t B, cudaStream_t stream) {
     static SmemOptIn opt_in;  // one per instantiation
     if (cudaError_t e = opt_in.ensure(matmul_mma_kernel<KIND, NT>, 160 * 1024); e != cudaSuccess) return e;
     dim3 grid((p.M + kRows - 1) / kRows, (p.N + 8 * NT - 1) / (8 * NT), B);
-    matmul_mma_kernel<KIND, NT><<<grid, kThreads, smem, stream>>>(p);
+    launch(matmul_mma_kernel<KIND, NT>, grid, dim3(kThreads), smem, stream, p);
     return cudaGetLastError();
 }
 
@@ -375,8 +380,7 @@ cudaError_t matmul(const MatmulArgs& a, int num_sms, cudaStream_t stream) {
     if (!aligned) {
         const size_t total = (size_t)a.M * a.N * a.B;
         const int grid = (int)std::min<size_t>((total + 127) / 128, (size_t)num_sms * 16);
-        matmul_generic_kernel<<<grid, 128, 0, stream>>>(a.kind, static_cast<const uint8_t*>(a.matrix), a.scale, a.table,
-                                                        a.K, a.M, a.N, a.B, a.in, a.out, a.act);
+        launch(matmul_generic_kernel, grid, dim3(128), 0, stream, a.kind, static_cast<const uint8_t*>(a.matrix), a.scale, a.table, a.K, a.M, a.N, a.B, a.in, a.out, a.act);
         return cudaGetLastError();
     }
     MmParams p;

@@ -4,6 +4,7 @@
 // point here as well.  They are latency-bound on the activations of a single job and are not
 // individually roofline-graded.
 #include "device.cuh"
+#include "launch.cuh"
 
 namespace wrk {
 namespace k {
@@ -38,6 +39,8 @@ constexpr int kLnRegs = 32;
 // With `delta`, src <- src + delta first (rounded to the data type, as the separate add stores it).
 __global__ void layer_norm_kernel(const __half* w, const __half* b, int dtype, const void* delta, void* src, void* x, uint32_t C,
                                   uint32_t rows, uint32_t wrows, float eps) {
+    pdl_launch_dependents();
+    pdl_wait();
     __shared__ float scratch[32];
     const bool cached = C <= (uint32_t)kLnRegs * blockDim.x;
     for (uint32_t row = blockIdx.x; row < rows; row += gridDim.x) {
@@ -95,6 +98,8 @@ __global__ void layer_norm_kernel(const __half* w, const __half* b, int dtype, c
 
 // normalize.wgsl l2_norm: x * rsqrt(sum x^2 + eps) per row of C.
 __global__ void l2_norm_kernel(int dtype, void* x, uint32_t C, uint32_t rows, float eps) {
+    pdl_launch_dependents();
+    pdl_wait();
     __shared__ float scratch[32];
     for (uint32_t row = blockIdx.x; row < rows; row += gridDim.x) {
         const size_t base = (size_t)row * C;
@@ -111,6 +116,8 @@ __global__ void l2_norm_kernel(int dtype, void* x, uint32_t C, uint32_t rows, fl
 
 // normalize.wgsl recenter: x - mean(x) per row of C.
 __global__ void recenter_kernel(int dtype, void* x, uint32_t C, uint32_t rows) {
+    pdl_launch_dependents();
+    pdl_wait();
     __shared__ float scratch[32];
     for (uint32_t row = blockIdx.x; row < rows; row += gridDim.x) {
         const size_t base = (size_t)row * C;
@@ -124,6 +131,8 @@ __global__ void recenter_kernel(int dtype, void* x, uint32_t C, uint32_t rows) {
 // normalize.wgsl rms_norm: fma(x * rsqrt(mean x^2 + eps), w, b) per row of C.
 __global__ void rms_norm_kernel(const __half* w, const __half* b, int dtype, void* x, uint32_t C, uint32_t rows,
                                 float eps) {
+    pdl_launch_dependents();
+    pdl_wait();
     __shared__ float scratch[32];
     for (uint32_t row = blockIdx.x; row < rows; row += gridDim.x) {
         const size_t base = (size_t)row * C;
@@ -141,6 +150,8 @@ __global__ void rms_norm_kernel(const __half* w, const __half* b, int dtype, voi
 // embed.wgsl: output[:, t, b] = input[:, tokens[t, b]] (fp16 rows of the embedding matrix, widened if the output is f32).
 __global__ void embed_kernel(const uint32_t* tokens, const __half* input, int dtype, void* output, uint32_t C,
                              uint32_t rows, uint32_t vocab, int32_t* status) {
+    pdl_launch_dependents();
+    pdl_wait();
     for (uint32_t row = blockIdx.x; row < rows; row += gridDim.x) {
         const uint32_t tok = tokens[row];
         if (tok >= vocab) {  // the reference reads out of bounds here; report instead
@@ -154,6 +165,8 @@ __global__ void embed_kernel(const uint32_t* tokens, const __half* input, int dt
 
 // reshape.wgsl broadcast: output[c, t, b] = input[c, t % in.T, b % in.B].
 __global__ void broadcast_kernel(DView in, DView out) {
+    pdl_launch_dependents();
+    pdl_wait();
     const uint32_t C = out.shape[0], T = out.shape[1], B = out.shape[2];
     const size_t total = (size_t)C * T * B;
     for (size_t o = (size_t)blockIdx.x * blockDim.x + threadIdx.x; o < total; o += (size_t)gridDim.x * blockDim.x) {
@@ -165,6 +178,8 @@ __global__ void broadcast_kernel(DView in, DView out) {
 
 // blend.wgsl: output = factor[0] * input + factor[1] * output.
 __global__ void blend_kernel(const float* factor, DView in, DView out) {
+    pdl_launch_dependents();
+    pdl_wait();
     const uint32_t C = out.shape[0], T = out.shape[1], B = out.shape[2];
     const size_t total = (size_t)C * T * B;
     const float fx = factor[0], fy = factor[1];
@@ -180,6 +195,8 @@ __global__ void blend_kernel(const float* factor, DView in, DView out) {
 // tensors, f32 sum over the common rank K.  One warp per 32 consecutive m of one n: lanes read xa rows, xb's row of K
 // is shared by the warp.
 __global__ void blend_lora_kernel(const float* factor, DView xa, DView xb, DView out, uint32_t K) {
+    pdl_launch_dependents();
+    pdl_wait();
     const uint32_t M = out.shape[0], N = out.shape[1], B = out.shape[2];
     const size_t total = (size_t)M * N * B;
     const float fx = factor[0], fy = factor[1];
@@ -196,6 +213,8 @@ __global__ void blend_lora_kernel(const float* factor, DView xa, DView xb, DView
 
 // softmax.wgsl: x <- exp(x - max) / sum exp(x - max) per row of C (two reductions, then the write).
 __global__ void softmax_kernel(int dtype, void* x, uint32_t C, uint32_t rows) {
+    pdl_launch_dependents();
+    pdl_wait();
     __shared__ float scratch[32];
     for (uint32_t row = blockIdx.x; row < rows; row += gridDim.x) {
         const size_t base = (size_t)row * C;
@@ -222,6 +241,8 @@ __global__ void softmax_kernel(int dtype, void* x, uint32_t C, uint32_t rows) {
 // previous token of the same sequence or, at the sequence's first token of the job, the carry row.
 __global__ void token_shift_kernel(const uint32_t* cursors, int wide, DView tm, DView state, DView in, DView out,
                                    int reversed) {
+    pdl_launch_dependents();
+    pdl_wait();
     const uint32_t C = out.shape[0], T = out.shape[1], Z = out.shape[2];
     const size_t total = (size_t)C * T * Z;
     for (size_t o = (size_t)blockIdx.x * blockDim.x + threadIdx.x; o < total; o += (size_t)gridDim.x * blockDim.x) {
@@ -239,6 +260,8 @@ __global__ void token_shift_kernel(const uint32_t* cursors, int wide, DView tm, 
 // Several token shifts of one input in one launch: out_i[c, t] = mix(x_t, prev, f_i[c]) as token_shift_kernel computes it,
 // with the input and the previous row read once.
 __global__ void token_shift_multi_kernel(const ShiftMultiArgs a) {
+    pdl_launch_dependents();
+    pdl_wait();
     const size_t total = (size_t)a.C * a.T;
     for (size_t o = (size_t)blockIdx.x * blockDim.x + threadIdx.x; o < total; o += (size_t)gridDim.x * blockDim.x) {
         const uint32_t c = o % a.C, t = o / a.C;
@@ -261,6 +284,8 @@ __global__ void token_shift_multi_kernel(const ShiftMultiArgs a) {
 //   k  <- k * (1 + (a - 1) * k_a)  (control_k_kernel),  n[.., 0..3] <- k, v, a, kk  (four blits).
 // Sums run in l2_norm_kernel's order for a block of 32 threads, so the results are bit-identical to the separate ops.
 __global__ void pack_v7_kernel(const PackV7Args p) {
+    pdl_launch_dependents();
+    pdl_wait();
     const uint32_t lane = threadIdx.x;
     const size_t plane = (size_t)p.rows * p.S;
     for (uint32_t row = blockIdx.x; row < p.rows; row += gridDim.x) {
@@ -291,6 +316,8 @@ __global__ void pack_v7_kernel(const PackV7Args p) {
 // channel_mix.wgsl: carry row <- x_in at the sequence's last token; x = sigmoid(r) * v (v7: x = v).
 __global__ void channel_mix_kernel(const uint32_t* cursors, int wide, DView state, int dtype, const void* r,
                                    const void* v, void* x, uint32_t C, uint32_t T, int v7) {
+    pdl_launch_dependents();
+    pdl_wait();
     const size_t total = (size_t)C * T;
     for (size_t o = (size_t)blockIdx.x * blockDim.x + threadIdx.x; o < total; o += (size_t)gridDim.x * blockDim.x) {
         const uint32_t c = o % C, t = o / C;
@@ -309,6 +336,8 @@ __global__ void channel_mix_kernel(const uint32_t* cursors, int wide, DView stat
 // The shift row of every sequence that has tokens in the job <- x at the sequence's last token (what the time-mix
 // and channel-mix ops do for their own channels, as an op of its own).
 __global__ void shift_carry_kernel(const uint32_t* cursors, int wide, DView state, int dtype, const void* x, uint32_t C, uint32_t T) {
+    pdl_launch_dependents();
+    pdl_wait();
     const size_t total = (size_t)C * T;
     for (size_t o = (size_t)blockIdx.x * blockDim.x + threadIdx.x; o < total; o += (size_t)gridDim.x * blockDim.x) {
         const uint32_t c = o % C, t = o / C;
@@ -318,6 +347,8 @@ __global__ void shift_carry_kernel(const uint32_t* cursors, int wide, DView stat
 }
 
 __global__ void binary_kernel(int is_mul, DView in, DView out, int act_x, int act_y, int act_out) {
+    pdl_launch_dependents();
+    pdl_wait();
     const uint32_t C = out.shape[0], T = out.shape[1], B = out.shape[2];
     const size_t total = (size_t)C * T * B;
     for (size_t o = (size_t)blockIdx.x * blockDim.x + threadIdx.x; o < total; o += (size_t)gridDim.x * blockDim.x) {
@@ -330,6 +361,8 @@ __global__ void binary_kernel(int is_mul, DView in, DView out, int act_x, int ac
 }
 
 __global__ void activate_kernel(DView x, int act) {
+    pdl_launch_dependents();
+    pdl_wait();
     const uint32_t C = x.shape[0], T = x.shape[1], B = x.shape[2];
     const size_t total = (size_t)C * T * B;
     for (size_t o = (size_t)blockIdx.x * blockDim.x + threadIdx.x; o < total; o += (size_t)gridDim.x * blockDim.x) {
@@ -340,6 +373,8 @@ __global__ void activate_kernel(DView x, int act) {
 }
 
 __global__ void blit_kernel(DView in, DView out, int transpose) {
+    pdl_launch_dependents();
+    pdl_wait();
     const uint32_t C = in.shape[0], T = in.shape[1], B = in.shape[2];
     const size_t total = (size_t)C * T * B;
     for (size_t o = (size_t)blockIdx.x * blockDim.x + threadIdx.x; o < total; o += (size_t)gridDim.x * blockDim.x) {
@@ -350,6 +385,8 @@ __global__ void blit_kernel(DView in, DView out, int transpose) {
 }
 
 __global__ void lerp_kernel(DView in, DView out, DView f, int reversed) {
+    pdl_launch_dependents();
+    pdl_wait();
     const uint32_t C = out.shape[0], T = out.shape[1], B = out.shape[2];
     const size_t total = (size_t)C * T * B;
     for (size_t o = (size_t)blockIdx.x * blockDim.x + threadIdx.x; o < total; o += (size_t)gridDim.x * blockDim.x) {
@@ -364,11 +401,15 @@ __global__ void lerp_kernel(DView in, DView out, DView f, int reversed) {
 }
 
 __global__ void affine_kernel(int dtype, void* x, size_t len, float scale, float bias) {
+    pdl_launch_dependents();
+    pdl_wait();
     for (size_t o = (size_t)blockIdx.x * blockDim.x + threadIdx.x; o < len; o += (size_t)gridDim.x * blockDim.x)
         dstore(x, dtype, o, scale * dload(x, dtype, o) + bias);
 }
 
 __global__ void control_k_kernel(const __half* p, DView a, DView k) {
+    pdl_launch_dependents();
+    pdl_wait();
     const uint32_t C = k.shape[0], T = k.shape[1], B = k.shape[2];
     const size_t total = (size_t)C * T * B;
     for (size_t o = (size_t)blockIdx.x * blockDim.x + threadIdx.x; o < total; o += (size_t)gridDim.x * blockDim.x) {
@@ -394,7 +435,7 @@ cudaError_t layer_norm_copy(const __half* w, const __half* b, int dtype, const v
     if (layer_norm_vec(w, b, dtype, delta, src, x, C, rows, wrows, eps, stream)) return cudaGetLastError();
     const int block = C <= 256 ? 32 : 256;
     const uint32_t grid = rows < 148u * 32u ? rows : 148u * 32u;
-    layer_norm_kernel<<<grid, block, 0, stream>>>(w, b, dtype, delta, src, x, C, rows, wrows, eps);
+    launch(layer_norm_kernel, grid, dim3(block), 0, stream, w, b, dtype, delta, src, x, C, rows, wrows, eps);
     return cudaGetLastError();
 }
 
@@ -402,7 +443,7 @@ cudaError_t l2_norm(int dtype, void* x, uint32_t C, uint32_t rows, float eps, cu
     if (rows == 0 || C == 0) return cudaSuccess;
     const int block = C <= 256 ? 32 : 256;
     const uint32_t grid = rows < 148u * 32u ? rows : 148u * 32u;
-    l2_norm_kernel<<<grid, block, 0, stream>>>(dtype, x, C, rows, eps);
+    launch(l2_norm_kernel, grid, dim3(block), 0, stream, dtype, x, C, rows, eps);
     return cudaGetLastError();
 }
 
@@ -410,7 +451,7 @@ cudaError_t softmax(int dtype, void* x, uint32_t C, uint32_t rows, cudaStream_t 
     if (rows == 0 || C == 0) return cudaSuccess;
     const int block = C <= 256 ? 32 : C <= 4096 ? 256 : 1024;
     const uint32_t grid = rows < 148u * 32u ? rows : 148u * 32u;
-    softmax_kernel<<<grid, block, 0, stream>>>(dtype, x, C, rows);
+    launch(softmax_kernel, grid, dim3(block), 0, stream, dtype, x, C, rows);
     return cudaGetLastError();
 }
 
@@ -418,7 +459,7 @@ cudaError_t recenter(int dtype, void* x, uint32_t C, uint32_t rows, cudaStream_t
     if (rows == 0 || C == 0) return cudaSuccess;
     const int block = C <= 256 ? 32 : 256;
     const uint32_t grid = rows < 148u * 32u ? rows : 148u * 32u;
-    recenter_kernel<<<grid, block, 0, stream>>>(dtype, x, C, rows);
+    launch(recenter_kernel, grid, dim3(block), 0, stream, dtype, x, C, rows);
     return cudaGetLastError();
 }
 
@@ -427,7 +468,7 @@ cudaError_t rms_norm(const __half* w, const __half* b, int dtype, void* x, uint3
     if (rows == 0 || C == 0) return cudaSuccess;
     const int block = C <= 256 ? 32 : 256;
     const uint32_t grid = rows < 148u * 32u ? rows : 148u * 32u;
-    rms_norm_kernel<<<grid, block, 0, stream>>>(w, b, dtype, x, C, rows, eps);
+    launch(rms_norm_kernel, grid, dim3(block), 0, stream, w, b, dtype, x, C, rows, eps);
     return cudaGetLastError();
 }
 
@@ -435,28 +476,28 @@ cudaError_t embed(const uint32_t* tokens, const __half* input, int dtype, void* 
                   uint32_t vocab, int32_t* status, cudaStream_t stream) {
     if (rows == 0 || C == 0) return cudaSuccess;
     const uint32_t grid = rows < 148u * 32u ? rows : 148u * 32u;
-    embed_kernel<<<grid, 256, 0, stream>>>(tokens, input, dtype, output, C, rows, vocab, status);
+    launch(embed_kernel, grid, dim3(256), 0, stream, tokens, input, dtype, output, C, rows, vocab, status);
     return cudaGetLastError();
 }
 
 cudaError_t broadcast(DView input, DView output, cudaStream_t stream) {
     const size_t total = (size_t)output.shape[0] * output.shape[1] * output.shape[2];
     if (total == 0) return cudaSuccess;
-    broadcast_kernel<<<ew_grid(total), kEw, 0, stream>>>(input, output);
+    launch(broadcast_kernel, dim3(ew_grid(total)), dim3(kEw), 0, stream, input, output);
     return cudaGetLastError();
 }
 
 cudaError_t blend(const float* factor, DView input, DView output, cudaStream_t stream) {
     const size_t total = (size_t)output.shape[0] * output.shape[1] * output.shape[2];
     if (total == 0) return cudaSuccess;
-    blend_kernel<<<ew_grid(total), kEw, 0, stream>>>(factor, input, output);
+    launch(blend_kernel, dim3(ew_grid(total)), dim3(kEw), 0, stream, factor, input, output);
     return cudaGetLastError();
 }
 
 cudaError_t blend_lora(const float* factor, DView xa, DView xb, DView output, uint32_t K, cudaStream_t stream) {
     const size_t total = (size_t)output.shape[0] * output.shape[1] * output.shape[2];
     if (total == 0) return cudaSuccess;
-    blend_lora_kernel<<<ew_grid(total), kEw, 0, stream>>>(factor, xa, xb, output, K);
+    launch(blend_lora_kernel, dim3(ew_grid(total)), dim3(kEw), 0, stream, factor, xa, xb, output, K);
     return cudaGetLastError();
 }
 
@@ -465,7 +506,7 @@ cudaError_t token_shift(const uint32_t* cursors, int wide, DView time_mix, DView
     const size_t total = (size_t)output.shape[0] * output.shape[1] * output.shape[2];
     if (total == 0) return cudaSuccess;
     if (token_shift_vec(cursors, wide, time_mix, nullptr, state, input, output, reversed, stream)) return cudaGetLastError();
-    token_shift_kernel<<<ew_grid(total), kEw, 0, stream>>>(cursors, wide, time_mix, state, input, output, reversed);
+    launch(token_shift_kernel, dim3(ew_grid(total)), dim3(kEw), 0, stream, cursors, wide, time_mix, state, input, output, reversed);
     return cudaGetLastError();
 }
 
@@ -473,14 +514,14 @@ cudaError_t token_shift_multi(const ShiftMultiArgs& a, cudaStream_t stream) {
     const size_t total = (size_t)a.C * a.T;
     if (total == 0 || a.count == 0) return cudaSuccess;
     if (token_shift_multi_vec(a, stream)) return cudaGetLastError();
-    token_shift_multi_kernel<<<ew_grid(total), kEw, 0, stream>>>(a);
+    launch(token_shift_multi_kernel, dim3(ew_grid(total)), dim3(kEw), 0, stream, a);
     return cudaGetLastError();
 }
 
 cudaError_t pack_v7(const PackV7Args& p, cudaStream_t stream) {
     if (p.rows == 0 || p.S == 0) return cudaSuccess;
     const uint32_t grid = p.rows < 148u * 32u ? p.rows : 148u * 32u;
-    pack_v7_kernel<<<grid, 32, 0, stream>>>(p);
+    launch(pack_v7_kernel, grid, dim3(32), 0, stream, p);
     return cudaGetLastError();
 }
 
@@ -488,7 +529,7 @@ cudaError_t shift_carry(const uint32_t* cursors, int wide, DView state, int dtyp
                         cudaStream_t stream) {
     const size_t total = (size_t)C * T;
     if (total == 0) return cudaSuccess;
-    shift_carry_kernel<<<ew_grid(total), kEw, 0, stream>>>(cursors, wide, state, dtype, x, C, T);
+    launch(shift_carry_kernel, dim3(ew_grid(total)), dim3(kEw), 0, stream, cursors, wide, state, dtype, x, C, T);
     return cudaGetLastError();
 }
 
@@ -497,7 +538,7 @@ cudaError_t channel_mix(const uint32_t* cursors, int wide, DView state, int dtyp
     const size_t total = (size_t)C * T;
     if (total == 0) return cudaSuccess;
     if (channel_mix_vec(cursors, wide, state, dtype, r, v, x, nullptr, C, T, v7, stream)) return cudaGetLastError();
-    channel_mix_kernel<<<ew_grid(total), kEw, 0, stream>>>(cursors, wide, state, dtype, r, v, x, C, T, v7);
+    launch(channel_mix_kernel, dim3(ew_grid(total)), dim3(kEw), 0, stream, cursors, wide, state, dtype, r, v, x, C, T, v7);
     return cudaGetLastError();
 }
 
@@ -505,7 +546,7 @@ cudaError_t binary(int is_mul, DView input, DView output, int act_x, int act_y, 
     const size_t total = (size_t)output.shape[0] * output.shape[1] * output.shape[2];
     if (total == 0) return cudaSuccess;
     if (binary_vec(is_mul, input, output, act_x, act_y, act_out, stream)) return cudaGetLastError();
-    binary_kernel<<<ew_grid(total), kEw, 0, stream>>>(is_mul, input, output, act_x, act_y, act_out);
+    launch(binary_kernel, dim3(ew_grid(total)), dim3(kEw), 0, stream, is_mul, input, output, act_x, act_y, act_out);
     return cudaGetLastError();
 }
 
@@ -513,7 +554,7 @@ cudaError_t activate(DView x, int act, cudaStream_t stream) {
     const size_t total = (size_t)x.shape[0] * x.shape[1] * x.shape[2];
     if (total == 0) return cudaSuccess;
     if (activate_vec(x, act, stream)) return cudaGetLastError();
-    activate_kernel<<<ew_grid(total), kEw, 0, stream>>>(x, act);
+    launch(activate_kernel, dim3(ew_grid(total)), dim3(kEw), 0, stream, x, act);
     return cudaGetLastError();
 }
 
@@ -521,27 +562,27 @@ cudaError_t blit(DView input, DView output, int transpose, cudaStream_t stream) 
     const size_t total = (size_t)input.shape[0] * input.shape[1] * input.shape[2];
     if (total == 0) return cudaSuccess;
     if (!transpose && blit_vec(input, output, stream)) return cudaGetLastError();
-    blit_kernel<<<ew_grid(total), kEw, 0, stream>>>(input, output, transpose);
+    launch(blit_kernel, dim3(ew_grid(total)), dim3(kEw), 0, stream, input, output, transpose);
     return cudaGetLastError();
 }
 
 cudaError_t lerp(DView input, DView output, DView factor, int reversed, cudaStream_t stream) {
     const size_t total = (size_t)output.shape[0] * output.shape[1] * output.shape[2];
     if (total == 0) return cudaSuccess;
-    lerp_kernel<<<ew_grid(total), kEw, 0, stream>>>(input, output, factor, reversed);
+    launch(lerp_kernel, dim3(ew_grid(total)), dim3(kEw), 0, stream, input, output, factor, reversed);
     return cudaGetLastError();
 }
 
 cudaError_t affine(int dtype, void* x, size_t len, float scale, float bias, cudaStream_t stream) {
     if (len == 0) return cudaSuccess;
-    affine_kernel<<<ew_grid(len), kEw, 0, stream>>>(dtype, x, len, scale, bias);
+    launch(affine_kernel, dim3(ew_grid(len)), dim3(kEw), 0, stream, dtype, x, len, scale, bias);
     return cudaGetLastError();
 }
 
 cudaError_t control_k_v7(const __half* p, DView a, DView k, cudaStream_t stream) {
     const size_t total = (size_t)k.shape[0] * k.shape[1] * k.shape[2];
     if (total == 0) return cudaSuccess;
-    control_k_kernel<<<ew_grid(total), kEw, 0, stream>>>(p, a, k);
+    launch(control_k_kernel, dim3(ew_grid(total)), dim3(kEw), 0, stream, p, a, k);
     return cudaGetLastError();
 }
 

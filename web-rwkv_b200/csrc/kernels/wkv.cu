@@ -12,6 +12,7 @@
 // State layout (reference: src/runtime/v6.rs:187-197): f32 view [C, S+1, B]; row 0 = token-shift
 // carry, row 1+i = key index i for all heads side by side (column h*S + j = value index j).
 #include "device.cuh"
+#include "launch.cuh"
 
 namespace wrk {
 namespace k {
@@ -64,6 +65,8 @@ __device__ __forceinline__ bool find_run(const uint32_t* cursors, int wide, uint
 // while the current chunk is computed (one barrier per chunk), so a token's step never waits for global memory.
 template <int S, int CW>
 __global__ void __launch_bounds__((S / 4) * (S / CW)) time_mix_v56_kernel(const WkvArgs a) {
+    pdl_launch_dependents();
+    pdl_wait();
     constexpr int RG = S / 4, NT = RG * (S / CW), CGW = 32 / RG, TC = S <= 64 ? 16 : 4, PI = (4 * S + NT - 1) / NT;
     static_assert(CW == 2 || CW == 4, "columns per thread");
     static_assert(RG == 8 || RG == 16 || RG == 32, "the row groups of a column group are lanes of one warp");
@@ -202,6 +205,8 @@ constexpr int kQtStride = 20;  // row stride of Qt in floats: 16-byte rows whose
 constexpr size_t kChunkedSmemFloats = 2 * 4 * kBlockTokens * 64 + 64 * kQtStride + kBlockTokens * 64 + kBlockTokens * kBlockTokens + 64 +
                                       64 * 64 + 4 * kBlockTokens * 64;
 __global__ void __launch_bounds__(256) time_mix_v56_chunked_kernel(const WkvArgs a) {
+    pdl_launch_dependents();
+    pdl_wait();
     constexpr int S = 64, L = kBlockTokens;
     enum { IN_K = 0, IN_R = 1, IN_W = 2, IN_V = 3 };
     extern __shared__ __align__(16) float wkv_smem[];
@@ -407,6 +412,8 @@ __global__ void __launch_bounds__(256) time_mix_v56_chunked_kernel(const WkvArgs
 // barrier per chunk.
 template <int S, int G>
 __global__ void __launch_bounds__((1 + G) * S) time_mix_v7_kernel(const WkvArgs a) {
+    pdl_launch_dependents();
+    pdl_wait();
     static_assert(G == 1 || G == 3, "three pairs of rows over the loader groups");
     constexpr int TC = 768 / S, P = 3 / G;
     enum { IN_R = 0, IN_W = 1, IN_K = 2, IN_V = 3, IN_A = 4, IN_B = 5 };
@@ -530,6 +537,8 @@ __global__ void __launch_bounds__((1 + G) * S) time_mix_v7_kernel(const WkvArgs 
 // them on an SM where the staged kernel above fits one.
 template <int S>
 __global__ void __launch_bounds__(S) time_mix_v7_short_kernel(const WkvArgs a) {
+    pdl_launch_dependents();
+    pdl_wait();
     __shared__ float sr[2][S], sw[2][S], sk[2][S], sa[2][S], sb[2][S];
     __shared__ RunScratch run;
     const uint32_t h = blockIdx.x, slot = blockIdx.y, j = threadIdx.x;
@@ -611,6 +620,8 @@ __global__ void __launch_bounds__(S) time_mix_v7_short_kernel(const WkvArgs a) {
 // x_j += (sum_i u_i k_i r_i) * v_j per (token, head): one warp per (token, head).
 __global__ void time_first_v7_kernel(const __half* u, int dtype, const void* r, const void* n, void* x, uint32_t S,
                                      uint32_t H, uint32_t T) {
+    pdl_launch_dependents();
+    pdl_wait();
     const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
     if (warp >= T * H) return;
     const uint32_t t = warp / H, h = warp % H;
@@ -630,9 +641,9 @@ cudaError_t time_mix_v56(const WkvArgs& a, cudaStream_t stream) {
     if (a.T == 0 || a.B == 0) return cudaSuccess;
     dim3 grid(a.H, a.B);
     switch (a.S) {
-        case 32: time_mix_v56_kernel<32, 4><<<grid, 64, 0, stream>>>(a); break;
-        case 64: time_mix_v56_kernel<64, 4><<<grid, 256, 0, stream>>>(a); break;
-        case 128: time_mix_v56_kernel<128, 4><<<grid, 1024, 0, stream>>>(a); break;
+        case 32: launch(time_mix_v56_kernel<32, 4>, grid, dim3(64), 0, stream, a); break;
+        case 64: launch(time_mix_v56_kernel<64, 4>, grid, dim3(256), 0, stream, a); break;
+        case 128: launch(time_mix_v56_kernel<128, 4>, grid, dim3(1024), 0, stream, a); break;
         default: return cudaErrorInvalidValue;
     }
     return cudaGetLastError();
@@ -647,7 +658,7 @@ cudaError_t time_mix_v56_chunked(const WkvArgs& a, cudaStream_t stream) {
     static SmemOptIn opt_in;
     const size_t smem = kChunkedSmemFloats * sizeof(float);
     if (cudaError_t e = opt_in.ensure(time_mix_v56_chunked_kernel, (int)smem); e != cudaSuccess) return e;
-    time_mix_v56_chunked_kernel<<<dim3(a.H, a.B), 256, smem, stream>>>(a);
+    launch(time_mix_v56_chunked_kernel, dim3(a.H, a.B), dim3(256), smem, stream, a);
     return cudaGetLastError();
 }
 
@@ -656,17 +667,17 @@ cudaError_t time_mix_v7(const WkvArgs& a, cudaStream_t stream) {
     dim3 grid(a.H, a.B);
     if (a.T <= 4 * a.B) {  // at most four tokens per sequence on average
         switch (a.S) {
-            case 32: time_mix_v7_short_kernel<32><<<grid, 32, 0, stream>>>(a); break;
-            case 64: time_mix_v7_short_kernel<64><<<grid, 64, 0, stream>>>(a); break;
-            case 128: time_mix_v7_short_kernel<128><<<grid, 128, 0, stream>>>(a); break;
+            case 32: launch(time_mix_v7_short_kernel<32>, grid, dim3(32), 0, stream, a); break;
+            case 64: launch(time_mix_v7_short_kernel<64>, grid, dim3(64), 0, stream, a); break;
+            case 128: launch(time_mix_v7_short_kernel<128>, grid, dim3(128), 0, stream, a); break;
             default: return cudaErrorInvalidValue;
         }
         return cudaGetLastError();
     }
     switch (a.S) {
-        case 32: time_mix_v7_kernel<32, 3><<<grid, 128, 0, stream>>>(a); break;
-        case 64: time_mix_v7_kernel<64, 3><<<grid, 256, 0, stream>>>(a); break;
-        case 128: time_mix_v7_kernel<128, 1><<<grid, 256, 0, stream>>>(a); break;
+        case 32: launch(time_mix_v7_kernel<32, 3>, grid, dim3(128), 0, stream, a); break;
+        case 64: launch(time_mix_v7_kernel<64, 3>, grid, dim3(256), 0, stream, a); break;
+        case 128: launch(time_mix_v7_kernel<128, 1>, grid, dim3(256), 0, stream, a); break;
         default: return cudaErrorInvalidValue;
     }
     return cudaGetLastError();
@@ -680,6 +691,8 @@ cudaError_t time_mix_v7(const WkvArgs& a, cudaStream_t stream) {
 __global__ void time_mix_v4_kernel(const uint32_t* cursors, int wide, const float* time_decay, const float* time_first,
                                    DView state, int dtype, const void* k, const void* v, const void* r, void* x,
                                    uint32_t C, uint32_t T) {
+    pdl_launch_dependents();
+    pdl_wait();
     const uint32_t c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= C) return;
     const float u = time_first[c], w = time_decay[c];
@@ -729,8 +742,7 @@ cudaError_t time_mix_v4(const uint32_t* cursors, int wide, const float* time_dec
                         int dtype, const void* k, const void* v, const void* r, void* x, uint32_t C, uint32_t T,
                         cudaStream_t stream) {
     if (T == 0 || C == 0) return cudaSuccess;
-    time_mix_v4_kernel<<<(C + 127) / 128, 128, 0, stream>>>(cursors, wide, time_decay, time_first, state, dtype, k, v, r, x,
-                                                            C, T);
+    launch(time_mix_v4_kernel, dim3((C + 127) / 128), dim3(128), 0, stream, cursors, wide, time_decay, time_first, state, dtype, k, v, r, x, C, T);
     return cudaGetLastError();
 }
 
@@ -739,7 +751,7 @@ cudaError_t time_first_v7(const __half* u, int dtype, const void* r, const void*
     if (T == 0) return cudaSuccess;
     const uint32_t warps = T * H;
     const uint32_t blocks = (warps * 32 + 255) / 256;
-    time_first_v7_kernel<<<blocks, 256, 0, stream>>>(u, dtype, r, n, x, S, H, T);
+    launch(time_first_v7_kernel, dim3(blocks), dim3(256), 0, stream, u, dtype, r, n, x, S, H, T);
     return cudaGetLastError();
 }
 

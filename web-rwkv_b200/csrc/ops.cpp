@@ -33,6 +33,12 @@ int32_t check_cursors(const wrk_tensor* cursors, uint32_t T) {
         for (auto q : _p) WRK_REQUIRE(q, WRK_ERR_INVALID_ARGUMENT, "null argument");     \
     } while (0)
 
+// The weights of a matmul, which its kernel fetches before it waits for the kernels in front of it.
+void add_early(wrk_op* op, std::initializer_list<const wrk_tensor*> weights) {
+    for (const wrk_tensor* t : weights)
+        if (t != nullptr) op->early.push_back(t->buf.get());
+}
+
 // Checks the operands of out = act(W x) and fills the kernels' argument block.
 int32_t matmul_args(int kind, wrk_tensor* matrix, wrk_tensor* scale, wrk_tensor* quant, const wrk_view* input,
                     const wrk_view* output, int32_t act, k::MatmulArgs* args) {
@@ -130,11 +136,13 @@ int32_t matmul_common(const char* name, int kind, wrk_tensor* matrix, wrk_tensor
             *out = new_atom(name, [f, sms](cudaStream_t s) { return k::fused_gemv(f, sms, s); },
                             {matrix, scale, quant, input->tensor, output->tensor, tt});
             wrk_tensor_release(tt);  // the atom keeps the buffer alive
+            add_early(*out, {matrix, scale, quant});
             return WRK_OK;
         }
     }
     *out = new_atom(name, [a, sms](cudaStream_t s) { return k::matmul(a, sms, s); },
                     {matrix, scale, quant, input->tensor, output->tensor});
+    add_early(*out, {matrix, scale, quant});
     return WRK_OK;
 }
 
@@ -1151,6 +1159,7 @@ int32_t wrk_matrix_matmul_group_op(wrk_matrix* const* matrices, const wrk_view* 
         for (uint32_t i = 0; i < count; ++i) {
             for (wrk_tensor* t : {matrices[i]->w, matrices[i]->m, matrices[i]->q, inputs[i].tensor, outputs[i].tensor})
                 if (t != nullptr && t->buf) op->keep.push_back(t->buf);
+            add_early(op, {matrices[i]->w, matrices[i]->m, matrices[i]->q});
         }
         *out = op;
         return WRK_OK;
