@@ -131,7 +131,29 @@ def test_v6_long_runs_cross_chunks(wrk, ctx):
     assert_close(gs, rs, "state")
 
 
-def _v7_case(wrk, ctx, H, seqs, B, wide, dtype=np.float16, seed=0, S=S):
+@pytest.mark.parametrize("head_size", [32, 64, 128])
+@pytest.mark.parametrize("alias", ["k", "r", "v"])
+def test_v6_output_over_an_input(wrk, ctx, head_size, alias):
+    """The outputs may replace k, r or v: heads are then not shared out among CTAs where every CTA reads that input.
+    Runs around the four tokens that are summed together and the 8 or 16 of a chunk."""
+    rng = np.random.default_rng(70 + head_size)
+    H, B, S, seqs = 3, 6, head_size, [(0, 3), (1, 4), (2, 5), (3, 15), (4, 16), (5, 33)]
+    cursors, T = _cursors(seqs, True)
+    t = {n: (rng.standard_normal((T, H, S)) * 0.5).astype(np.float32) for n in ("k", "v", "r")}
+    w = np.exp(-np.exp(rng.uniform(-6, 1, (T, H, S)))).astype(np.float32)
+    u = rng.uniform(-1, 1, (H, S)).astype(np.float32)
+    state = (rng.standard_normal((B, S + 2, S * H)) * 0.1).astype(np.float32)
+    dev = {n: ctx.from_numpy(v) for n, v in t.items()}
+    t_state = ctx.from_numpy(state)
+    ctx.run(wrk.time_mix_v6(ctx.from_numpy(cursors), ctx.from_numpy(w), ctx.from_numpy(u), t_state.view(y=(0, S + 1)), dev["k"], dev["v"],
+                            dev["r"], dev[alias]))
+    ref_x, ref_state = t[alias].copy(), state.copy()
+    oracle.time_mix_v56(True, cursors, w, u, oracle.View(ref_state, y=(0, S + 1)), t["k"], t["v"], t["r"], ref_x, S, H)
+    assert_close(dev[alias].numpy().reshape(T, H, S), ref_x, "x")
+    assert_close(t_state.numpy().reshape(ref_state.shape), ref_state, "state")
+
+
+def _v7_case(wrk, ctx, H, seqs, B, wide, dtype=np.float16, seed=0, S=S, over_r=False):
     rng = np.random.default_rng(seed)
     C = S * H
     cursors, T = _cursors(seqs, wide)
@@ -143,11 +165,11 @@ def _v7_case(wrk, ctx, H, seqs, B, wide, dtype=np.float16, seed=0, S=S):
     kk = rng.standard_normal((T, H, S)).astype(np.float32)
     kk /= np.linalg.norm(kk, axis=-1, keepdims=True)  # the model L2-normalises kk per head
     n = np.stack([k, v, a, kk]).astype(dtype)
-    x = rng.standard_normal((T, H, S)).astype(dtype)
+    x = r.copy() if over_r else rng.standard_normal((T, H, S)).astype(dtype)
     state = (rng.standard_normal((B, S + 2, C)) * 0.1).astype(np.float32)
 
     t_state, t_x = ctx.from_numpy(state), ctx.from_numpy(x)
-    op = wrk.time_mix_v7(ctx.from_numpy(cursors), t_state.view(y=(0, S + 1)), ctx.from_numpy(r), ctx.from_numpy(w),
+    op = wrk.time_mix_v7(ctx.from_numpy(cursors), t_state.view(y=(0, S + 1)), t_x if over_r else ctx.from_numpy(r), ctx.from_numpy(w),
                          ctx.from_numpy(n), t_x)
     ctx.run(op)
     got_x, got_state = t_x.numpy().reshape(T, H, S), t_state.numpy().reshape(B, S + 2, C)
@@ -168,6 +190,16 @@ def test_v7_multi_sequence(wrk, ctx, wide, dtype):
 @pytest.mark.parametrize("head_size", [32, 128])
 def test_v7_other_head_sizes(wrk, ctx, head_size):
     gx, gs, rx, rs = _v7_case(wrk, ctx, 3, [(0, 29), (1, 24), (2, 1)], 3, True, seed=50 + head_size, S=head_size)
+    assert_close(gx, rx, "x")
+    assert_close(gs, rs, "state")
+
+
+@pytest.mark.parametrize("head_size", [32, 64, 128])
+@pytest.mark.parametrize("over_r", [False, True])
+def test_v7_runs_around_a_chunk(wrk, ctx, head_size, over_r):
+    # around the four tokens that are summed together and the 4, 8 or 16 of a chunk; the outputs may replace r
+    gx, gs, rx, rs = _v7_case(wrk, ctx, 3, [(0, 3), (1, 4), (2, 5), (3, 15), (4, 16), (5, 33)], 6, True, seed=80 + head_size, S=head_size,
+                              over_r=over_r)
     assert_close(gx, rx, "x")
     assert_close(gs, rs, "state")
 

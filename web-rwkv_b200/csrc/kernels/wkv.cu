@@ -55,27 +55,64 @@ __device__ __forceinline__ bool find_run(const uint32_t* cursors, int wide, uint
     return count != 0;
 }
 
-// One CTA of (S / 4) (S / CW) threads per (head, batch slot): a thread keeps a 4 x CW tile of the head's S x S state
-// in registers for the sequence's whole run of tokens (rows = key index, columns = value index), so every k, r, w
-// value it fetches from shared memory feeds CW columns and every v value four rows.  (Measured at S = 64, 64 heads:
-// CW = 4, 8 warps: 0.34 us per token; CW = 2, 16 warps: 0.40 us.)  The S / 4 row groups of a column
-// group are lanes of ONE warp: a token's output column is summed by shuffles alone, and nothing but the state's own
-// recurrence (one fma deep per token) ties a token to the one before it - no barrier, no shared-memory partials.  The
-// tokens' k, r, w and v rows reach shared memory a chunk of TC tokens at a time, loaded a chunk ahead into registers
-// while the current chunk is computed (one barrier per chunk), so a token's step never waits for global memory.
-template <int S, int CW>
-__global__ void __launch_bounds__((S / 4) * (S / CW)) time_mix_v56_kernel(const WkvArgs a) {
+// Four consecutive channels from element i, a multiple of four.
+__device__ __forceinline__ float4 load_quad(const void* base, int dtype, size_t i) {
+    if (dtype != WRK_F16) return *reinterpret_cast<const float4*>(static_cast<const float*>(base) + i);
+    const uint2 q = *reinterpret_cast<const uint2*>(static_cast<const __half*>(base) + i);
+    const float2 lo = __half22float2(*reinterpret_cast<const __half2*>(&q.x)), hi = __half22float2(*reinterpret_cast<const __half2*>(&q.y));
+    return make_float4(lo.x, lo.y, hi.x, hi.y);
+}
+__device__ __forceinline__ float4 splat4(float v) { return make_float4(v, v, v, v); }
+__device__ __forceinline__ float2 lo2(const float4& v) { return make_float2(v.x, v.y); }
+__device__ __forceinline__ float2 hi2(const float4& v) { return make_float2(v.z, v.w); }
+
+// Sums N values per lane over G neighbouring lanes (both powers of two).  Every step halves the values a lane still carries
+// and sends the other half to its partner: N - 1 shuffles instead of N log2 G.  Lane g of the G ends with the sums of values
+// g N / G .. in y[0 ..] (N >= G), or with value g N / G (N < G).
+template <int N, int G>
+__device__ __forceinline__ void sum_scatter(float (&y)[N], uint32_t g) {
+    int width = N;
+#pragma unroll
+    for (int mask = G / 2; mask >= 1; mask /= 2) {
+        if (width > 1) {
+            width /= 2;
+            const bool upper = (g & mask) != 0;
+#pragma unroll
+            for (int i = 0; i < N / 2; ++i) {
+                if (i >= width) break;
+                const float keep = upper ? y[i + width] : y[i], send = upper ? y[i] : y[i + width];
+                y[i] = keep + __shfl_xor_sync(0xffffffffu, send, mask);
+            }
+        } else {
+            y[0] += __shfl_xor_sync(0xffffffffu, y[0], mask);
+        }
+    }
+}
+
+// v5 / v6.  The columns of a head's S x S state (rows = key index, columns = value index) do not depend on one another, so
+// a CTA takes NC of them, for the sequence's whole run of tokens: 64 heads of 64 channels are 128 CTAs of 32 columns, one
+// per SM.  A thread keeps a 4 x 4 tile of the state in registers, as pairs of rows (two products per instruction); the
+// S / 4 row groups of a column group are lanes of one warp.  A token is tied to the one before it by one fma of the state
+// alone; four tokens' outputs are summed over the row groups together (sum_scatter: 15 shuffles for 16 values).  The
+// tokens' k, r, w and v rows reach shared memory a chunk of TC tokens at a time, loaded a chunk ahead into registers while
+// the current chunk is computed (one barrier per chunk).  Past the run's end k, r, v are 0 and w is 1: such a token changes
+// nothing.
+// Measured at 64 heads of 64, one sequence: 35 us for 256 tokens and 0.12 us per further token.  A CTA per whole head
+// took 95 us serially and 76 us in blocks of 16 tokens (three matrix products per block on the same 64 SMs).  Tiles of
+// 4 x 2 with twice the warps: 33 us, but 6 instead of 4 us for a single token.
+template <int S, int NC>
+__global__ void __launch_bounds__((S / 4) * (NC / 4)) time_mix_v56_kernel(const WkvArgs a) {
     pdl_launch_dependents();
     pdl_wait();
-    constexpr int RG = S / 4, NT = RG * (S / CW), CGW = 32 / RG, TC = S <= 64 ? 16 : 4, PI = (4 * S + NT - 1) / NT;
-    static_assert(CW == 2 || CW == 4, "columns per thread");
+    constexpr int RG = S / 4, NT = RG * (NC / 4), CGW = 32 / RG, TC = S <= 64 ? 16 : 8, QT = (TC * RG + NT - 1) / NT;
     static_assert(RG == 8 || RG == 16 || RG == 32, "the row groups of a column group are lanes of one warp");
-    enum { IN_K = 0, IN_R = 1, IN_W = 2, IN_V = 3 };
-    __shared__ __align__(16) float sin[2][4][TC][S];
+    enum { IN_K = 0, IN_R = 1, IN_W = 2 };
+    __shared__ __align__(16) float sin[2][3][TC][S], sv[2][TC][NC];
     __shared__ RunScratch run;
-    const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const uint32_t rg = lane % RG, cg = warp * CGW + lane / RG;  // rows 4 rg .. 4 rg + 3, columns CW cg .. CW cg + CW - 1
-    const uint32_t h = blockIdx.x, slot = blockIdx.y, C = a.S * a.H, c0 = h * S;
+    const uint32_t tid = threadIdx.x, lane = tid & 31;
+    const uint32_t rg = lane % RG, cg = (tid >> 5) * CGW + lane / RG;  // rows 4 rg .., columns 4 cg .. of the CTA's
+    const uint32_t h = blockIdx.x / (S / NC), part = blockIdx.x % (S / NC), slot = blockIdx.y, C = a.S * a.H, c0 = h * S;
+    const uint32_t v0 = c0 + part * NC;  // the CTA's first column among all channels
 
     uint32_t start, count, carry;
     if (!find_run(a.cursors, a.wide, a.T, slot, &run, start, count, &carry)) return;
@@ -83,82 +120,82 @@ __global__ void __launch_bounds__((S / 4) * (S / CW)) time_mix_v56_kernel(const 
     // row, so it is written now, before the token's input is overwritten with its output; the token loop below then
     // has no cursor to look at and no branch.
     if (carry != 0) {
-        for (uint32_t j = tid; j < S; j += NT)
-            static_cast<float*>(a.state.base)[a.state.index(c0 + j, 0, slot)] = dload(a.x, a.dtype, (size_t)(carry - 1) * C + c0 + j);
+        for (uint32_t j = tid; j < NC; j += NT)
+            static_cast<float*>(a.state.base)[a.state.index(v0 + j, 0, slot)] = dload(a.x, a.dtype, (size_t)(carry - 1) * C + v0 + j);
     }
 
-    float st[4][CW], u[4];  // st[row][column]
+    float2 st[2][4], u[2];  // st[pair of rows][column]
+    float* state[4];
+    bool vec = true;  // a view's rows may start anywhere
 #pragma unroll
     for (int r = 0; r < 4; ++r) {
-        u[r] = a.time_first[c0 + 4 * rg + r];
+        state[r] = static_cast<float*>(a.state.base) + a.state.index(v0 + 4 * cg, 1 + 4 * rg + r, slot);
+        vec = vec && reinterpret_cast<uintptr_t>(state[r]) % 16 == 0;
+    }
+    auto load_row = [&](const float* p) { return vec ? *reinterpret_cast<const float4*>(p) : make_float4(p[0], p[1], p[2], p[3]); };
 #pragma unroll
-        for (int cc = 0; cc < CW; ++cc)
-            st[r][cc] = static_cast<const float*>(a.state.base)[a.state.index(c0 + CW * cg + cc, 1 + 4 * rg + r, slot)];
+    for (int p = 0; p < 2; ++p) {
+        u[p] = make_float2(a.time_first[c0 + 4 * rg + 2 * p], a.time_first[c0 + 4 * rg + 2 * p + 1]);
+        const float4 s0 = load_row(state[2 * p]), s1 = load_row(state[2 * p + 1]);
+        st[p][0] = make_float2(s0.x, s1.x), st[p][1] = make_float2(s0.y, s1.y);
+        st[p][2] = make_float2(s0.z, s1.z), st[p][3] = make_float2(s0.w, s1.w);
     }
 
-    // staging: (tensor, channel) pairs tid, tid + NT, ... of the 4 S pairs; element (token, channel) of chunk `chunk`
-    // (zero past the run's end)
-    float stage[PI][TC];
+    // staging: (token, four channels) pairs tid, tid + NT, ... of the TC RG pairs of a chunk
+    float4 gk[QT], gr[QT], gw[QT], gv[QT];
     auto load_chunk = [&](uint32_t chunk) {
 #pragma unroll
-        for (int pi = 0; pi < PI; ++pi) {
-            const uint32_t pair = tid + pi * NT, tensor = pair / S, c = c0 + pair % S;
-#pragma unroll
-            for (int n = 0; n < TC; ++n) {
-                const uint32_t m = chunk * TC + n;
-                const size_t ti = (size_t)(start + m) * C + c;
-                float v = 0.f;
-                if (pair < 4 * S && m < count) {
-                    if (tensor == IN_K) v = dload(a.k, a.dtype, ti);
-                    else if (tensor == IN_R) v = dload(a.r, a.dtype, ti);
-                    else if (tensor == IN_W) v = a.per_token_decay ? a.time_decay[ti] : a.time_decay[c];
-                    else v = dload(a.v, a.dtype, ti);
-                }
-                stage[pi][n] = v;
+        for (int q = 0; q < QT; ++q) {
+            const uint32_t idx = tid + q * NT, m = chunk * TC + idx / RG, c = 4 * (idx % RG);
+            gk[q] = gr[q] = gv[q] = splat4(0.f);
+            gw[q] = splat4(1.f);
+            if (idx < TC * RG && m < count) {
+                const size_t ti = (size_t)(start + m) * C;
+                gk[q] = load_quad(a.k, a.dtype, ti + c0 + c);
+                gr[q] = load_quad(a.r, a.dtype, ti + c0 + c);
+                gw[q] = *reinterpret_cast<const float4*>(a.time_decay + (a.per_token_decay ? ti : 0) + c0 + c);
+                if (c < NC) gv[q] = load_quad(a.v, a.dtype, ti + v0 + c);
             }
         }
     };
     auto store_chunk = [&](int buf) {
 #pragma unroll
-        for (int pi = 0; pi < PI; ++pi) {
-            const uint32_t pair = tid + pi * NT;
-            if (pair < 4 * S) {
-#pragma unroll
-                for (int n = 0; n < TC; ++n) sin[buf][pair / S][n][pair % S] = stage[pi][n];
+        for (int q = 0; q < QT; ++q) {
+            const uint32_t idx = tid + q * NT, n = idx / RG, c = 4 * (idx % RG);
+            if (idx < TC * RG) {
+                *reinterpret_cast<float4*>(&sin[buf][IN_K][n][c]) = gk[q];
+                *reinterpret_cast<float4*>(&sin[buf][IN_R][n][c]) = gr[q];
+                *reinterpret_cast<float4*>(&sin[buf][IN_W][n][c]) = gw[q];
+                if (c < NC) *reinterpret_cast<float4*>(&sv[buf][n][c]) = gv[q];
             }
         }
     };
-    // one token: the tile's share of the four output columns, summed over the row groups; lane rg == 0 stores them
-    auto token = [&](int buf, uint32_t n, uint32_t t) {
-        const float4 kq = *reinterpret_cast<const float4*>(&sin[buf][IN_K][n][4 * rg]);
-        const float4 rq = *reinterpret_cast<const float4*>(&sin[buf][IN_R][n][4 * rg]);
-        const float4 wq = *reinterpret_cast<const float4*>(&sin[buf][IN_W][n][4 * rg]);
-        const float kr[4] = {kq.x, kq.y, kq.z, kq.w}, rr[4] = {rq.x, rq.y, rq.z, rq.w}, wr[4] = {wq.x, wq.y, wq.z, wq.w};
-        float vc[CW], y[CW];
+    // four tokens, n0 .. of the chunk; the first of them is token t of the job, `left` of them exist
+    auto tokens4 = [&](int buf, uint32_t n0, uint32_t t, uint32_t left) {
+        float y[16];
 #pragma unroll
-        for (int cc = 0; cc < CW; cc += 2) {
-            const float2 vq = *reinterpret_cast<const float2*>(&sin[buf][IN_V][n][CW * cg + cc]);
-            vc[cc] = vq.x, vc[cc + 1] = vq.y;
-            y[cc] = y[cc + 1] = 0.f;
-        }
+        for (int n = 0; n < 4; ++n) {
+            const float4 kq = *reinterpret_cast<const float4*>(&sin[buf][IN_K][n0 + n][4 * rg]);
+            const float4 rq = *reinterpret_cast<const float4*>(&sin[buf][IN_R][n0 + n][4 * rg]);
+            const float4 wq = *reinterpret_cast<const float4*>(&sin[buf][IN_W][n0 + n][4 * rg]);
+            const float4 vq = *reinterpret_cast<const float4*>(&sv[buf][n0 + n][4 * cg]);
+            const float vc[4] = {vq.x, vq.y, vq.z, vq.w};
 #pragma unroll
-        for (int r = 0; r < 4; ++r) {
-#pragma unroll
-            for (int cc = 0; cc < CW; ++cc) {
-                const float kv = kr[r] * vc[cc];
-                y[cc] = fmaf(rr[r], fmaf(u[r], kv, st[r][cc]), y[cc]);
-                st[r][cc] = fmaf(wr[r], st[r][cc], kv);
+            for (int cc = 0; cc < 4; ++cc) {
+                const float2 v2 = make_float2(vc[cc], vc[cc]);
+                const float2 kv0 = __fmul2_rn(lo2(kq), v2), kv1 = __fmul2_rn(hi2(kq), v2);
+                const float2 y2 = __ffma2_rn(hi2(rq), __ffma2_rn(u[1], kv1, st[1][cc]), __fmul2_rn(lo2(rq), __ffma2_rn(u[0], kv0, st[0][cc])));
+                st[0][cc] = __ffma2_rn(lo2(wq), st[0][cc], kv0);
+                st[1][cc] = __ffma2_rn(hi2(wq), st[1][cc], kv1);
+                y[4 * n + cc] = y2.x + y2.y;
             }
         }
+        sum_scatter<16, RG>(y, rg);
+        constexpr int OUT = RG <= 16 ? 16 / RG : 1;
 #pragma unroll
-        for (int off = 1; off < RG; off <<= 1) {
-#pragma unroll
-            for (int cc = 0; cc < CW; ++cc) y[cc] += __shfl_xor_sync(0xffffffffu, y[cc], off);
-        }
-        if (rg == 0) {
-            const size_t ti = (size_t)t * C + c0 + CW * cg;
-#pragma unroll
-            for (int cc = 0; cc < CW; ++cc) dstore(a.x, a.dtype, ti + cc, y[cc]);
+        for (int e = 0; e < OUT; ++e) {
+            const uint32_t i = rg * 16 / RG + e, n = i / 4;
+            if ((RG <= 16 || (rg & 1) == 0) && n < left) dstore(a.x, a.dtype, (size_t)(t + n) * C + v0 + 4 * cg + i % 4, y[e]);
         }
     };
     const uint32_t chunks = (count + TC - 1) / TC;
@@ -170,364 +207,163 @@ __global__ void __launch_bounds__((S / 4) * (S / CW)) time_mix_v56_kernel(const 
         const int buf = chunk & 1;
         const bool more = chunk + 1 < chunks;
         if (more) load_chunk(chunk + 1);  // in flight while this chunk's tokens are computed
-        const uint32_t len = min((uint32_t)TC, count - chunk * TC), t0 = start + chunk * TC;
-        if (len == TC) {
-#pragma unroll 4
-            for (uint32_t n = 0; n < TC; ++n) token(buf, n, t0 + n);
+        const uint32_t left = count - chunk * TC, t0 = start + chunk * TC;
+        if (left >= TC) {
+#pragma unroll
+            for (uint32_t n = 0; n < TC; n += 4) tokens4(buf, n, t0 + n, 4);
         } else {
-            for (uint32_t n = 0; n < len; ++n) token(buf, n, t0 + n);
+#pragma unroll 1
+            for (uint32_t n = 0; n < left; n += 4) tokens4(buf, n, t0 + n, left - n);
         }
         if (more) store_chunk(buf ^ 1);  // last read during the previous chunk, before its closing barrier
         __syncthreads();
     }
 #pragma unroll
-    for (int r = 0; r < 4; ++r)
-#pragma unroll
-        for (int cc = 0; cc < CW; ++cc)
-            static_cast<float*>(a.state.base)[a.state.index(c0 + CW * cg + cc, 1 + 4 * rg + r, slot)] = st[r][cc];
-}
-
-// ---- v5 / v6 in blocks of 16 tokens ("chunk-parallel") ------------------------------------------------------------
-// The recurrence  y_t = r_t . (u k_t v_t^T + S_(t-1)),  S_t = diag(w_t) S_(t-1) + k_t v_t^T  unrolled over a block of
-// L = 16 tokens that starts from state S0 (rows i = key index, columns j = value index, per head):
-//   y_t   = (r_t Pe_t) S0  +  sum_(s<=t) A[t][s] v_s,      S_end = diag(Pe_L) S0 + sum_s (k_s E_s) v_s^T
-//   Pe_t  = prod_(m<t) w_m   (Pe_0 = 1),   E_s = prod_(m>s) w_m,
-//   A[t][s] = sum_i r_t[i] k_s[i] prod_(s<m<t) w_m[i]  (s < t),   A[t][t] = sum_i r_t[i] u[i] k_t[i].
-// Every product of decays is taken forwards (no division, nothing can overflow; what underflows is a contribution that
-// has decayed to nothing).  The work of a block is then three small matrix products - [16 x 64][64 x 64] for the state's
-// share of y, [16 x 16][16 x 64] for the block's own tokens and [64 x 16][16 x 64] for the new state - in which no
-// element waits for another: 4 x 4 register tiles in fp32 on the CUDA cores, operands from shared memory.  The serial
-// kernel above spends about 650 cycles on a token's chain of dependent steps; this one about 130 per token.
-// One CTA of 256 threads per (head of 64 channels, batch slot); the state tile of a thread stays in registers from
-// block to block; the tokens' rows are staged a block ahead as in the serial kernel.
-constexpr int kBlockTokens = 16;
-constexpr int kQtStride = 20;  // row stride of Qt in floats: 16-byte rows whose vector stores do not collide
-constexpr size_t kChunkedSmemFloats = 2 * 4 * kBlockTokens * 64 + 64 * kQtStride + kBlockTokens * 64 + kBlockTokens * kBlockTokens + 64 +
-                                      64 * 64 + 4 * kBlockTokens * 64;
-__global__ void __launch_bounds__(256) time_mix_v56_chunked_kernel(const WkvArgs a) {
-    pdl_launch_dependents();
-    pdl_wait();
-    constexpr int S = 64, L = kBlockTokens;
-    enum { IN_K = 0, IN_R = 1, IN_W = 2, IN_V = 3 };
-    extern __shared__ __align__(16) float wkv_smem[];
-    float(*sin)[4][L][S] = reinterpret_cast<float(*)[4][L][S]>(wkv_smem);              // [2]: staged k, r, w, v
-    float(*Qt)[kQtStride] = reinterpret_cast<float(*)[kQtStride]>(wkv_smem + 2 * 4 * L * S);  // [S]: Qt[i][t] = r_t[i] Pe_t[i]
-    float(*Kd)[S] = reinterpret_cast<float(*)[S]>(&Qt[S][0]);                            // [L]: Kd[s][i] = k_s[i] E_s[i]
-    float(*At)[L] = reinterpret_cast<float(*)[L]>(&Kd[L][0]);                            // [L]: At[s][t] = A[t][s], 0 for s > t
-    float* PL = &At[L][0];                                                               // [S]: the block's whole decay
-    float(*S0)[S] = reinterpret_cast<float(*)[S]>(PL + S);                               // [S]: the state at the block's start
-    float* red = &S0[S][0];  // [4][L][S] partial outputs of the four key ranges; before that [L s][L t][16] partials of A
-    __shared__ RunScratch run;
-    const uint32_t tid = threadIdx.x;
-    const uint32_t h = blockIdx.x, slot = blockIdx.y, C = a.S * a.H, c0 = h * S;
-    const uint32_t ri = tid / 16, cj = tid % 16;               // state tile: rows 4 ri .., columns 4 cj ..
-    const uint32_t tg = tid / 64, tt = (tid % 64) / 16;        // output tile: key range 16 tg .., tokens 4 tt .., columns 4 cj ..
-
-    uint32_t start, count, carry;
-    if (!find_run(a.cursors, a.wide, a.T, slot, &run, start, count, &carry)) return;
-    if (carry != 0 && tid < S)  // the carry row takes the layer input of the run's closing token (nothing here reads the row)
-        static_cast<float*>(a.state.base)[a.state.index(c0 + tid, 0, slot)] = dload(a.x, a.dtype, (size_t)(carry - 1) * C + c0 + tid);
-
-    float st[4][4];
-#pragma unroll
-    for (int r = 0; r < 4; ++r)
-#pragma unroll
-        for (int cc = 0; cc < 4; ++cc)
-            st[r][cc] = static_cast<const float*>(a.state.base)[a.state.index(c0 + 4 * cj + cc, 1 + 4 * ri + r, slot)];
-    float u4[4];  // time_first of the keys this thread takes in the A partials: 4 (tid % 16) ..
-#pragma unroll
-    for (int e = 0; e < 4; ++e) u4[e] = a.time_first[c0 + 4 * cj + e];
-
-    // staging: thread (tensor = tid / 64, channel = tid % 64) takes the block's 16 tokens of its tensor and channel;
-    // past the run's end k, r, v are 0 and w is 1 (such a token changes nothing)
-    float stage[L];
-    const uint32_t tensor = tid / S, ch = tid % S;
-    auto load_chunk = [&](uint32_t chunk) {
-#pragma unroll
-        for (int n = 0; n < L; ++n) {
-            const uint32_t m = chunk * L + n;
-            const size_t ti = (size_t)(start + m) * C + c0 + ch;
-            float v = tensor == IN_W ? 1.0f : 0.0f;
-            if (m < count) {
-                if (tensor == IN_K) v = dload(a.k, a.dtype, ti);
-                else if (tensor == IN_R) v = dload(a.r, a.dtype, ti);
-                else if (tensor == IN_W) v = a.per_token_decay ? a.time_decay[ti] : a.time_decay[c0 + ch];
-                else v = dload(a.v, a.dtype, ti);
-            }
-            stage[n] = v;
-        }
-    };
-    auto store_chunk = [&](int buf) {
-#pragma unroll
-        for (int n = 0; n < L; ++n) sin[buf][tensor][n][ch] = stage[n];
-    };
-    const uint32_t chunks = (count + L - 1) / L;
-    load_chunk(0);
-    store_chunk(0);
-    __syncthreads();
-
-    for (uint32_t chunk = 0; chunk < chunks; ++chunk) {
-        const int buf = chunk & 1;
-        const bool more = chunk + 1 < chunks;
-        if (more) load_chunk(chunk + 1);  // in flight while this block is computed
-        const float(*sk)[S] = sin[buf][IN_K];
-        const float(*sr)[S] = sin[buf][IN_R];
-        const float(*sw)[S] = sin[buf][IN_W];
-        const float(*sv)[S] = sin[buf][IN_V];
-
-        // (1) the state tile to shared memory; the decay products; the partial sums of A
-#pragma unroll
-        for (int r = 0; r < 4; ++r) *reinterpret_cast<float4*>(&S0[4 * ri + r][4 * cj]) = make_float4(st[r][0], st[r][1], st[r][2], st[r][3]);
-        {
-            // thread (key i = tid % 64, quarter tq = tid / 64): Qt[i][4 tq ..], Kd[4 tq ..][i]; quarter 3 ends on the whole product
-            const uint32_t i = tid % S, tq = tid / S;
-            float pe = 1.0f;
-            for (uint32_t t = 0; t < 4 * tq; ++t) pe *= sw[t][i];
-            float q[4];
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                q[e] = sr[4 * tq + e][i] * pe;
-                pe *= sw[4 * tq + e][i];
-            }
-            *reinterpret_cast<float4*>(&Qt[i][4 * tq]) = make_float4(q[0], q[1], q[2], q[3]);
-            if (tq == 3) PL[i] = pe;
-            float en = 1.0f;
-            for (uint32_t s2 = L - 1; s2 > 4 * tq + 3; --s2) en *= sw[s2][i];
-#pragma unroll
-            for (int e = 3; e >= 0; --e) {
-                Kd[4 * tq + e][i] = sk[4 * tq + e][i] * en;
-                en *= sw[4 * tq + e][i];
-            }
-        }
-        {
-            // thread (s = tid / 16, keys 4 cj ..): its share of A[t][s] for t = s .. L - 1, into red[s][t][cj]
-            const uint32_t s2 = tid / 16;
-            const float4 kq = *reinterpret_cast<const float4*>(&sk[s2][4 * cj]);
-            const float kk[4] = {kq.x, kq.y, kq.z, kq.w};
-            float d[4] = {1.0f, 1.0f, 1.0f, 1.0f};
-            for (uint32_t t = 0; t < s2; ++t) red[(s2 * L + t) * 16 + cj] = 0.0f;
-            {
-                const float4 rq = *reinterpret_cast<const float4*>(&sr[s2][4 * cj]);
-                red[(s2 * L + s2) * 16 + cj] = (rq.x * kk[0] * u4[0] + rq.y * kk[1] * u4[1]) + (rq.z * kk[2] * u4[2] + rq.w * kk[3] * u4[3]);
-            }
-            for (uint32_t t = s2 + 1; t < L; ++t) {
-                const float4 rq = *reinterpret_cast<const float4*>(&sr[t][4 * cj]);
-                const float4 wq = *reinterpret_cast<const float4*>(&sw[t][4 * cj]);
-                red[(s2 * L + t) * 16 + cj] = (rq.x * kk[0] * d[0] + rq.y * kk[1] * d[1]) + (rq.z * kk[2] * d[2] + rq.w * kk[3] * d[3]);
-                d[0] *= wq.x, d[1] *= wq.y, d[2] *= wq.z, d[3] *= wq.w;
-            }
-        }
-        __syncthreads();
-        // (2) A[t][s] summed over the 16 key groups: thread (s, t) = (tid / 16, tid % 16)
-        {
-            const float4* p4 = reinterpret_cast<const float4*>(red + (size_t)tid * 16);
-            const float4 p0 = p4[0], p1 = p4[1], p2 = p4[2], p3 = p4[3];
-            At[tid / 16][tid % 16] = ((p0.x + p0.y) + (p0.z + p0.w)) + ((p1.x + p1.y) + (p1.z + p1.w)) +
-                                     (((p2.x + p2.y) + (p2.z + p2.w)) + ((p3.x + p3.y) + (p3.z + p3.w)));
-        }
-        __syncthreads();
-        // (3) the outputs of tokens 4 tt .. and columns 4 cj .., summed over keys 16 tg .. (the state's share) and over the
-        // block's tokens 4 tg .. (their own share); then the new state tile
-        {
-            float acc[4][4];
-#pragma unroll
-            for (int e = 0; e < 4; ++e)
-#pragma unroll
-                for (int cc = 0; cc < 4; ++cc) acc[e][cc] = 0.0f;
-#pragma unroll 4
-            for (uint32_t i = 16 * tg; i < 16 * tg + 16; ++i) {
-                const float4 q4 = *reinterpret_cast<const float4*>(&Qt[i][4 * tt]);
-                const float4 s4 = *reinterpret_cast<const float4*>(&S0[i][4 * cj]);
-                const float qv[4] = {q4.x, q4.y, q4.z, q4.w}, sv4[4] = {s4.x, s4.y, s4.z, s4.w};
-#pragma unroll
-                for (int e = 0; e < 4; ++e)
-#pragma unroll
-                    for (int cc = 0; cc < 4; ++cc) acc[e][cc] = fmaf(qv[e], sv4[cc], acc[e][cc]);
-            }
-#pragma unroll
-            for (uint32_t s2 = 4 * tg; s2 < 4 * tg + 4; ++s2) {
-                const float4 a4 = *reinterpret_cast<const float4*>(&At[s2][4 * tt]);
-                const float4 v4 = *reinterpret_cast<const float4*>(&sv[s2][4 * cj]);
-                const float av[4] = {a4.x, a4.y, a4.z, a4.w}, vv[4] = {v4.x, v4.y, v4.z, v4.w};
-#pragma unroll
-                for (int e = 0; e < 4; ++e)
-#pragma unroll
-                    for (int cc = 0; cc < 4; ++cc) acc[e][cc] = fmaf(av[e], vv[cc], acc[e][cc]);
-            }
-            // red is free again: every thread has passed the barrier that follows its last read in (2)
-#pragma unroll
-            for (int e = 0; e < 4; ++e)
-                *reinterpret_cast<float4*>(&red[((size_t)tg * L + 4 * tt + e) * S + 4 * cj]) = make_float4(acc[e][0], acc[e][1], acc[e][2], acc[e][3]);
-        }
-        {
-            const float4 pl = *reinterpret_cast<const float4*>(&PL[4 * ri]);
-            const float plv[4] = {pl.x, pl.y, pl.z, pl.w};
-#pragma unroll
-            for (int r = 0; r < 4; ++r)
-#pragma unroll
-                for (int cc = 0; cc < 4; ++cc) st[r][cc] *= plv[r];
-#pragma unroll 4
-            for (uint32_t s2 = 0; s2 < L; ++s2) {
-                const float4 k4 = *reinterpret_cast<const float4*>(&Kd[s2][4 * ri]);
-                const float4 v4 = *reinterpret_cast<const float4*>(&sv[s2][4 * cj]);
-                const float kv[4] = {k4.x, k4.y, k4.z, k4.w}, vv[4] = {v4.x, v4.y, v4.z, v4.w};
-#pragma unroll
-                for (int r = 0; r < 4; ++r)
-#pragma unroll
-                    for (int cc = 0; cc < 4; ++cc) st[r][cc] = fmaf(kv[r], vv[cc], st[r][cc]);
-            }
-        }
-        __syncthreads();
-        // (4) token t = tid / 16, columns 4 cj ..: the four key ranges' partial outputs
-        {
-            const uint32_t t = tid / 16, m = chunk * L + t;
-            if (m < count) {
-                float4 y = *reinterpret_cast<const float4*>(&red[((size_t)0 * L + t) * S + 4 * cj]);
-#pragma unroll
-                for (int g = 1; g < 4; ++g) {
-                    const float4 p = *reinterpret_cast<const float4*>(&red[((size_t)g * L + t) * S + 4 * cj]);
-                    y.x += p.x, y.y += p.y, y.z += p.z, y.w += p.w;
-                }
-                const size_t ti = (size_t)(start + m) * C + c0 + 4 * cj;
-                dstore(a.x, a.dtype, ti, y.x);
-                dstore(a.x, a.dtype, ti + 1, y.y);
-                dstore(a.x, a.dtype, ti + 2, y.z);
-                dstore(a.x, a.dtype, ti + 3, y.w);
-            }
-        }
-        if (more) store_chunk(buf ^ 1);  // last read during the previous block, before its closing barrier
-        __syncthreads();
+    for (int r = 0; r < 4; ++r) {
+        const float2* s = st[r / 2];
+        const float4 v = r % 2 == 0 ? make_float4(s[0].x, s[1].x, s[2].x, s[3].x) : make_float4(s[0].y, s[1].y, s[2].y, s[3].y);
+        if (vec) *reinterpret_cast<float4*>(state[r]) = v;
+        else state[r][0] = v.x, state[r][1] = v.y, state[r][2] = v.z, state[r][3] = v.w;
     }
-#pragma unroll
-    for (int r = 0; r < 4; ++r)
-#pragma unroll
-        for (int cc = 0; cc < 4; ++cc)
-            static_cast<float*>(a.state.base)[a.state.index(c0 + 4 * cj + cc, 1 + 4 * ri + r, slot)] = st[r][cc];
 }
 
-// v7: one CTA of (1 + G) * S threads per (head, batch slot).  Thread j of the first S keeps the whole column j of the
-// state in registers, so a token needs no exchange between threads; the other G groups of S threads fetch the tokens'
-// rows a chunk of 768 / S tokens ahead (three pairs: r and the decay; k and v; a and kk, 3 / G pairs per group), apply
-// the per-token transforms (w -> exp(-0.606531 sigmoid(w)), -kk, kk a) and hand them over through shared memory, one
-// barrier per chunk.
-template <int S, int G>
-__global__ void __launch_bounds__((1 + G) * S) time_mix_v7_kernel(const WkvArgs a) {
+// v7: a CTA takes NC columns of a head's state, as above.  NC S / RPT threads compute: a thread keeps RPT rows of one column
+// (quads of rows S / RPT quads apart, so that the row groups' shared-memory reads meet no bank twice), the S / RPT row
+// groups of a column are neighbouring lanes; `sa` is summed over them in log2(S / RPT) shuffles per token, the outputs of
+// four tokens together.  Four more warps fetch the tokens' rows a chunk ahead, apply the per-token transforms
+// (w -> exp(-0.606531 sigmoid(w)), -kk, kk a) and hand them over through shared memory, one barrier per chunk.
+// Measured at 64 heads of 64, one sequence of 256 tokens: 62 us (0.23 us per further token); a thread per whole column, on
+// 64 SMs, took 113 us; eight rows per thread and twice the warps 66 us.
+constexpr int kV7Loaders = 128;
+// tokens of a chunk: two chunks fit 47 KB of shared memory
+template <int S, int NC>
+constexpr int kV7Chunk = 128 * (5 * S + NC) <= 47 * 1024 ? 16 : 64 * (5 * S + NC) <= 47 * 1024 ? 8 : 4;
+template <int S, int NC, int RPT>
+__global__ void __launch_bounds__(NC * (S / RPT) + kV7Loaders) time_mix_v7_kernel(const WkvArgs a) {
     pdl_launch_dependents();
     pdl_wait();
-    static_assert(G == 1 || G == 3, "three pairs of rows over the loader groups");
-    constexpr int TC = 768 / S, P = 3 / G;
-    enum { IN_R = 0, IN_W = 1, IN_K = 2, IN_V = 3, IN_A = 4, IN_B = 5 };
-    __shared__ __align__(16) float sin[2][6][TC][S];
+    constexpr int RG = S / RPT, NT = NC * RG, TC = kV7Chunk<S, NC>, QUADS = S / 4, QT = (TC * QUADS + kV7Loaders - 1) / kV7Loaders;
+    enum { IN_R = 0, IN_W = 1, IN_K = 2, IN_A = 3, IN_B = 4 };
+    __shared__ __align__(16) float sin[2][5][TC][S], sv[2][TC][NC];
     __shared__ RunScratch run;
-    const uint32_t h = blockIdx.x, slot = blockIdx.y, j = threadIdx.x % S, q = threadIdx.x / S;
-    const uint32_t C = a.S * a.H, c = h * S + j;
+    const uint32_t tid = threadIdx.x, rg = tid % RG, col = tid / RG;
+    const uint32_t h = blockIdx.x / (S / NC), part = blockIdx.x % (S / NC), slot = blockIdx.y, C = a.S * a.H, c0 = h * S, v0 = c0 + part * NC;
     const size_t plane = (size_t)a.T * C;
 
     uint32_t start, count, carry;
     if (!find_run(a.cursors, a.wide, a.T, slot, &run, start, count, &carry)) return;
     // the carry row takes the layer input of the run's closing token: written now (nothing here reads the row), before
     // the token's input is overwritten with its output
-    if (carry != 0 && q == 0)
-        static_cast<float*>(a.state.base)[a.state.index(c, 0, slot)] = dload(a.x, a.dtype, (size_t)(carry - 1) * C + c);
+    if (carry != 0 && tid < NC)
+        static_cast<float*>(a.state.base)[a.state.index(v0 + tid, 0, slot)] = dload(a.x, a.dtype, (size_t)(carry - 1) * C + v0 + tid);
 
-    float st[S];
-    if (q == 0) {
-#pragma unroll
-        for (int i = 0; i < S; ++i) st[i] = static_cast<const float*>(a.state.base)[a.state.index(c, 1 + i, slot)];
-    }
-
-    auto decay = [](float w) { return expf(-0.606531f * (1.0f / (1.0f + expf(-w)))); };
-    // loader group q (1..G): the pairs of staged rows it owns, element (token, channel j) of chunk `chunk` (zero past
-    // the run's end)
-    float s0[P][TC], s1[P][TC];
-    auto load_chunk = [&](uint32_t chunk) {
-#pragma unroll
-        for (int pi = 0; pi < P; ++pi) {
-            const uint32_t pair = G == 1 ? (uint32_t)pi : q - 1;
-#pragma unroll
-            for (int n = 0; n < TC; ++n) {
-                const uint32_t m = chunk * TC + n;
-                const size_t ti = (size_t)(start + m) * C + c;
-                float x0 = 0.f, x1 = 0.f;
-                if (m < count) {
-                    if (pair == 0) x0 = dload(a.r, a.dtype, ti), x1 = dload(a.w, a.dtype, ti);
-                    else if (pair == 1) x0 = dload(a.n, a.dtype, ti), x1 = dload(a.n, a.dtype, ti + plane);
-                    else x0 = dload(a.n, a.dtype, ti + 2 * plane), x1 = dload(a.n, a.dtype, ti + 3 * plane);
-                }
-                s0[pi][n] = x0;
-                s1[pi][n] = x1;
-            }
-        }
-    };
-    auto store_chunk = [&](int buf) {
-#pragma unroll
-        for (int pi = 0; pi < P; ++pi) {
-            const uint32_t pair = G == 1 ? (uint32_t)pi : q - 1;
-#pragma unroll
-            for (int n = 0; n < TC; ++n) {
-                if (pair == 0) sin[buf][IN_R][n][j] = s0[pi][n], sin[buf][IN_W][n][j] = decay(s1[pi][n]);
-                else if (pair == 1) sin[buf][IN_K][n][j] = s0[pi][n], sin[buf][IN_V][n][j] = s1[pi][n];
-                else sin[buf][IN_A][n][j] = -s1[pi][n], sin[buf][IN_B][n][j] = s1[pi][n] * s0[pi][n];
-            }
-        }
-    };
     const uint32_t chunks = (count + TC - 1) / TC;
-    if (q != 0) {
-        load_chunk(0);
-        store_chunk(0);
+    if (tid >= NT) {
+        const uint32_t lid = tid - NT;
+        auto decay = [](float w) { return expf(-0.606531f * (1.0f / (1.0f + expf(-w)))); };
+        // (token, four channels) pairs lid, lid + kV7Loaders, ... of the chunk; zero past the run's end
+        auto stage = [&](uint32_t chunk) {
+            float4 gr[QT], gw[QT], gk[QT], ga[QT], gkk[QT], gv[QT];
+#pragma unroll
+            for (int q = 0; q < QT; ++q) {
+                const uint32_t idx = lid + q * kV7Loaders, m = chunk * TC + idx / QUADS, c = 4 * (idx % QUADS);
+                gr[q] = gw[q] = gk[q] = ga[q] = gkk[q] = gv[q] = splat4(0.f);
+                if (idx < TC * QUADS && m < count) {
+                    const size_t ti = (size_t)(start + m) * C;
+                    gr[q] = load_quad(a.r, a.dtype, ti + c0 + c);
+                    gw[q] = load_quad(a.w, a.dtype, ti + c0 + c);
+                    gk[q] = load_quad(a.n, a.dtype, ti + c0 + c);
+                    ga[q] = load_quad(a.n, a.dtype, ti + c0 + c + 2 * plane);
+                    gkk[q] = load_quad(a.n, a.dtype, ti + c0 + c + 3 * plane);
+                    if (c < NC) gv[q] = load_quad(a.n, a.dtype, ti + v0 + c + plane);
+                }
+            }
+            const int buf = chunk & 1;
+#pragma unroll
+            for (int q = 0; q < QT; ++q) {
+                const uint32_t idx = lid + q * kV7Loaders, n = idx / QUADS, c = 4 * (idx % QUADS);
+                if (idx >= TC * QUADS) break;
+                *reinterpret_cast<float4*>(&sin[buf][IN_R][n][c]) = gr[q];
+                *reinterpret_cast<float4*>(&sin[buf][IN_W][n][c]) = make_float4(decay(gw[q].x), decay(gw[q].y), decay(gw[q].z), decay(gw[q].w));
+                *reinterpret_cast<float4*>(&sin[buf][IN_K][n][c]) = gk[q];
+                *reinterpret_cast<float4*>(&sin[buf][IN_A][n][c]) = make_float4(-gkk[q].x, -gkk[q].y, -gkk[q].z, -gkk[q].w);
+                *reinterpret_cast<float4*>(&sin[buf][IN_B][n][c]) =
+                    make_float4(gkk[q].x * ga[q].x, gkk[q].y * ga[q].y, gkk[q].z * ga[q].z, gkk[q].w * ga[q].w);
+                if (c < NC) *reinterpret_cast<float4*>(&sv[buf][n][c]) = gv[q];
+            }
+        };
+        stage(0);
+        __syncthreads();
+#pragma unroll 1
+        for (uint32_t chunk = 0; chunk < chunks; ++chunk) {
+            if (chunk + 1 < chunks) stage(chunk + 1);  // that buffer was last read two chunks ago, before that chunk's closing barrier
+            __syncthreads();
+        }
+        return;
     }
-    __syncthreads();
 
+    float2 st[RPT / 2];
+    auto row = [&](uint32_t i) { return 1 + 4 * ((i / 2) * RG + rg) + 2 * (i % 2); };  // state row of st[i].x; st[i].y is the next
+#pragma unroll
+    for (int i = 0; i < RPT / 2; ++i)
+        st[i] = make_float2(static_cast<const float*>(a.state.base)[a.state.index(v0 + col, row(i), slot)],
+                            static_cast<const float*>(a.state.base)[a.state.index(v0 + col, row(i) + 1, slot)]);
+    auto token = [&](int buf, uint32_t n) {
+        const float4* r4 = reinterpret_cast<const float4*>(sin[buf][IN_R][n]) + rg;
+        const float4* w4 = reinterpret_cast<const float4*>(sin[buf][IN_W][n]) + rg;
+        const float4* k4 = reinterpret_cast<const float4*>(sin[buf][IN_K][n]) + rg;
+        const float4* a4 = reinterpret_cast<const float4*>(sin[buf][IN_A][n]) + rg;
+        const float4* b4 = reinterpret_cast<const float4*>(sin[buf][IN_B][n]) + rg;
+        float2 z0 = make_float2(0.f, 0.f), z1 = z0;
+#pragma unroll
+        for (int i = 0; i < RPT / 4; ++i) {
+            const float4 av = a4[i * RG];
+            z0 = __ffma2_rn(st[2 * i], lo2(av), z0);
+            z1 = __ffma2_rn(st[2 * i + 1], hi2(av), z1);
+        }
+        float sa = (z0.x + z0.y) + (z1.x + z1.y);
+#pragma unroll
+        for (int mask = 1; mask < RG; mask *= 2) sa += __shfl_xor_sync(0xffffffffu, sa, mask);
+        const float vj = sv[buf][n][col];
+        const float2 v2 = make_float2(vj, vj), sa2 = make_float2(sa, sa);
+        float2 y0 = make_float2(0.f, 0.f), y1 = y0;
+#pragma unroll
+        for (int i = 0; i < RPT / 4; ++i) {
+            const float4 wv = w4[i * RG], kv = k4[i * RG], bv = b4[i * RG], rv = r4[i * RG];
+            st[2 * i] = __ffma2_rn(sa2, lo2(bv), __ffma2_rn(lo2(kv), v2, __fmul2_rn(st[2 * i], lo2(wv))));
+            st[2 * i + 1] = __ffma2_rn(sa2, hi2(bv), __ffma2_rn(hi2(kv), v2, __fmul2_rn(st[2 * i + 1], hi2(wv))));
+            y0 = __ffma2_rn(lo2(rv), st[2 * i], y0);
+            y1 = __ffma2_rn(hi2(rv), st[2 * i + 1], y1);
+        }
+        return (y0.x + y0.y) + (y1.x + y1.y);
+    };
+    __syncthreads();
+#pragma unroll 1
     for (uint32_t chunk = 0; chunk < chunks; ++chunk) {
         const int buf = chunk & 1;
-        const bool more = chunk + 1 < chunks;
-        if (q != 0) {
-            if (more) {
-                load_chunk(chunk + 1);
-                store_chunk(buf ^ 1);  // last read two chunks ago, before that chunk's closing barrier
+        const uint32_t len = min((uint32_t)TC, count - chunk * TC), t0 = start + chunk * TC;
+#pragma unroll 1
+        for (uint32_t n0 = 0; n0 < len; n0 += 4) {
+            float y[4];
+#pragma unroll
+            for (uint32_t n = 0; n < 4; ++n) {
+                y[n] = 0.f;
+                if (n0 + n < len) y[n] = token(buf, n0 + n);  // the same for every thread
             }
-        } else {
-            const uint32_t len = min((uint32_t)TC, count - chunk * TC);
-            for (uint32_t n = 0; n < len; ++n) {
-                const uint32_t t = start + chunk * TC + n;
-                const size_t ti = (size_t)t * C + c;
-                const float vj = sin[buf][IN_V][n][j];
-                const float4* r4 = reinterpret_cast<const float4*>(sin[buf][IN_R][n]);
-                const float4* w4 = reinterpret_cast<const float4*>(sin[buf][IN_W][n]);
-                const float4* k4 = reinterpret_cast<const float4*>(sin[buf][IN_K][n]);
-                const float4* a4 = reinterpret_cast<const float4*>(sin[buf][IN_A][n]);
-                const float4* b4 = reinterpret_cast<const float4*>(sin[buf][IN_B][n]);
-                float z0 = 0.f, z1 = 0.f, z2 = 0.f, z3 = 0.f;
+            sum_scatter<4, RG>(y, rg);
+            constexpr uint32_t OUT = RG <= 4 ? 4 / RG : 1, COPIES = RG <= 4 ? 1 : RG / 4;
 #pragma unroll
-                for (int i = 0; i < S; i += 4) {
-                    const float4 av = a4[i / 4];
-                    z0 = fmaf(st[i], av.x, z0);
-                    z1 = fmaf(st[i + 1], av.y, z1);
-                    z2 = fmaf(st[i + 2], av.z, z2);
-                    z3 = fmaf(st[i + 3], av.w, z3);
-                }
-                const float sav = (z0 + z1) + (z2 + z3);
-                float y0 = 0.f, y1 = 0.f, y2 = 0.f, y3 = 0.f;
-#pragma unroll
-                for (int i = 0; i < S; i += 4) {
-                    const float4 wv = w4[i / 4], kv = k4[i / 4], bv = b4[i / 4], rv = r4[i / 4];
-                    st[i] = st[i] * wv.x + kv.x * vj + sav * bv.x;
-                    y0 = fmaf(rv.x, st[i], y0);
-                    st[i + 1] = st[i + 1] * wv.y + kv.y * vj + sav * bv.y;
-                    y1 = fmaf(rv.y, st[i + 1], y1);
-                    st[i + 2] = st[i + 2] * wv.z + kv.z * vj + sav * bv.z;
-                    y2 = fmaf(rv.z, st[i + 2], y2);
-                    st[i + 3] = st[i + 3] * wv.w + kv.w * vj + sav * bv.w;
-                    y3 = fmaf(rv.w, st[i + 3], y3);
-                }
-                dstore(a.x, a.dtype, ti, (y0 + y1) + (y2 + y3));
+            for (uint32_t e = 0; e < OUT; ++e) {
+                const uint32_t n = rg * 4 / RG + e;
+                if (rg % COPIES == 0 && n0 + n < len) dstore(a.x, a.dtype, (size_t)(t0 + n0 + n) * C + v0 + col, y[e]);
             }
         }
         __syncthreads();
     }
-    if (q == 0) {
 #pragma unroll
-        for (int i = 0; i < S; ++i) static_cast<float*>(a.state.base)[a.state.index(c, 1 + i, slot)] = st[i];
+    for (int i = 0; i < RPT / 2; ++i) {
+        static_cast<float*>(a.state.base)[a.state.index(v0 + col, row(i), slot)] = st[i].x;
+        static_cast<float*>(a.state.base)[a.state.index(v0 + col, row(i) + 1, slot)] = st[i].y;
     }
 }
 
@@ -637,28 +473,21 @@ __global__ void time_first_v7_kernel(const __half* u, int dtype, const void* r, 
 
 }  // namespace
 
+// A job's kernels start early, on the SMs that the kernels before them leave free: CTAs that then compute for a long time
+// sit several to an SM.  With more than 64 tokens the recurrence waits for the kernel before it to end (256 tokens of one
+// sequence among four slots, 40 heads: 60 us when started early, against 35 alone; a launch that waits costs about 2 us).
+static bool wkv_early(const WkvArgs& a) { return a.T <= 64; }
+
+// A head's columns are shared out among CTAs unless the outputs overwrite an input that every CTA of the head reads.
 cudaError_t time_mix_v56(const WkvArgs& a, cudaStream_t stream) {
     if (a.T == 0 || a.B == 0) return cudaSuccess;
-    dim3 grid(a.H, a.B);
-    switch (a.S) {
-        case 32: launch(time_mix_v56_kernel<32, 4>, grid, dim3(64), 0, stream, a); break;
-        case 64: launch(time_mix_v56_kernel<64, 4>, grid, dim3(256), 0, stream, a); break;
-        case 128: launch(time_mix_v56_kernel<128, 4>, grid, dim3(1024), 0, stream, a); break;
-        default: return cudaErrorInvalidValue;
-    }
-    return cudaGetLastError();
-}
-
-// The block form of time_mix_v56 (heads of 64 channels only).
-bool time_mix_v56_chunked_supported(const WkvArgs& a) { return a.S == 64; }
-
-cudaError_t time_mix_v56_chunked(const WkvArgs& a, cudaStream_t stream) {
-    if (a.T == 0 || a.B == 0) return cudaSuccess;
-    if (!time_mix_v56_chunked_supported(a)) return cudaErrorInvalidValue;
-    static SmemOptIn opt_in;
-    const size_t smem = kChunkedSmemFloats * sizeof(float);
-    if (cudaError_t e = opt_in.ensure(time_mix_v56_chunked_kernel, (int)smem); e != cudaSuccess) return e;
-    launch(time_mix_v56_chunked_kernel, dim3(a.H, a.B), dim3(256), smem, stream, a);
+    const bool whole = a.x == a.k || a.x == a.r || a.x == a.time_decay, early = wkv_early(a);
+    if (a.S == 32) launch_early(early, time_mix_v56_kernel<32, 32>, dim3(a.H, a.B), dim3(64), 0, stream, a);
+    else if (a.S == 64 && whole) launch_early(early, time_mix_v56_kernel<64, 64>, dim3(a.H, a.B), dim3(256), 0, stream, a);
+    else if (a.S == 64) launch_early(early, time_mix_v56_kernel<64, 32>, dim3(2 * a.H, a.B), dim3(128), 0, stream, a);
+    else if (a.S == 128 && whole) launch_early(early, time_mix_v56_kernel<128, 128>, dim3(a.H, a.B), dim3(1024), 0, stream, a);
+    else if (a.S == 128) launch_early(early, time_mix_v56_kernel<128, 32>, dim3(4 * a.H, a.B), dim3(256), 0, stream, a);
+    else return cudaErrorInvalidValue;
     return cudaGetLastError();
 }
 
@@ -674,12 +503,14 @@ cudaError_t time_mix_v7(const WkvArgs& a, cudaStream_t stream) {
         }
         return cudaGetLastError();
     }
-    switch (a.S) {
-        case 32: launch(time_mix_v7_kernel<32, 3>, grid, dim3(128), 0, stream, a); break;
-        case 64: launch(time_mix_v7_kernel<64, 3>, grid, dim3(256), 0, stream, a); break;
-        case 128: launch(time_mix_v7_kernel<128, 1>, grid, dim3(256), 0, stream, a); break;
-        default: return cudaErrorInvalidValue;
-    }
+    const bool whole = a.x == a.r || a.x == a.w || a.x == a.n, early = wkv_early(a);  // as in time_mix_v56
+    constexpr int L = kV7Loaders;
+    if (a.S == 32) launch_early(early, time_mix_v7_kernel<32, 32, 16>, grid, dim3(64 + L), 0, stream, a);
+    else if (a.S == 64 && whole) launch_early(early, time_mix_v7_kernel<64, 64, 16>, grid, dim3(256 + L), 0, stream, a);
+    else if (a.S == 64) launch_early(early, time_mix_v7_kernel<64, 32, 16>, dim3(2 * a.H, a.B), dim3(128 + L), 0, stream, a);
+    else if (a.S == 128 && whole) launch_early(early, time_mix_v7_kernel<128, 128, 32>, grid, dim3(512 + L), 0, stream, a);
+    else if (a.S == 128) launch_early(early, time_mix_v7_kernel<128, 32, 16>, dim3(4 * a.H, a.B), dim3(256 + L), 0, stream, a);
+    else return cudaErrorInvalidValue;
     return cudaGetLastError();
 }
 

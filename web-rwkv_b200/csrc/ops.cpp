@@ -181,12 +181,7 @@ int32_t time_mix_v56(const char* name, int per_token, wrk_tensor* cursors, wrk_t
     a.per_token_decay = per_token;
     a.k = k->ptr(); a.v = v->ptr(); a.r = r->ptr(); a.x = x->ptr();
     a.status = x->ctx->device_status;
-    if (blocks) {
-        WRK_REQUIRE(k::time_mix_v56_chunked_supported(a), WRK_ERR_UNSUPPORTED, "time_mix_blocks takes heads of 64 channels");
-        *out = new_atom(name, [a](cudaStream_t s) { return k::time_mix_v56_chunked(a, s); },
-                        {cursors, time_decay, time_first, state->tensor, k, v, r, x});
-        return WRK_OK;
-    }
+    if (blocks) WRK_REQUIRE(S == 64, WRK_ERR_UNSUPPORTED, "time_mix_blocks takes heads of 64 channels");
     *out = new_atom(name, [a](cudaStream_t s) { return k::time_mix_v56(a, s); },
                     {cursors, time_decay, time_first, state->tensor, k, v, r, x});
     return WRK_OK;
