@@ -247,6 +247,18 @@ def test_blit_views_and_transpose(wrk, ctx):
     assert e.value.status == -5
 
 
+@pytest.mark.parametrize("T,C", [(1, 8), (3, 12), (300, 2056)])  # 12 channels: the general kernel
+def test_lerp_sizes(wrk, ctx, T, C):
+    rng = np.random.default_rng(8)
+    a, b = (rng.standard_normal((T, C)).astype(np.float16) for _ in range(2))
+    f = rng.uniform(0, 1, (T, C)).astype(np.float16)
+    for reversed_ in (True, False):
+        t_b, ref = ctx.from_numpy(b), b.copy()
+        ctx.run(wrk.lerp(ctx.from_numpy(a), t_b, ctx.from_numpy(f), reversed_))
+        oracle.lerp(a, ref, f, reversed_)
+        assert_close(t_b.numpy().reshape(T, C), ref, "lerp")
+
+
 @pytest.mark.parametrize("reversed_", [True, False])
 def test_lerp_affine_control_k(wrk, ctx, reversed_):
     rng = np.random.default_rng(7)

@@ -85,11 +85,11 @@ __global__ void binary_vec_kernel(int is_mul, const In* in, Out* out, uint32_t c
         float x[8], y[8];
         load8(in + (size_t)(in_row ? (plane8 ? o / plane8 * c8 : 0u) + o % c8 : o) * 8, x);
         load8(out + (size_t)o * 8, y);
+        activate_n(act_x, x);
+        activate_n(act_y, y);
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            const float ax = activate_f(act_x, x[i]), ay = activate_f(act_y, y[i]);
-            y[i] = activate_f(act_out, is_mul ? ax * ay : ax + ay);
-        }
+        for (int i = 0; i < 8; ++i) y[i] = is_mul ? x[i] * y[i] : x[i] + y[i];
+        activate_n(act_out, y);
         store8(out + (size_t)o * 8, y);
     }
 }
@@ -118,8 +118,7 @@ __global__ void activate_vec_kernel(T* x, uint32_t total8, int act) {
     for (uint32_t o = blockIdx.x * blockDim.x + threadIdx.x; o < total8; o += gridDim.x * blockDim.x) {
         float v[8];
         load8(x + (size_t)o * 8, v);
-#pragma unroll
-        for (int i = 0; i < 8; ++i) v[i] = activate_f(act, v[i]);
+        activate_n(act, v);
         store8(x + (size_t)o * 8, v);
     }
 }
@@ -145,6 +144,21 @@ bool blit_typed(const DView& input, const DView& output, cudaStream_t stream) {
     if (!fits32(total)) return false;
     launch(blit_vec_kernel<In, Out>, dim3(vec_grid(total / 8)), dim3(kVecThreads), 0, stream, in, out, (uint32_t)(total / 8));
     return true;
+}
+
+// ---- lerp.wgsl on f16 tensors of one shape: out <- mix(in, out, f), or mix(out, in, f) when reversed --------------
+__global__ void lerp_vec_kernel(const __half* in, __half* out, const __half* f, uint32_t total8, int reversed) {
+    pdl_launch_dependents();
+    pdl_wait();
+    for (uint32_t o = blockIdx.x * blockDim.x + threadIdx.x; o < total8; o += gridDim.x * blockDim.x) {
+        float x[8], y[8], g[8];
+        load8(in + (size_t)o * 8, x);
+        load8(out + (size_t)o * 8, y);
+        load8(f + (size_t)o * 8, g);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) y[i] = reversed ? mix_f(y[i], x[i], g[i]) : mix_f(x[i], y[i], g[i]);
+        store8(out + (size_t)o * 8, y);
+    }
 }
 
 // ---- token_shift.wgsl: out[c, t, z] <- mix(x_t, x_(t-1) or the carry row, f[c, (t,) z]) --------------------------
@@ -286,8 +300,9 @@ __global__ void layer_norm_rows_kernel(const __half* w, const __half* b, const T
             } else {
                 float g[8];
                 load8(gate + at, g);
+                activate_n(gate_act, g);
 #pragma unroll
-                for (int i = 0; i < 8; ++i) v[i] = activate_f(gate_act, g[i]) * __half2float(__float2half_rn(v[i]));
+                for (int i = 0; i < 8; ++i) v[i] = g[i] * __half2float(__float2half_rn(v[i]));
                 store8(gated + at, v);
             }
         }
@@ -425,6 +440,17 @@ bool blit_vec(const DView& input, const DView& output, cudaStream_t stream) {
     if (input.dtype == WRK_F32 && output.dtype == WRK_F16) return blit_typed<float, __half>(input, output, stream);
     if (input.dtype == WRK_F16 && output.dtype == WRK_F32) return blit_typed<__half, float>(input, output, stream);
     return false;
+}
+
+bool lerp_vec(const DView& input, const DView& output, const DView& factor, int reversed, cudaStream_t stream) {
+    __half *in, *out, *f;
+    if (!dense_as<__half>(input, &in) || !dense_as<__half>(output, &out) || !dense_as<__half>(factor, &f)) return false;
+    for (int i = 0; i < 3; ++i)
+        if (input.shape[i] != output.shape[i] || factor.shape[i] != output.shape[i]) return false;
+    const size_t total = (size_t)output.shape[0] * output.shape[1] * output.shape[2];
+    if (!fits32(total)) return false;
+    launch(lerp_vec_kernel, dim3(vec_grid(total / 8)), dim3(kVecThreads), 0, stream, in, out, f, (uint32_t)(total / 8), reversed);
+    return true;
 }
 
 namespace {

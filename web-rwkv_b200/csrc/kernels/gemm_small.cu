@@ -101,14 +101,44 @@ __global__ void __launch_bounds__(kSmallThreads) matmul_small_kernel(const Small
         }
     }
 
+    // The tile through shared memory (the operands have been read): eight rows of a token, adjacent elements of the output, per
+    // thread, stored as 16-byte pieces where the output's alignment allows it.
+    __syncthreads();
+    float(*st)[kTileM + 4] = reinterpret_cast<float(*)[kTileM + 4]>(&sx[0][0]);
+    static_assert(sizeof(float) * kTileN * (kTileM + 4) <= sizeof(sx), "the output tile takes the activations' place");
     // accumulator element e of n-tile j: row wm + g + 8 (e / 2), token wn + 8 j + 2 t4 + (e & 1)
 #pragma unroll
     for (int j = 0; j < 4; ++j)
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-            const uint32_t m = m0 + wm + g + 8 * (e >> 1), n = n0 + wn + j * 8 + 2 * t4 + (e & 1);
-            if (m < p.M && n < p.N) dstore(p.out.base, p.out.dtype, p.out.index(m, n, batch), activate_f(p.act, acc[j][e]));
+        for (int e = 0; e < 4; ++e) st[wn + j * 8 + 2 * t4 + (e & 1)][wm + g + 8 * (e >> 1)] = acc[j][e];
+    __syncthreads();
+#pragma unroll 1
+    for (uint32_t i = threadIdx.x; i < (uint32_t)kTileN * (kTileM / 8); i += kSmallThreads) {
+        const uint32_t n = n0 + i / (kTileM / 8), row = i % (kTileM / 8) * 8, m = m0 + row;
+        if (n >= p.N || m >= p.M) continue;
+        const float4 lo = *reinterpret_cast<const float4*>(&st[n - n0][row]), hi = *reinterpret_cast<const float4*>(&st[n - n0][row + 4]);
+        float v[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
+        activate_n(p.act, v);
+        const size_t at = p.out.index(m, n, batch);
+        const bool f16 = p.out.dtype == WRK_F16;
+        const uintptr_t to = reinterpret_cast<uintptr_t>(p.out.base) + at * (f16 ? 2 : 4);
+        if (m + 8 <= p.M && to % 16 == 0) {
+            if (f16) {
+                uint4 raw;
+                __half2* h = reinterpret_cast<__half2*>(&raw);
+#pragma unroll
+                for (int e = 0; e < 4; ++e) h[e] = __floats2half2_rn(v[2 * e], v[2 * e + 1]);
+                *reinterpret_cast<uint4*>(to) = raw;
+            } else {
+                reinterpret_cast<float4*>(to)[0] = make_float4(v[0], v[1], v[2], v[3]);
+                reinterpret_cast<float4*>(to)[1] = make_float4(v[4], v[5], v[6], v[7]);
+            }
+        } else {
+#pragma unroll
+            for (int e = 0; e < 8; ++e)
+                if (m + e < p.M) dstore(p.out.base, p.out.dtype, at + e, v[e]);
         }
+    }
 }
 
 }  // namespace

@@ -100,6 +100,8 @@ struct WkvArgs {
     int32_t* status;          // device status word
 };
 cudaError_t time_mix_v56(const WkvArgs& a, cudaStream_t stream);
+bool time_mix_v56_chunked_supported(const WkvArgs& a);
+cudaError_t time_mix_v56_chunked(const WkvArgs& a, cudaStream_t stream);
 cudaError_t time_mix_v7(const WkvArgs& a, cudaStream_t stream);
 cudaError_t time_mix_v4(const uint32_t* cursors, int wide, const float* time_decay, const float* time_first, DView state,
                         int dtype, const void* k, const void* v, const void* r, void* x, uint32_t C, uint32_t T,
@@ -119,6 +121,8 @@ cudaError_t rms_norm(const __half* w, const __half* b, int dtype, void* x, uint3
                      cudaStream_t stream);
 cudaError_t embed(const uint32_t* tokens, const __half* input, int dtype, void* output, uint32_t C, uint32_t rows,
                   uint32_t vocab, int32_t* status, cudaStream_t stream);
+// out[t] = table[tokens[t]] for rows of `row_pieces` 16-byte pieces; tokens and table may be pinned host memory
+cudaError_t gather_rows(const uint32_t* tokens, const void* table, void* out, uint32_t row_pieces, uint32_t rows, cudaStream_t stream);
 cudaError_t broadcast(DView input, DView output, cudaStream_t stream);
 cudaError_t blend(const float* factor, DView input, DView output, cudaStream_t stream);
 cudaError_t blend_lora(const float* factor, DView xa, DView xb, DView output, uint32_t K, cudaStream_t stream);
@@ -142,6 +146,7 @@ bool layer_norm_vec(const __half* w, const __half* b, int dtype, const void* del
 bool binary_vec(int is_mul, const DView& input, const DView& output, int act_x, int act_y, int act_out, cudaStream_t stream);
 bool activate_vec(const DView& x, int act, cudaStream_t stream);
 bool blit_vec(const DView& input, const DView& output, cudaStream_t stream);
+bool lerp_vec(const DView& input, const DView& output, const DView& factor, int reversed, cudaStream_t stream);
 // `bias`: null, or one row [C, 1, Z] added to the factors first (the sum rounded to f16, as a separate add stores it)
 bool token_shift_vec(const uint32_t* cursors, int wide, const DView& time_mix, const DView* bias, const DView& state,
                      const DView& input, const DView& output, int reversed, cudaStream_t stream);

@@ -163,6 +163,21 @@ __global__ void embed_kernel(const uint32_t* tokens, const __half* input, int dt
     }
 }
 
+// The embedding rows of a job's tokens, from pinned host memory over the bus: out[t] = table[tokens[t]], 16-byte pieces.
+__global__ void __launch_bounds__(256) gather_rows_kernel(const uint32_t* tokens, const uint4* table, uint4* out, uint32_t row_pieces) {
+    const uint4* src = table + (size_t)tokens[blockIdx.x] * row_pieces;
+    uint4* dst = out + (size_t)blockIdx.x * row_pieces;
+    for (uint32_t c = threadIdx.x; c < row_pieces; c += 4 * 256) {
+        uint4 v[4];  // in flight together: a round trip over the bus takes more than a microsecond
+#pragma unroll
+        for (uint32_t i = 0; i < 4; ++i)
+            if (c + i * 256 < row_pieces) v[i] = src[c + i * 256];
+#pragma unroll
+        for (uint32_t i = 0; i < 4; ++i)
+            if (c + i * 256 < row_pieces) dst[c + i * 256] = v[i];
+    }
+}
+
 // reshape.wgsl broadcast: output[c, t, b] = input[c, t % in.T, b % in.B].
 __global__ void broadcast_kernel(DView in, DView out) {
     pdl_launch_dependents();
@@ -286,9 +301,9 @@ __global__ void token_shift_multi_kernel(const ShiftMultiArgs a) {
 __global__ void pack_v7_kernel(const PackV7Args p) {
     pdl_launch_dependents();
     pdl_wait();
-    const uint32_t lane = threadIdx.x;
+    const uint32_t lane = threadIdx.x & 31, warps = blockDim.x / 32;
     const size_t plane = (size_t)p.rows * p.S;
-    for (uint32_t row = blockIdx.x; row < p.rows; row += gridDim.x) {
+    for (uint32_t row = blockIdx.x * warps + threadIdx.x / 32; row < p.rows; row += gridDim.x * warps) {
         const size_t base = (size_t)row * p.S;
         const uint32_t c0 = (row % p.H) * p.S;
         float s = 0.f;
@@ -480,6 +495,12 @@ cudaError_t embed(const uint32_t* tokens, const __half* input, int dtype, void* 
     return cudaGetLastError();
 }
 
+cudaError_t gather_rows(const uint32_t* tokens, const void* table, void* out, uint32_t row_pieces, uint32_t rows, cudaStream_t stream) {
+    if (rows == 0 || row_pieces == 0) return cudaSuccess;
+    gather_rows_kernel<<<rows, 256, 0, stream>>>(tokens, static_cast<const uint4*>(table), static_cast<uint4*>(out), row_pieces);
+    return cudaGetLastError();
+}
+
 cudaError_t broadcast(DView input, DView output, cudaStream_t stream) {
     const size_t total = (size_t)output.shape[0] * output.shape[1] * output.shape[2];
     if (total == 0) return cudaSuccess;
@@ -520,8 +541,9 @@ cudaError_t token_shift_multi(const ShiftMultiArgs& a, cudaStream_t stream) {
 
 cudaError_t pack_v7(const PackV7Args& p, cudaStream_t stream) {
     if (p.rows == 0 || p.S == 0) return cudaSuccess;
-    const uint32_t grid = p.rows < 148u * 32u ? p.rows : 148u * 32u;
-    launch(pack_v7_kernel, grid, dim3(32), 0, stream, p);
+    // eight rows per CTA where that still leaves a CTA for every SM (256 tokens of 64 heads in CTAs of a warp: 7.7 us)
+    const uint32_t warps = p.rows >= 8 * 148u ? 8 : 1, ctas = (p.rows + warps - 1) / warps;
+    launch(pack_v7_kernel, ctas < 148u * 32u ? ctas : 148u * 32u, dim3(32 * warps), 0, stream, p);
     return cudaGetLastError();
 }
 
@@ -569,6 +591,7 @@ cudaError_t blit(DView input, DView output, int transpose, cudaStream_t stream) 
 cudaError_t lerp(DView input, DView output, DView factor, int reversed, cudaStream_t stream) {
     const size_t total = (size_t)output.shape[0] * output.shape[1] * output.shape[2];
     if (total == 0) return cudaSuccess;
+    if (lerp_vec(input, output, factor, reversed, stream)) return cudaGetLastError();
     launch(lerp_kernel, dim3(ew_grid(total)), dim3(kEw), 0, stream, input, output, factor, reversed);
     return cudaGetLastError();
 }
