@@ -57,6 +57,23 @@ def test_int8_weights_distribution_and_edges(wrk, ctx):
     assert (q[0, :128] == 0).all() and (q[1, :128] == 0).all()
 
 
+def test_int8_weights_between_levels(wrk, ctx):
+    # weights at, just below and just above the middle between two levels, in blocks of many ranges; infinities and NaN
+    rng = np.random.default_rng(5)
+    m = (rng.integers(0, 511, (96, 256)) / 2.0).astype(np.float16)
+    m[:, ::128], m[:, 1::128] = 0.0, 255.0
+    m *= (2.0 ** rng.integers(-14, 8, (96, 1))).astype(np.float16)
+    bits = m.view(np.uint16)
+    bits[32:64] = np.where(bits[32:64] > 0, bits[32:64] - 1, 0)
+    bits[64:96] += 1
+    m[0, 5], m[1, 7], m[2, 9] = np.inf, -np.inf, np.nan
+    q, mm = _int8_roundtrip(wrk, ctx, m)
+    q_ref, mm_ref = oracle.quantize_mat_int8(m)
+    finite = np.isfinite(m.astype(np.float32)).reshape(-1, 128).all(axis=1)
+    assert np.array_equal(mm.view(np.uint16).reshape(-1, 2)[finite], mm_ref.view(np.uint16).reshape(-1, 2)[finite])
+    assert np.array_equal(q.reshape(-1, 128)[finite], q_ref.reshape(-1, 128)[finite])
+
+
 def test_int8_ragged_length(wrk, ctx):
     # total length not a multiple of 128 nor of 8: the last block is short
     rng = np.random.default_rng(3)

@@ -26,19 +26,36 @@ __device__ __forceinline__ void unpack8(const uint4& raw, float v[8]) {
     }
 }
 
+// The reference's level of a weight: floor(0.5 + 255 clamp((v - mn) / range)), every operation rounded to f32.
+__device__ __noinline__ uint32_t int8_level(float v, float mn, float range) {
+    float x = __fdiv_rn(__fsub_rn(v, mn), range);
+    x = (x > 0.0f) ? x : 0.0f;  // false for NaN: a degenerate block maps to 0
+    x = (x > 1.0f) ? 1.0f : x;
+    return (uint32_t)floorf(__fadd_rn(0.5f, __fmul_rn(255.0f, x))) & 0xffu;
+}
+
 // One lane handles 8 consecutive elements; 16 lanes share an Int8 block of 128.
+// A division per weight made this kernel instruction-bound.  t = (v - mn) (255 / range) is within 255 * 2^-22 < 7e-5 of the
+// exact 255 (v - mn) / range, and so is the reference's rounded 255 x: where 0.5 + t is at least 2^-12 away from a whole
+// number, both have the same floor.  The rest (one weight in 2000; every weight of a block without a range, and what
+// is not finite: the comparison is false for NaN) is divided.
 __global__ void __launch_bounds__(256) quantize_int8_kernel(const __half* __restrict__ input, size_t len,
                                                             __half* __restrict__ minmax,
                                                             uint8_t* __restrict__ output) {
     const size_t nvec = (len + 7) / 8;
     const size_t nvec_pad = (nvec + 15) / 16 * 16;  // whole 16-lane groups stay converged for the shuffles
-    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < nvec_pad;
-         i += (size_t)gridDim.x * blockDim.x) {
+    const size_t step = (size_t)gridDim.x * blockDim.x;
+    size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    uint4 next = make_uint4(0, 0, 0, 0);
+    if (i * 8 + 8 <= len) next = *reinterpret_cast<const uint4*>(input + i * 8);
+    for (; i < nvec_pad; i += step) {
         const size_t e0 = i * 8;
+        const uint4 raw = next;
+        if ((i + step) * 8 + 8 <= len) next = *reinterpret_cast<const uint4*>(input + (i + step) * 8);  // while this one is packed
         float v[8];
         int valid = 0;
         if (e0 + 8 <= len) {
-            unpack8(*reinterpret_cast<const uint4*>(input + e0), v);
+            unpack8(raw, v);
             valid = 8;
         } else if (e0 < len) {
             valid = (int)(len - e0);
@@ -61,15 +78,13 @@ __global__ void __launch_bounds__(256) quantize_int8_kernel(const __half* __rest
             const size_t blk = e0 / 128;
             reinterpret_cast<__half2*>(minmax)[blk] = __floats2half2_rn(mn, mx);
         }
-        const float range = __fsub_rn(mx, mn);
+        const float range = __fsub_rn(mx, mn), scale = __fdiv_rn(255.0f, range);
         uint32_t packed[2] = {0u, 0u};
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
-            float x = __fdiv_rn(__fsub_rn(v[j], mn), range);
-            x = (x > 0.0f) ? x : 0.0f;  // false for NaN: a degenerate block maps to 0
-            x = (x > 1.0f) ? 1.0f : x;
-            const float q = floorf(__fadd_rn(0.5f, __fmul_rn(255.0f, x)));
-            packed[j >> 2] |= ((uint32_t)q & 0xffu) << ((j & 3) * 8);
+            const float t = __fadd_rn(0.5f, __fmul_rn(__fsub_rn(v[j], mn), scale)), q = floorf(t), f = __fsub_rn(t, q);
+            const uint32_t level = fabsf(__fsub_rn(f, 0.5f)) < 0.5f - 0x1p-12f ? (uint32_t)q : int8_level(v[j], mn, range);
+            packed[j >> 2] |= level << ((j & 3) * 8);
         }
         if (valid == 8) {
             *reinterpret_cast<uint2*>(output + e0) = make_uint2(packed[0], packed[1]);
