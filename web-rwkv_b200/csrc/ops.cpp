@@ -230,6 +230,11 @@ double reg_inc_beta(double a, double b, double x) {
 // Distribution function of Student's t with nu degrees of freedom, and its inverse by bisection (monotone, 200
 // halvings of a bracket that doubles until it contains the root: exact to the last bit of a double).
 double student_cdf(double t, double nu) {
+    if (blocks && k::time_mix_v56_chunked_supported(a)) {
+        *out = new_atom(name, [a](cudaStream_t s) { return k::time_mix_v56_chunked(a, s); },
+                        {cursors, time_decay, time_first, state->tensor, k, v, r, x});
+        return WRK_OK;
+    }
     const double tail = 0.5 * reg_inc_beta(0.5 * nu, 0.5, nu / (nu + t * t));
     return t >= 0.0 ? 1.0 - tail : tail;
 }
