@@ -265,3 +265,45 @@ def test_group_of_matrices_in_one_launch(wrk, ctx, kind, n):
         assert_close(y.numpy().reshape(n, M), want, f"group {kind} M={M}")
         assert_close(y.numpy().reshape(n, M), single.numpy().reshape(n, M), f"group vs single {kind} M={M}")
     assert ctx.device_status() == 0
+
+
+@pytest.mark.parametrize("n", [1, 3, 8])
+def test_group_of_few_tokens_streams_in_one_launch(wrk, ctx, n):
+    """Matrices of different formats, widths and heights (below and above the number of CTAs): one weight-streaming launch
+    with the single ops' results; a group in which one matmul reads another's output keeps its order."""
+    rng = np.random.default_rng(170 + n)
+    shapes, acts = [("fp16", 1024, 64), ("int8", 1024, 1000), ("fp16", 64, 512), ("int8", 256, 33)], [wrk.ACT_TANH, wrk.ACT_NONE, wrk.ACT_SIGMOID, wrk.ACT_NONE]
+    mats, xs, ys, singles = [], [], [], []
+    for kind, K, M in shapes:
+        mats.append(_make_matrix(wrk, ctx, kind, (rng.standard_normal((M, K), dtype=np.float32) * 0.02).astype(np.float16))[0])
+        xs.append(ctx.from_numpy(rng.standard_normal((n, K), dtype=np.float32).astype(np.float16)))
+        ys.append(ctx.tensor(wrk.F16, [M, n]))
+        singles.append(ctx.tensor(wrk.F16, [M, n]))
+    before = ctx.launch_count()
+    ctx.run(wrk.matmul_group_op(mats, xs, ys, acts, turbo=False))
+    assert ctx.launch_count() - before == 1
+    for mat, x, y, act in zip(mats, xs, singles, acts):
+        ctx.run(mat.matmul_op(x, y, act=act))
+    for y, single in zip(ys, singles):
+        assert np.array_equal(y.numpy(), single.numpy())  # a row's sum does not depend on the CTA that forms it
+    chained = ctx.tensor(wrk.F16, [512, n])
+    before = ctx.launch_count()
+    ctx.run(wrk.matmul_group_op([mats[0], mats[2]], [xs[0], ys[0]], [ys[0], chained], [acts[0], acts[2]], turbo=False))
+    assert ctx.launch_count() - before == 2
+    again = ctx.tensor(wrk.F16, [512, n])
+    ctx.run(mats[2].matmul_op(ys[0], again, act=acts[2]))
+    assert np.array_equal(chained.numpy(), again.numpy())
+
+
+@pytest.mark.parametrize("kind", ["int8", "nf4", "fp16"])
+@pytest.mark.parametrize("n", [5, 8])
+def test_few_tokens_of_a_long_k(wrk, ctx, kind, n):
+    # activations that one launch's shared memory does not hold: the tokens are shared out over launches
+    rng = np.random.default_rng(190 + n)
+    K, M = 18432, 80
+    mat, (okind, om, oscale) = _make_matrix(wrk, ctx, kind, (rng.standard_normal((M, K), dtype=np.float32) * 0.02).astype(np.float16))
+    x = rng.standard_normal((n, K), dtype=np.float32).astype(np.float16)
+    y, want = ctx.tensor(wrk.F32, [M, n]), np.zeros((n, M), dtype=np.float32)
+    ctx.run(mat.matmul_op(ctx.from_numpy(x), y))
+    oracle.matmul(okind, om, oscale, x, want)
+    assert_close(y.numpy().reshape(n, M), want, f"{kind} n={n}")

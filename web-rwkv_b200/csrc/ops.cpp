@@ -88,58 +88,106 @@ int32_t matmul_args(int kind, wrk_tensor* matrix, wrk_tensor* scale, wrk_tensor*
     return WRK_OK;
 }
 
+// A matmul of few tokens, fp16 activations and whole rows: what the weight-streaming kernel of the decode path takes.
+bool streams(const k::MatmulArgs& a) {
+    const uint32_t need = a.kind == k::MAT_FP16 ? 32 : 128;
+    return a.B == 1 && a.N >= 1 && a.N <= (uint32_t)k::kDecodeMaxTokens && a.in.dtype == WRK_F16 && a.K % need == 0 &&
+           a.in.index(0, 0, 0) % 8 == 0 && a.in.stride[0] % 8 == 0;
+}
+
+// Tokens t0 .. t0 + n of `count` matmuls as one weight-streaming launch; *out stays null when it cannot take them together.
+int32_t stream_op(const char* name, wrk_context* ctx, const k::MatmulArgs* args, uint32_t count, uint32_t t0, uint32_t n,
+                  const std::vector<wrk_tensor*>& weights, const std::vector<wrk_tensor*>& tensors, wrk_op** out) {
+    *out = nullptr;
+    const int sms = ctx->num_sms;
+    k::FusedGemvArgs f{};
+    f.T = n;
+    f.prologue = k::PRO_NONE;
+    f.epilogue = k::EPI_STORE;
+    f.status = ctx->device_status;
+    f.rescale = 1.0f;
+    f.num_problems = (int)count;
+    for (uint32_t i = 0; i < count; ++i) {
+        const k::MatmulArgs& a = args[i];
+        if (a.table != nullptr) {
+            if (f.table != nullptr && f.table != a.table) return WRK_OK;  // a launch has one code book
+            f.table = a.table;
+        }
+        f.C = std::max(f.C, a.K);
+        const size_t in0 = a.in.index(0, t0, 0), out0 = a.out.index(0, t0, 0);
+        k::GemvProblem& p = f.p[i];
+        p.w = static_cast<const uint8_t*>(a.matrix);
+        p.scale = a.scale;
+        p.kind = a.kind;
+        p.K = a.K;
+        p.M = a.M;
+        p.x = static_cast<const __half*>(a.in.base) + in0;
+        p.x_stride = a.in.stride[0];
+        p.out = a.out.dtype == WRK_F16 ? static_cast<void*>(static_cast<__half*>(a.out.base) + out0)
+                                       : static_cast<void*>(static_cast<float*>(a.out.base) + out0);
+        p.out_stride = a.out.stride[0];
+        p.out_dtype = a.out.dtype;
+        p.act = a.act;
+    }
+    std::vector<k::GemvSegment> table;
+    if (!k::fused_gemv_partition(f, sms, table)) return WRK_OK;
+    const uint32_t tshape[4] = {(uint32_t)(table.size() * 4), 1, 1, 1};
+    wrk_tensor* tt = nullptr;
+    WRK_TRY(wrk_tensor_from_data(ctx, WRK_U32, tshape, table.data(), table.size() * sizeof(k::GemvSegment), &tt));
+    f.segments = static_cast<const k::GemvSegment*>(tt->ptr());
+    k::fused_gemv_inline_partition(f, sms, table);
+    *out = new_atom(name, [f, sms](cudaStream_t s) { return k::fused_gemv(f, sms, s); }, {tt});
+    wrk_tensor_release(tt);  // the atom keeps the buffer alive
+    for (wrk_tensor* t : weights) {
+        if (t == nullptr || !t->buf) continue;
+        (*out)->keep.push_back(t->buf);
+        add_early(*out, {t});
+    }
+    for (wrk_tensor* t : tensors)
+        if (t->buf) (*out)->keep.push_back(t->buf);
+    return WRK_OK;
+}
+
+// Tokens of one weight-streaming launch over `k` columns: its shared memory holds all their activations.
+uint32_t stream_tokens(uint32_t n, uint32_t k) {
+    while (n > 0 && k::fused_gemv_smem(n, k, k, k::PRO_NONE, 2) > 200 * 1024) --n;
+    return n;
+}
+
 int32_t matmul_common(const char* name, int kind, wrk_tensor* matrix, wrk_tensor* scale, wrk_tensor* quant,
                       const wrk_view* input, const wrk_view* output, int32_t act, wrk_op** out) {
     REQ_NN(out);
     k::MatmulArgs a;
     WRK_TRY(matmul_args(kind, matrix, scale, quant, input, output, act, &a));
-    const uint32_t m = a.M, n = a.N, b = a.B, k = a.K;
-    (void)m;
-    const int sms = matrix->ctx->num_sms;
-    // few tokens, fp16 activations, whole rows: the weight-streaming kernel of the decode path
-    const uint32_t need = kind == k::MAT_FP16 ? 32 : 128;
-    const size_t in_row0 = a.in.index(0, 0, 0), out_row0 = a.out.index(0, 0, 0);
-    const bool stream_ok = b == 1 && n >= 1 && n <= (uint32_t)k::kDecodeMaxTokens && a.in.dtype == WRK_F16 &&
-                           k % need == 0 && in_row0 % 8 == 0 && a.in.stride[0] % 8 == 0 &&
-                           k::fused_gemv_smem(n, k, k, k::PRO_NONE, 2) <= 200 * 1024;
-    if (stream_ok) {
-        k::FusedGemvArgs f{};
-        f.T = n;
-        f.C = k;
-        f.prologue = k::PRO_NONE;
-        f.epilogue = k::EPI_STORE;
-        f.table = a.table;
-        f.status = matrix->ctx->device_status;
-        f.rescale = 1.0f;
-        f.num_problems = 1;
-        k::GemvProblem& p = f.p[0];
-        p.w = static_cast<const uint8_t*>(a.matrix);
-        p.scale = a.scale;
-        p.kind = kind;
-        p.K = k;
-        p.M = m;
-        p.x = static_cast<const __half*>(a.in.base) + in_row0;
-        p.x_stride = a.in.stride[0];
-        p.out = a.out.dtype == WRK_F16 ? static_cast<void*>(static_cast<__half*>(a.out.base) + out_row0)
-                                       : static_cast<void*>(static_cast<float*>(a.out.base) + out_row0);
-        p.out_stride = a.out.stride[0];
-        p.out_dtype = a.out.dtype;
-        p.act = act;
-        std::vector<k::GemvSegment> table;
-        if (k::fused_gemv_partition(f, sms, table)) {
-            const uint32_t tshape[4] = {(uint32_t)(table.size() * 4), 1, 1, 1};
-            wrk_tensor* tt = nullptr;
-            WRK_TRY(wrk_tensor_from_data(matrix->ctx, WRK_U32, tshape, table.data(),
-                                         table.size() * sizeof(k::GemvSegment), &tt));
-            f.segments = static_cast<const k::GemvSegment*>(tt->ptr());
-            k::fused_gemv_inline_partition(f, sms, table);
-            *out = new_atom(name, [f, sms](cudaStream_t s) { return k::fused_gemv(f, sms, s); },
-                            {matrix, scale, quant, input->tensor, output->tensor, tt});
-            wrk_tensor_release(tt);  // the atom keeps the buffer alive
-            add_early(*out, {matrix, scale, quant});
-            return WRK_OK;
+    if (streams(a)) {
+        // A long K: as few launches as hold the tokens, of about the same number each (8 tokens of a 14336 -> 4096 Int8 matrix:
+        // two launches of 4; the mma.sync kernel below, which stages a part of K at a time, took 92 us).  Not where the
+        // outputs might overwrite activations that a later launch reads.
+        const uint32_t most = stream_tokens(a.N, a.K), parts = most ? (a.N + most - 1) / most : 0;
+        if (parts == 1 || (parts > 1 && input->tensor->buf != output->tensor->buf)) {
+            std::vector<wrk_op*> ops;
+            int32_t status = WRK_OK;
+            for (uint32_t i = 0; i < parts && status == WRK_OK; ++i) {
+                const uint32_t t0 = a.N * i / parts, t1 = a.N * (i + 1) / parts;
+                wrk_op* o = nullptr;
+                status = stream_op(name, matrix->ctx, &a, 1, t0, t1 - t0, {matrix, scale, quant}, {input->tensor, output->tensor}, &o);
+                if (o == nullptr) break;
+                ops.push_back(o);
+            }
+            if (status == WRK_OK && ops.size() == parts) {
+                if (parts == 1) {
+                    *out = ops[0];
+                    return WRK_OK;
+                }
+                status = wrk_op_list(ops.data(), ops.size(), out);
+                for (wrk_op* o : ops) wrk_op_release(o);
+                return status;
+            }
+            for (wrk_op* o : ops) wrk_op_release(o);
+            if (status != WRK_OK) return status;
         }
     }
+    const int sms = matrix->ctx->num_sms;
     *out = new_atom(name, [a, sms](cudaStream_t s) { return k::matmul(a, sms, s); },
                     {matrix, scale, quant, input->tensor, output->tensor});
     add_early(*out, {matrix, scale, quant});
@@ -182,6 +230,11 @@ int32_t time_mix_v56(const char* name, int per_token, wrk_tensor* cursors, wrk_t
     a.k = k->ptr(); a.v = v->ptr(); a.r = r->ptr(); a.x = x->ptr();
     a.status = x->ctx->device_status;
     if (blocks) WRK_REQUIRE(S == 64, WRK_ERR_UNSUPPORTED, "time_mix_blocks takes heads of 64 channels");
+    if (blocks && k::time_mix_v56_chunked_supported(a)) {
+        *out = new_atom(name, [a](cudaStream_t s) { return k::time_mix_v56_chunked(a, s); },
+                        {cursors, time_decay, time_first, state->tensor, k, v, r, x});
+        return WRK_OK;
+    }
     *out = new_atom(name, [a](cudaStream_t s) { return k::time_mix_v56(a, s); },
                     {cursors, time_decay, time_first, state->tensor, k, v, r, x});
     return WRK_OK;
@@ -230,11 +283,6 @@ double reg_inc_beta(double a, double b, double x) {
 // Distribution function of Student's t with nu degrees of freedom, and its inverse by bisection (monotone, 200
 // halvings of a bracket that doubles until it contains the root: exact to the last bit of a double).
 double student_cdf(double t, double nu) {
-    if (blocks && k::time_mix_v56_chunked_supported(a)) {
-        *out = new_atom(name, [a](cudaStream_t s) { return k::time_mix_v56_chunked(a, s); },
-                        {cursors, time_decay, time_first, state->tensor, k, v, r, x});
-        return WRK_OK;
-    }
     const double tail = 0.5 * reg_inc_beta(0.5 * nu, 0.5, nu / (nu + t * t));
     return t >= 0.0 ? 1.0 - tail : tail;
 }
@@ -1143,15 +1191,23 @@ int32_t wrk_matrix_matmul_group_op(wrk_matrix* const* matrices, const wrk_view* 
     REQ_NN(matrices, inputs, outputs, acts, out);
     WRK_REQUIRE(count >= 1 && count <= 4, WRK_ERR_INVALID_ARGUMENT, "a group holds 1 to 4 matrices, not %u", count);
     k::MatmulArgs args[4];
-    bool one_launch = turbo != 0;
-    for (uint32_t i = 0; i < count && one_launch; ++i) {
+    bool gemm = turbo != 0, stream = true;
+    uint32_t kmax = 0;
+    std::vector<wrk_tensor*> weights, tensors;
+    for (uint32_t i = 0; i < count; ++i) {
         wrk_matrix* m = matrices[i];
         REQ_NN(m);
         const int kind = m->kind == 0 ? k::MAT_FP16 : m->kind == 1 ? k::MAT_INT8 : k::MAT_NF4;
         WRK_TRY(matmul_args(kind, m->w, m->m, m->q, &inputs[i], &outputs[i], acts[i], &args[i]));
+        kmax = std::max(kmax, args[i].K);
+        stream = stream && streams(args[i]) && args[i].N == args[0].N;
+        for (uint32_t j = 0; j < i; ++j)
+            stream = stream && inputs[i].tensor->buf != outputs[j].tensor->buf && inputs[j].tensor->buf != outputs[i].tensor->buf;
+        weights.insert(weights.end(), {m->w, m->m, m->q});
+        tensors.insert(tensors.end(), {inputs[i].tensor, outputs[i].tensor});
     }
-    one_launch = one_launch && k::matmul_umma_group_supported(args, (int)count);
-    if (one_launch) {
+    gemm = gemm && k::matmul_umma_group_supported(args, (int)count);
+    if (gemm) {
         std::vector<k::MatmulArgs> all(args, args + count);
         int32_t* status = args[0].status;
         wrk_op* op = new_atom("matmul_group", [all, status](cudaStream_t s) { return k::matmul_umma_group(all.data(), (int)all.size(), status, s); },
@@ -1163,6 +1219,10 @@ int32_t wrk_matrix_matmul_group_op(wrk_matrix* const* matrices, const wrk_view* 
         }
         *out = op;
         return WRK_OK;
+    }
+    if (stream && stream_tokens(args[0].N, kmax) == args[0].N) {
+        WRK_TRY(stream_op("matmul_group", matrices[0]->w->ctx, args, count, 0, args[0].N, weights, tensors, out));
+        if (*out != nullptr) return WRK_OK;
     }
     // shapes the grouped kernel does not take: the same work as a list of single matmuls
     std::vector<wrk_op*> ops;

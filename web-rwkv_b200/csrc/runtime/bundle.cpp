@@ -70,6 +70,7 @@ struct wrk_bundle {
     size_t stage_tokens = 0;
     std::mutex mutex;
     ~wrk_bundle() {
+        if (model) cudaStreamSynchronize(model->ctx->stream);  // a loaded job may still read the staging buffers and the embedding table
         jobs.clear();
         if (stage_input) cudaFreeHost(stage_input);
         if (stage_cursors) cudaFreeHost(stage_cursors);
@@ -254,6 +255,12 @@ struct GroupItem {
     wrk_view in, out;
     int32_t act;
 };
+// A group with `turbo` asks for the tensor-core kernel, one of up to 8 tokens without it gets a weight-streaming launch.
+// v5 and v7 ask for it from 16 tokens on (9 to 15: a launch per matrix; the tests count the launches of such a job), v6 for
+// whole chunks of 32 only: a group splits K less than its matrices would alone, and the order of the sums shows in the
+// states of a deep v6 model.  Measured: 16 tokens of a 2048-wide fp16 v5 model of twelve layers, 97 GEMM launches of
+// 6.3 us -> 49 of 9.0 us; one token of eight 4096-wide Int8 v7 layers, 111 streaming launches of 7.5 us -> 49 of 13.1 us;
+// 64 tokens of those, the adapters' first matrices 325 us as 31 launches -> 155 us as 8.
 int32_t matmul_group(OpList& ops, std::initializer_list<GroupItem> items, bool turbo) {
     wrk_matrix* ms[4];
     wrk_view ins[4], outs[4];
@@ -509,7 +516,7 @@ int32_t layer_v56(wrk_bundle* bd, OpList& ops, const Buffers& B, uint32_t index,
         WRK_TRY(matmul_group(ops, {{L.att_w_k, V(B["att_kx"]), V(B["att_k"]), WRK_ACT_NONE},
                                    {L.att_w_v, V(B["att_vx"]), V(B["att_v"]), WRK_ACT_NONE},
                                    {L.att_w_r, V(B["att_rx"]), V(B["att_r"]), WRK_ACT_NONE},
-                                   {L.att_w_g, V(B["att_gx"]), V(B["att_g"]), WRK_ACT_NONE}}, turbo));
+                                   {L.att_w_g, V(B["att_gx"]), V(B["att_g"]), WRK_ACT_NONE}}, T >= 16));
     } else {
         WRK_TRY(token_shift(ops, cursors, V(L.time_mix_k), state_att(bd, index, S), B["att_x"], B["att_kx"], false));
         WRK_TRY(token_shift(ops, cursors, V(L.time_mix_v), state_att(bd, index, S), B["att_x"], B["att_vx"], false));
@@ -571,7 +578,7 @@ int32_t layer_v56(wrk_bundle* bd, OpList& ops, const Buffers& B, uint32_t index,
     HOOK(PRE_FFN_LINEAR);
     if (merged) {  // key and receptance read different shifts of one input: one launch; value follows
         WRK_TRY(matmul_group(ops, {{L.ffn_w_k, V(B["ffn_kx"]), V(B["ffn_k"]), WRK_ACT_SQUARED_RELU},
-                                   {L.ffn_w_r, V(B["ffn_rx"]), V(B["ffn_r"]), WRK_ACT_NONE}}, turbo));
+                                   {L.ffn_w_r, V(B["ffn_rx"]), V(B["ffn_r"]), WRK_ACT_NONE}}, v6 ? turbo : T >= 16));
     } else {
         WRK_TRY(matmul(ops, L.ffn_w_k, V(B["ffn_kx"]), V(B["ffn_k"]), WRK_ACT_SQUARED_RELU, turbo));
         HOOK(POST_FFN_ACTIVATE);
@@ -640,7 +647,7 @@ int32_t layer_v7(wrk_bundle* bd, OpList& ops, const Buffers& B, uint32_t index, 
     if (merged) {
         WRK_TRY(matmul_group(ops, {{L.att_w_r, V(B["att_rx"]), V(B["att_r"]), WRK_ACT_NONE},
                                    {L.att_w_k, V(B["att_kx"]), V(B["att_k"]), WRK_ACT_NONE},
-                                   {L.att_w_v, V(B["att_vx"]), V(B["att_v"]), WRK_ACT_NONE}}, turbo));
+                                   {L.att_w_v, V(B["att_vx"]), V(B["att_v"]), WRK_ACT_NONE}}, T >= 16));
     } else {
         WRK_TRY(matmul(ops, L.att_w_r, V(B["att_rx"]), V(B["att_r"]), WRK_ACT_NONE, turbo));
         WRK_TRY(matmul(ops, L.att_w_k, V(B["att_kx"]), V(B["att_k"]), WRK_ACT_NONE, turbo));
@@ -648,14 +655,30 @@ int32_t layer_v7(wrk_bundle* bd, OpList& ops, const Buffers& B, uint32_t index, 
     }
     HOOK(POST_ATT_LINEAR);
     HOOK(PRE_ATT_ADAPT);
-    WRK_TRY(matmul(ops, L.w1, V(B["att_wx"]), V(B["aux_w"]), WRK_ACT_TANH, turbo));
-    WRK_TRY(matmul(ops, L.w2, V(B["aux_w"]), V(B["att_w"]), WRK_ACT_NONE, turbo));
-    WRK_TRY(add(ops, V(L.w0), V(B["att_w"])));
-    WRK_TRY(matmul(ops, L.a1, V(B["att_ax"]), V(B["aux_a"]), WRK_ACT_NONE, turbo));
-    WRK_TRY(matmul(ops, L.a2, V(B["aux_a"]), V(B["att_a"]), WRK_ACT_NONE, turbo));
-    WRK_TRY(add(ops, V(L.a0), V(B["att_a"]), WRK_ACT_SIGMOID));
-    WRK_TRY(matmul(ops, L.g1, V(B["att_gx"]), V(B["aux_g"]), WRK_ACT_SIGMOID, turbo));
-    WRK_TRY(matmul(ops, L.g2, V(B["aux_g"]), V(B["att_g"]), WRK_ACT_NONE, turbo));
+    if (merged) {  // the adapters' first matrices together, then their second ones (the value residual's among them)
+        const GroupItem w1{L.w1, V(B["att_wx"]), V(B["aux_w"]), WRK_ACT_TANH}, a1{L.a1, V(B["att_ax"]), V(B["aux_a"]), WRK_ACT_NONE},
+            g1{L.g1, V(B["att_gx"]), V(B["aux_g"]), WRK_ACT_SIGMOID};
+        const GroupItem w2{L.w2, V(B["aux_w"]), V(B["att_w"]), WRK_ACT_NONE}, a2{L.a2, V(B["aux_a"]), V(B["att_a"]), WRK_ACT_NONE},
+            g2{L.g2, V(B["aux_g"]), V(B["att_g"]), WRK_ACT_NONE};
+        if (index == 0) {
+            WRK_TRY(matmul_group(ops, {w1, a1, g1}, T >= 16));
+            WRK_TRY(matmul_group(ops, {w2, a2, g2}, T >= 16));
+        } else {
+            WRK_TRY(matmul_group(ops, {w1, a1, g1, {L.v1, V(B["att_vx"]), V(B["aux_v"]), WRK_ACT_NONE}}, T >= 16));
+            WRK_TRY(matmul_group(ops, {w2, a2, g2, {L.v2, V(B["aux_v"]), V(B["att_vv"]), WRK_ACT_NONE}}, T >= 16));
+        }
+        WRK_TRY(add(ops, V(L.w0), V(B["att_w"])));
+        WRK_TRY(add(ops, V(L.a0), V(B["att_a"]), WRK_ACT_SIGMOID));
+    } else {
+        WRK_TRY(matmul(ops, L.w1, V(B["att_wx"]), V(B["aux_w"]), WRK_ACT_TANH, turbo));
+        WRK_TRY(matmul(ops, L.w2, V(B["aux_w"]), V(B["att_w"]), WRK_ACT_NONE, turbo));
+        WRK_TRY(add(ops, V(L.w0), V(B["att_w"])));
+        WRK_TRY(matmul(ops, L.a1, V(B["att_ax"]), V(B["aux_a"]), WRK_ACT_NONE, turbo));
+        WRK_TRY(matmul(ops, L.a2, V(B["aux_a"]), V(B["att_a"]), WRK_ACT_NONE, turbo));
+        WRK_TRY(add(ops, V(L.a0), V(B["att_a"]), WRK_ACT_SIGMOID));
+        WRK_TRY(matmul(ops, L.g1, V(B["att_gx"]), V(B["aux_g"]), WRK_ACT_SIGMOID, turbo));
+        WRK_TRY(matmul(ops, L.g2, V(B["aux_g"]), V(B["att_g"]), WRK_ACT_NONE, turbo));
+    }
     HOOK(POST_ATT_ADAPT);
     HOOK(PRE_ATT_CONTROL);
     if (!merged) {
@@ -675,8 +698,10 @@ int32_t layer_v7(wrk_bundle* bd, OpList& ops, const Buffers& B, uint32_t index, 
     if (index == 0) {
         WRK_TRY(blit(ops, V(B["att_v"]), V(B["att_v0"])));
     } else {
-        WRK_TRY(matmul(ops, L.v1, V(B["att_vx"]), V(B["aux_v"]), WRK_ACT_NONE, turbo));
-        WRK_TRY(matmul(ops, L.v2, V(B["aux_v"]), V(B["att_vv"]), WRK_ACT_NONE, turbo));
+        if (!merged) {
+            WRK_TRY(matmul(ops, L.v1, V(B["att_vx"]), V(B["aux_v"]), WRK_ACT_NONE, turbo));
+            WRK_TRY(matmul(ops, L.v2, V(B["aux_v"]), V(B["att_vv"]), WRK_ACT_NONE, turbo));
+        }
         WRK_TRY(add(ops, V(L.v0), V(B["att_vv"]), WRK_ACT_SIGMOID));
         const wrk_view in = V(B["att_v0"]), out = V(B["att_v"]), f = V(B["att_vv"]);
         ADD(wrk_op_lerp(&in, &out, &f, 1, &_o));
@@ -1809,13 +1834,23 @@ int32_t wrk_job_load(wrk_job* job, const uint32_t* tokens, size_t count) {
     WRK_TRY(upload_cursors(job));
     // the previous upload from the staging buffers must have been consumed
     WRK_CUDA(cudaStreamSynchronize(ctx->stream));
-    for (uint32_t t = 0; t < T; ++t) {
-        const uint32_t tok = tokens[t];
-        WRK_REQUIRE(tok < m->num_vocab_padded, WRK_ERR_INVALID_ARGUMENT, "token %u out of vocabulary %u", tok,
+    for (uint32_t t = 0; t < T; ++t)
+        WRK_REQUIRE(tokens[t] < m->num_vocab_padded, WRK_ERR_INVALID_ARGUMENT, "token %u out of vocabulary %u", tokens[t],
                     m->num_vocab_padded);
-        std::memcpy(b->stage_input + (size_t)t * C, m->embed_host + (size_t)tok * C, (size_t)C * 2);
-    }
     const Buffers& B = *job->job->buffer;
+    // From 16 tokens on the device fetches the rows itself, from the pinned table, while the host submits the job (a job of 256
+    // rows of 8 KB ends 0.1 ms earlier than with rows copied by the host and sent); a few rows cost the host less than
+    // the kernel's two round trips over the bus.
+    if (T >= 16 && C % 8 == 0) {
+        uint32_t* ids = reinterpret_cast<uint32_t*>(b->stage_input);
+        std::memcpy(ids, tokens, (size_t)T * sizeof(uint32_t));
+        WRK_CUDA(cudaSetDevice(ctx->device));
+        WRK_CUDA(k::gather_rows(ids, m->embed_host, B["input"]->ptr(), C / 8, T, ctx->stream));
+        ctx->launches.fetch_add(1);
+        return WRK_OK;
+    }
+    for (uint32_t t = 0; t < T; ++t)
+        std::memcpy(b->stage_input + (size_t)t * C, m->embed_host + (size_t)tokens[t] * C, (size_t)C * 2);
     WRK_CUDA(cudaMemcpyAsync(B["input"]->ptr(), b->stage_input, (size_t)T * C * 2, cudaMemcpyHostToDevice, ctx->stream));
     return WRK_OK;
 }
