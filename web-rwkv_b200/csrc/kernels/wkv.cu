@@ -366,7 +366,7 @@ __global__ void __launch_bounds__(256) time_mix_v56_chunked_kernel(const WkvArgs
                 const float4 rq = *reinterpret_cast<const float4*>(&sr[s2][4 * cj]);
                 red[(s2 * L + s2) * 16 + cj] = (rq.x * kk[0] * u4[0] + rq.y * kk[1] * u4[1]) + (rq.z * kk[2] * u4[2] + rq.w * kk[3] * u4[3]);
             }
-#pragma unroll 5
+            // (not unrolled by hand: a peeled first step, d = 1, would let the compiler fuse other products)
             for (uint32_t t = s2 + 1; t < L; ++t) {
                 const float4 rq = *reinterpret_cast<const float4*>(&sr[t][4 * cj]);
                 const float4 wq = *reinterpret_cast<const float4*>(&sw[t][4 * cj]);
