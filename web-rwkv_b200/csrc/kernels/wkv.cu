@@ -241,7 +241,7 @@ __global__ void __launch_bounds__((S / 4) * (NC / 4)) time_mix_v56_kernel(const 
 // Two CTAs of 256 threads per (head of 64 channels, batch slot), each with 32 of the state's columns, which do not depend on one
 // another (both form A and the decay products); the state tile of a thread stays in registers from block to block; the
 // tokens' rows are staged a block ahead as in the serial kernel.  Every element is summed in the order that one CTA per head
-// took, so its bits are the same.  256 tokens of 64 heads: 76 -> 68 us.
+// took, so its bits are the same.  256 tokens of 64 heads: 76 -> 68 us, and 53 with the loads of a block in flight together.
 // The serial kernel above is faster (35 us), but it sums in another order, and what that changes in the last bit of a
 // state grows through the layers of a deep model (24 layers of random weights: to 1e-2 of the last layer's state).
 constexpr int kBlockTokens = 16;
