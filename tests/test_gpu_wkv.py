@@ -131,9 +131,9 @@ def test_v6_long_runs_cross_chunks(wrk, ctx):
     assert_close(gs, rs, "state")
 
 
-@pytest.mark.parametrize("head_size", [32, 64, 128])
+@pytest.mark.parametrize("head_size,blocks", [(32, False), (64, False), (64, True), (128, False)])
 @pytest.mark.parametrize("alias", ["k", "r", "v"])
-def test_v6_output_over_an_input(wrk, ctx, head_size, alias):
+def test_v6_output_over_an_input(wrk, ctx, head_size, blocks, alias):
     """The outputs may replace k, r or v: heads are then not shared out among CTAs where every CTA reads that input.
     Runs around the four tokens that are summed together and the 8 or 16 of a chunk."""
     rng = np.random.default_rng(70 + head_size)
@@ -145,8 +145,8 @@ def test_v6_output_over_an_input(wrk, ctx, head_size, alias):
     state = (rng.standard_normal((B, S + 2, S * H)) * 0.1).astype(np.float32)
     dev = {n: ctx.from_numpy(v) for n, v in t.items()}
     t_state = ctx.from_numpy(state)
-    ctx.run(wrk.time_mix_v6(ctx.from_numpy(cursors), ctx.from_numpy(w), ctx.from_numpy(u), t_state.view(y=(0, S + 1)), dev["k"], dev["v"],
-                            dev["r"], dev[alias]))
+    args = (ctx.from_numpy(cursors), ctx.from_numpy(w), ctx.from_numpy(u), t_state.view(y=(0, S + 1)), dev["k"], dev["v"], dev["r"], dev[alias])
+    ctx.run(wrk.time_mix_blocks(True, *args) if blocks else wrk.time_mix_v6(*args))
     ref_x, ref_state = t[alias].copy(), state.copy()
     oracle.time_mix_v56(True, cursors, w, u, oracle.View(ref_state, y=(0, S + 1)), t["k"], t["v"], t["r"], ref_x, S, H)
     assert_close(dev[alias].numpy().reshape(T, H, S), ref_x, "x")

@@ -2,12 +2,10 @@
 //
 // Replaces time_mix_v5.wgsl, time_mix_v6.wgsl and time_mix_v7.wgsl.  The reference runs one
 // dispatch with C/4 threads that is serial over every token of the job and round-trips the whole
-// S x S state through global memory on each token.  Here one CTA of S threads owns one
-// (sequence, head) pair: thread j keeps column j of the head's state (S fp32 values) in registers
-// for the sequence's whole run of tokens, the per-token vectors shared by the head (k, r, w, ...)
-// are broadcast through double-buffered shared memory (one barrier per token, next token's loads
-// issued before the current token's math), and the state touches HBM once on the way in and once
-// on the way out.  Sequences are independent, so the grid is (heads, batch slots).
+// S x S state through global memory on each token.  Here a CTA owns a share of the columns of one (sequence, head) pair and
+// keeps them in registers for the sequence's whole run of tokens; the per-token vectors shared by the head (k, r, w, ...)
+// reach shared memory a chunk ahead, and the state touches HBM once on the way in and once on the way out.  Sequences,
+// heads and columns are independent, so the grid is (heads x shares of the columns, batch slots).
 //
 // State layout (reference: src/runtime/v6.rs:187-197): f32 view [C, S+1, B]; row 0 = token-shift
 // carry, row 1+i = key index i for all heads side by side (column h*S + j = value index j).
