@@ -301,6 +301,11 @@ int32_t wrk_matrix_matmul_op_sparse(wrk_matrix* m, const wrk_view* input, const 
  * sums over K (a single op may split K over CTAs where the group does not). */
 int32_t wrk_matrix_matmul_group_op(wrk_matrix* const* matrices, const wrk_view* inputs, const wrk_view* outputs, const int32_t* acts,
                                    uint32_t count, int32_t turbo, wrk_op** out);
+/* No counterpart in the reference: how a tensor-core launch of these sizes is laid out (no device is touched).  kind as in
+ * wrk_matrix_parts; row_tiles: tiles of 128 rows of all its matrices.  plan: tokens per CTA, CTAs along K, most units of K of a
+ * CTA (pairs of 64-column steps; fp16: stages), steps per activation stage, accumulator and all tensor-memory columns, stages of
+ * dequantized weights, activations and packed weights, dynamic shared memory in bytes. */
+int32_t wrk_matmul_plan(int32_t kind, uint32_t k, uint32_t n, uint32_t row_tiles, uint32_t num_sms, uint32_t plan[10]);
 /* The default NF4 table of Float4Quant::new, matrix.rs:48-70. */
 int32_t wrk_nf4_table(float table[16]);
 /* Float4Quant::new_student(nu) / quantile_student, matrix.rs:29-44 and 72-77: the SF4 code book.  The Student-t

@@ -88,3 +88,11 @@ def test_a_matmul_waits_for_the_op_that_writes_its_weights(wrk, ctx):
         matrix.load(np.zeros((M, K), dtype=np.float16))
         ctx.encode(ops, use_graph=graph).submit()
         assert_close(y.numpy().reshape(N, M), x.astype(np.float32) @ w.astype(np.float32).T, f"graph={graph}")
+
+
+@pytest.mark.parametrize("kind,k,n", [("int8", 768, 65), ("int8", 768, 80), ("nf4", 896, 96), ("nf4", 768, 112)])
+def test_more_pairs_than_raw_stages(wrk, ctx, kind, k, n):
+    # six or seven pairs of steps through a ring that shared memory cuts to fewer stages
+    got, want = _run(wrk, ctx, kind, k, 500, n, turbo=True, seed=k + n)
+    assert_close(got, want, f"{kind} {k} n={n}")
+    assert ctx.device_status() == 0

@@ -532,6 +532,13 @@ class Matrix:
         return _mk(fn, self.handle, pi, po, act, int(turbo), keep=(self, ki, ko))
 
 
+def matmul_plan(kind, k, n, row_tiles, num_sms=148):
+    """`wrk_matmul_plan`: the layout of a tensor-core launch of these sizes, as a dict."""
+    plan = (ctypes.c_uint32 * 10)()
+    check(lib().wrk_matmul_plan(*(ctypes.c_uint32(v) for v in (kind, k, n, row_tiles, num_sms)), plan))
+    return dict(zip(("n_tile", "splits", "walk", "bu", "acc_cols", "tmem_cols", "a_stages", "b_stages", "raw", "smem"), plan))
+
+
 def matmul_group_op(matrices, inputs, outputs, acts=None, turbo=True):
     """Up to four `Matrix.matmul_op` of one point of a layer as one op (one tensor-core launch where the shapes allow)."""
     n = len(matrices)

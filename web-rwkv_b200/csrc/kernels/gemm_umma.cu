@@ -696,6 +696,71 @@ bool matmul_umma_group_supported(const MatmulArgs* a, int count) {
     return true;
 }
 
+// Output tiles are 128 rows x n_tile tokens; K is split across the CTAs of a thread-block cluster while the
+// tiles alone leave SMs idle: a split keeps at least eight steps, a cluster at most 8 CTAs.  Up to 512 tokens,
+// 128-token tiles replace 256-token ones when that doubles the CTAs of the single wave without lengthening a CTA's
+// K walk: smaller operand stages (a deeper ring) and smaller partial tiles.  (Measured: 2048x2048 Int8, 256 tokens:
+// 22.8 -> 15.9 us; where the K walk would double instead, 31 -> 37 us, so those keep 256.)
+UmmaPlan umma_plan(int kind, uint32_t K, uint32_t N, uint32_t row_tiles, uint32_t num_sms) {
+    UmmaPlan p{};
+    const bool quantized = kind != MAT_FP16;
+    const uint32_t nk = K / BK;
+    auto splits_for = [&](uint32_t n_tile) {
+        const uint32_t tiles = row_tiles * ((N + n_tile - 1) / n_tile);
+        uint32_t want = std::max<uint32_t>(1, num_sms / tiles);
+        want = std::min<uint32_t>(want, std::max<uint32_t>(1, nk / 8));
+        want = std::min<uint32_t>(want, 8);
+        while (nk % 4 == 0 && nk % (4 * want) != 0) --want;  // equal shares where K allows them
+        return want;
+    };
+    p.n_tile = std::min<uint32_t>(256, (N + 15) / 16 * 16);
+    p.splits = splits_for(p.n_tile);
+    if (p.n_tile > 128 && N <= 512) {
+        const uint32_t s2 = splits_for(128);
+        if (s2 >= p.splits && row_tiles * ((N + 127) / 128) * s2 <= num_sms) p.n_tile = 128, p.splits = s2;
+    }
+    // a copy of activations brings two steps unless a step's tile is large already; fewer, larger copies: issuing one costs
+    // its thread about 0.2 us, as much as the MMAs of a step of 64 tokens take
+    p.bu = p.n_tile <= 128 ? 2 : 1;
+    // tensor memory: the accumulator and (quantized weights) A stages of a pair of steps
+    p.acc_cols = (p.n_tile + 31) / 32 * 32;
+    uint32_t cols = p.acc_cols;
+    if (quantized) {
+        cols = p.acc_cols <= 64 ? 256 : 512;
+        p.a_stages = std::min<uint32_t>(kMaxStages, (cols - p.acc_cols) / (2 * A_STEP_COLS));
+    }
+    for (p.tmem_cols = 32; p.tmem_cols < cols;) p.tmem_cols *= 2;
+    const uint32_t unit = quantized ? 2 : p.bu;
+    p.walk = ((nk + unit - 1) / unit + p.splits - 1) / p.splits;
+    const uint32_t b_bytes = p.bu * p.n_tile * BK * 2;
+    const uint32_t raw_bytes = kind == MAT_INT8 ? BM * 128 : kind == MAT_NF4 ? BM * 64 : 0;
+    const uint32_t budget = 222u * 1024;  // of an SM's shared memory: less the static part and the alignment slack
+    size_t smem = 0;
+    if (quantized) {
+        p.b_stages = std::min<uint32_t>(kMaxStages, std::max<uint32_t>(2, p.walk * (2 / p.bu)));
+        p.raw = std::min<uint32_t>(kMaxRaw, std::max<uint32_t>(2, p.walk));
+        auto bytes = [&] { return p.b_stages * b_bytes + p.raw * raw_bytes + SCALE_BYTES; };
+        while (bytes() > budget) {
+            if (p.raw > 4) --p.raw;
+            else if (p.b_stages > 4) --p.b_stages;
+            else if (p.raw > 2) --p.raw;
+            else --p.b_stages;
+        }
+        // The dequantizing groups take alternate pairs.  With an even ring a raw stage always belongs to one group, whose
+        // waits see its phases in order.  With an odd one it changes hands with every use, and a group may only test it for
+        // pair u when pair u - raw has arrived (a barrier two phases behind looks complete): its last pair, u - 2, waited
+        // for the MMAs of pair u - 2 - a_stages, which tells it so only if raw >= a_stages + 2.
+        if (p.raw < p.walk && p.raw % 2 == 1 && p.raw < p.a_stages + 2) --p.raw;
+        smem = bytes();
+    } else {
+        const uint32_t stage = b_bytes + p.bu * A_STEP_BYTES;
+        p.b_stages = std::min<uint32_t>(std::min<uint32_t>(kMaxStages, budget / stage), std::max<uint32_t>(2, p.walk));
+        smem = p.b_stages * stage;
+    }
+    p.smem = (uint32_t)std::max<size_t>(smem, (size_t)p.n_tile * BM * sizeof(float)) + 1024;  // at the end the f32 tile lies there
+    return p;
+}
+
 cudaError_t matmul_umma_group(const MatmulArgs* args, int count, int32_t* status, cudaStream_t stream) {
     if (!matmul_umma_group_supported(args, count)) return cudaErrorInvalidValue;
     const MatmulArgs& a = args[0];
@@ -710,66 +775,17 @@ cudaError_t matmul_umma_group(const MatmulArgs* args, int count, int32_t* status
     g.K = a.K;
     g.N = a.N;
     g.status = status;
-    const bool quantized = a.kind != MAT_FP16;
-    const uint32_t nk = a.K / BK;
-    // Output tiles are 128 rows x n_tile tokens; K is split across the CTAs of a thread-block cluster while the
-    // tiles alone leave SMs idle: a split keeps at least eight steps, a cluster at most 8 CTAs.  Up to 512 tokens,
-    // 128-token tiles replace 256-token ones when that doubles the CTAs of the single wave without lengthening a CTA's
-    // K walk: smaller operand stages (a deeper ring) and smaller partial tiles.  (Measured: 2048x2048 Int8, 256 tokens:
-    // 22.8 -> 15.9 us; where the K walk would double instead, 31 -> 37 us, so those keep 256.)
     int sms = 148, device = 0;
     if (cudaGetDevice(&device) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
-    auto splits_for = [&](uint32_t n_tile) {
-        const uint32_t tiles = row_tiles * ((a.N + n_tile - 1) / n_tile);
-        uint32_t want = std::max<uint32_t>(1, (uint32_t)sms / tiles);
-        want = std::min<uint32_t>(want, std::max<uint32_t>(1, nk / 8));
-        want = std::min<uint32_t>(want, 8);
-        while (nk % 4 == 0 && nk % (4 * want) != 0) --want;  // equal shares where K allows them
-        return want;
-    };
-    g.n_tile = std::min<uint32_t>(256, (a.N + 15) / 16 * 16);
-    g.splits = splits_for(g.n_tile);
-    if (g.n_tile > 128 && a.N <= 512) {
-        const uint32_t s2 = splits_for(128);
-        if (s2 >= g.splits && row_tiles * ((a.N + 127) / 128) * s2 <= (uint32_t)sms) g.n_tile = 128, g.splits = s2;
-    }
-    // a copy of activations brings two steps unless a step's tile is large already; fewer, larger copies: issuing one costs
-    // its thread about 0.2 us, as much as the MMAs of a step of 64 tokens take
-    g.bu = g.n_tile <= 128 ? 2 : 1;
-    // tensor memory: the accumulator and (quantized weights) A stages of a pair of steps
-    g.acc_cols = (g.n_tile + 31) / 32 * 32;
-    g.tmem_cols = g.acc_cols;
-    if (quantized) {
-        g.tmem_cols = g.acc_cols <= 64 ? 256 : 512;
-        g.a_stages = std::min<uint32_t>(kMaxStages, (g.tmem_cols - g.acc_cols) / (2 * A_STEP_COLS));
-    }
-    for (uint32_t c = 32;; c *= 2)
-        if (c >= g.tmem_cols) {
-            g.tmem_cols = c;
-            break;
-        }
-    const uint32_t unit = quantized ? 2 : g.bu, walk = ((nk + unit - 1) / unit + g.splits - 1) / g.splits;  // most units of a CTA
-    const uint32_t b_bytes = g.bu * g.n_tile * BK * 2;
-    const uint32_t raw_bytes = a.kind == MAT_INT8 ? BM * 128 : a.kind == MAT_NF4 ? BM * 64 : 0;
-    const uint32_t budget = 222u * 1024;  // of an SM's shared memory: less the static part and the alignment slack
-    size_t smem = 0;
-    if (quantized) {
-        g.b_stages = std::min<uint32_t>(kMaxStages, std::max<uint32_t>(2, walk * (2 / g.bu)));
-        g.raw = std::min<uint32_t>(kMaxRaw, std::max<uint32_t>(2, walk));
-        auto bytes = [&] { return g.b_stages * b_bytes + g.raw * raw_bytes + SCALE_BYTES; };
-        while (bytes() > budget) {
-            if (g.raw > 4) --g.raw;
-            else if (g.b_stages > 4) --g.b_stages;
-            else if (g.raw > 2) --g.raw;
-            else --g.b_stages;
-        }
-        smem = bytes();
-    } else {
-        const uint32_t stage = b_bytes + g.bu * A_STEP_BYTES;
-        g.b_stages = std::min<uint32_t>(std::min<uint32_t>(kMaxStages, budget / stage), std::max<uint32_t>(2, walk));
-        smem = g.b_stages * stage;
-    }
-    smem = std::max<size_t>(smem, (size_t)g.n_tile * BM * sizeof(float)) + 1024;  // at the end the f32 tile lies there
+    const UmmaPlan plan = umma_plan(a.kind, a.K, a.N, row_tiles, (uint32_t)sms);
+    g.n_tile = plan.n_tile;
+    g.acc_cols = plan.acc_cols;
+    g.tmem_cols = plan.tmem_cols;
+    g.bu = plan.bu;
+    g.a_stages = plan.a_stages;
+    g.b_stages = plan.b_stages;
+    g.raw = plan.raw;
+    g.splits = plan.splits;
 
     for (int i = 0; i < count; ++i) {
         const MatmulArgs& ai = args[i];
@@ -798,7 +814,7 @@ cudaError_t matmul_umma_group(const MatmulArgs* args, int count, int32_t* status
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = grid;
     cfg.blockDim = dim3(kUmmaThreads, 1, 1);
-    cfg.dynamicSmemBytes = smem;
+    cfg.dynamicSmemBytes = plan.smem;
     cfg.stream = stream;
     cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeClusterDimension;

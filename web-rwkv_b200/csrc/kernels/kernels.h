@@ -64,6 +64,17 @@ cudaError_t matmul_umma(const MatmulArgs& a, int32_t* status, cudaStream_t strea
 // Up to four matrices of one weight format, K and token count (each with its own activations, output and activation
 // function) as the row tiles of one launch.
 bool matmul_umma_group_supported(const MatmulArgs* a, int count);
+// The tiles, rings and memory of such a launch over `row_tiles` tiles of 128 rows.
+struct UmmaPlan {
+    uint32_t n_tile;     // tokens per CTA
+    uint32_t splits;     // CTAs along K per output tile
+    uint32_t walk;       // most units (pairs of steps, or stages of fp16 weights) that a CTA takes
+    uint32_t bu;         // steps per stage of activations
+    uint32_t acc_cols, tmem_cols;
+    uint32_t a_stages, b_stages, raw;
+    uint32_t smem;       // dynamic shared memory, bytes
+};
+UmmaPlan umma_plan(int kind, uint32_t K, uint32_t N, uint32_t row_tiles, uint32_t num_sms);
 cudaError_t matmul_umma_group(const MatmulArgs* a, int count, int32_t* status, cudaStream_t stream);
 
 // ---- one-shot all-reduce over peer memory (peer_reduce.cu) --------------------------------------------

@@ -1186,6 +1186,16 @@ int32_t wrk_matrix_matmul_op_sparse(wrk_matrix* m, const wrk_view* input, const 
     return matrix_matmul(m, input, output, act, turbo, 1, out);
 }
 
+int32_t wrk_matmul_plan(int32_t kind, uint32_t k, uint32_t n, uint32_t row_tiles, uint32_t num_sms, uint32_t plan[10]) {
+    REQ_NN(plan);
+    WRK_REQUIRE(kind >= 0 && kind <= 2 && k >= 128 && k % 128 == 0 && n > 0 && row_tiles > 0 && num_sms > 0, WRK_ERR_INVALID_ARGUMENT,
+                "no such matmul: kind %d, k = %u, n = %u, %u row tiles, %u SMs", kind, k, n, row_tiles, num_sms);
+    const k::UmmaPlan p = k::umma_plan(kind == 0 ? k::MAT_FP16 : kind == 1 ? k::MAT_INT8 : k::MAT_NF4, k, n, row_tiles, num_sms);
+    const uint32_t values[10] = {p.n_tile, p.splits, p.walk, p.bu, p.acc_cols, p.tmem_cols, p.a_stages, p.b_stages, p.raw, p.smem};
+    std::copy(values, values + 10, plan);
+    return WRK_OK;
+}
+
 int32_t wrk_matrix_matmul_group_op(wrk_matrix* const* matrices, const wrk_view* inputs, const wrk_view* outputs, const int32_t* acts,
                                    uint32_t count, int32_t turbo, wrk_op** out) {
     REQ_NN(matrices, inputs, outputs, acts, out);
