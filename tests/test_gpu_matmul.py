@@ -307,3 +307,37 @@ def test_few_tokens_of_a_long_k(wrk, ctx, kind, n):
     ctx.run(mat.matmul_op(ctx.from_numpy(x), y))
     oracle.matmul(okind, om, oscale, x, want)
     assert_close(y.numpy().reshape(n, M), want, f"{kind} n={n}")
+
+
+def _float64(mat, w, x):
+    """W x in float64 with the weights that the matrix holds."""
+    kind, q, scale, _ = mat.parts()
+    M, K = w.shape
+    if kind == 1:
+        mm = scale.numpy().reshape(M, K // 128, 1, 2).astype(np.float64)
+        q = q.numpy().reshape(M, K // 128, 128).astype(np.float64)
+        w = (q * ((mm[..., 1] - mm[..., 0]) / 255.0) + mm[..., 0]).reshape(M, K)
+    return x.astype(np.float64) @ w.astype(np.float64).T
+
+
+def _relative_error(got, want):
+    return float(np.linalg.norm(got.astype(np.float64) - want) / np.linalg.norm(want))
+
+
+@pytest.mark.parametrize("kind", ["int8", "fp16"])
+@pytest.mark.parametrize("k,n", [(768, 9), (1024, 12), (4096, 15), (384, 16), (2688, 33), (8064, 256)])
+def test_few_tokens_and_odd_blocks_keep_the_bytes_exact(wrk, ctx, kind, k, n):
+    """9 to 15 tokens, and Int8 rows of an odd number of blocks, against float64.  Exact bytes and f32 sums leave about
+    sqrt(K) 2^-24 (5e-6 at K = 8064); a weight rounded to fp16 has an error of up to 2^-11, which leaves 2e-4."""
+    if kind == "fp16" and n > 15:
+        pytest.skip("fp16 rows have no blocks")
+    rng = np.random.default_rng(k + n)
+    w = (rng.standard_normal((256, k), dtype=np.float32) * 0.02).astype(np.float16)
+    x = rng.standard_normal((n, k), dtype=np.float32).astype(np.float16)
+    mat, _ = _make_matrix(wrk, ctx, kind, w)
+    for turbo in (False, True):
+        y = ctx.tensor(wrk.F32, [256, n])
+        ctx.run(mat.matmul_op(ctx.from_numpy(x), y, turbo=turbo))
+        err = _relative_error(y.numpy().reshape(n, 256), _float64(mat, w, x))
+        # fp16: the tensor cores' own sums; the mma.sync kernel's are within 4e-7 at 1024 columns, tcgen05's are not
+        assert err <= (1e-5 if kind == "int8" else 4e-7 * max(1.0, k / 1024)), f"{kind} {k} n={n} turbo={turbo}: {err:.3g}"
