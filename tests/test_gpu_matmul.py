@@ -341,3 +341,16 @@ def test_few_tokens_and_odd_blocks_keep_the_bytes_exact(wrk, ctx, kind, k, n):
         err = _relative_error(y.numpy().reshape(n, 256), _float64(mat, w, x))
         # fp16: the tensor cores' own sums; the mma.sync kernel's are within 4e-7 at 1024 columns, tcgen05's are not
         assert err <= (1e-5 if kind == "int8" else 4e-7 * max(1.0, k / 1024)), f"{kind} {k} n={n} turbo={turbo}: {err:.3g}"
+
+
+def test_int8_rows_too_long_for_one_streaming_launch_keep_their_sums(wrk, ctx):
+    # 8 tokens of 14336 columns, whose activations one weight-streaming launch does not hold: exact bytes, a block's sum scaled by
+    # itself; sums whose terms carry the bytes' offset of 1024 would lose 2e-6
+    rng = np.random.default_rng(21)
+    w = (rng.standard_normal((256, 14336), dtype=np.float32) * 0.02).astype(np.float16)
+    x = rng.standard_normal((8, 14336), dtype=np.float32).astype(np.float16)
+    mat, _ = _make_matrix(wrk, ctx, "int8", w)
+    y = ctx.tensor(wrk.F32, [256, 8])
+    ctx.run(mat.matmul_op(ctx.from_numpy(x), y))
+    err = _relative_error(y.numpy().reshape(8, 256), _float64(mat, w, x))
+    assert err <= 6e-7, err

@@ -160,11 +160,12 @@ int32_t matmul_common(const char* name, int kind, wrk_tensor* matrix, wrk_tensor
     k::MatmulArgs a;
     WRK_TRY(matmul_args(kind, matrix, scale, quant, input, output, act, &a));
     if (streams(a)) {
-        // A long K: as few launches as hold the tokens, of about the same number each (8 tokens of a 14336 -> 4096 Int8 matrix:
-        // two launches of 4; the mma.sync kernel below, which stages a part of K at a time, took 92 us).  Not where the
-        // outputs might overwrite activations that a later launch reads.
+        // A long K: as few launches as hold the tokens, of about the same number each (8 tokens of a 14336 -> 4096 fp16 matrix:
+        // two launches of 4).  Not where the outputs might overwrite activations that a later launch reads, and not Int8: the
+        // mma.sync kernel below, which stages a part of K at a time and scales every block's own sum, has a relative error of
+        // 2.8e-7 there, the weight-streaming kernel 2.0e-6 (fp16: 2.2e-6 and 1.3e-7; NF4 the same).
         const uint32_t most = stream_tokens(a.N, a.K), parts = most ? (a.N + most - 1) / most : 0;
-        if (parts == 1 || (parts > 1 && input->tensor->buf != output->tensor->buf)) {
+        if (parts == 1 || (parts > 1 && kind != k::MAT_INT8 && input->tensor->buf != output->tensor->buf)) {
             std::vector<wrk_op*> ops;
             int32_t status = WRK_OK;
             for (uint32_t i = 0; i < parts && status == WRK_OK; ++i) {
