@@ -295,10 +295,9 @@ int32_t wrk_matrix_matmul_op_sparse(wrk_matrix* m, const wrk_view* input, const 
                                     int32_t turbo, wrk_op** out);
 /* No counterpart in the reference: up to four Matrix::matmul_op of one point of a layer (e.g. key / value / receptance /
  * gate, each with its own input, output and activation) as one op.  Matrices of one format, input width and token count
- * with 16 or more tokens and `turbo` run as the row tiles of a single tensor-core launch, which fills the SMs without
- * splitting K; matmuls of the same 1 to 8 tokens, of any formats and widths, share a weight-streaming launch unless one
- * reads what another writes; anything else becomes the list of the single ops.  Results are those of the single ops up to the order of the fp32
- * sums over K (a single op may split K over CTAs where the group does not). */
+ * with 16 or more tokens and `turbo` run as the row tiles of a single tensor-core launch; matmuls of the same 1 to 8 tokens, of any formats and widths, share a weight-streaming launch unless one
+ * reads what another writes; anything else becomes the list of the single ops.  Results are those of the single ops; the
+ * tensor-core launch of a multiple of 32 tokens may sum over K in another order (it splits K less than a single op would). */
 int32_t wrk_matrix_matmul_group_op(wrk_matrix* const* matrices, const wrk_view* inputs, const wrk_view* outputs, const int32_t* acts,
                                    uint32_t count, int32_t turbo, wrk_op** out);
 /* No counterpart in the reference: how a tensor-core launch of these sizes is laid out (no device is touched).  kind as in

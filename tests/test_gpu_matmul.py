@@ -354,3 +354,23 @@ def test_int8_rows_too_long_for_one_streaming_launch_keep_their_sums(wrk, ctx):
     ctx.run(mat.matmul_op(ctx.from_numpy(x), y))
     err = _relative_error(y.numpy().reshape(8, 256), _float64(mat, w, x))
     assert err <= 6e-7, err
+
+
+@pytest.mark.parametrize("kind", KINDS)
+@pytest.mark.parametrize("heights,n,launches", [([2048] * 4, 16, 1), ([512, 300, 512], 24, 1), ([6400, 256], 40, 2), ([256, 256], 100, 1)])
+def test_group_keeps_the_sums_of_the_single_ops(wrk, ctx, kind, heights, n, launches):
+    """Token counts that are no multiple of 32: the launch splits K as each matmul alone would (2048 rows of 2048 columns:
+    over four CTAs), so the bits agree; matrices that would be split differently (6400 rows: two) are launched one by one."""
+    rng = np.random.default_rng(300 + n)
+    mats, xs, ys, singles = [], [], [], []
+    for M in heights:
+        mats.append(_make_matrix(wrk, ctx, kind, (rng.standard_normal((M, 2048), dtype=np.float32) * 0.02).astype(np.float16))[0])
+        xs.append(ctx.from_numpy(rng.standard_normal((n, 2048), dtype=np.float32).astype(np.float16)))
+        ys.append(ctx.tensor(wrk.F32, [M, n]))
+        singles.append(ctx.tensor(wrk.F32, [M, n]))
+    before = ctx.launch_count()
+    ctx.run(wrk.matmul_group_op(mats, xs, ys, turbo=True))
+    assert ctx.launch_count() - before == launches
+    for mat, x, y, single in zip(mats, xs, ys, singles):
+        ctx.run(mat.matmul_op(x, single, turbo=True))
+        assert np.array_equal(y.numpy(), single.numpy())

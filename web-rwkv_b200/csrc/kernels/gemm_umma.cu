@@ -691,15 +691,6 @@ bool matmul_umma_supported(const MatmulArgs& a) {
     return encode_tiled() != nullptr;
 }
 
-bool matmul_umma_group_supported(const MatmulArgs* a, int count) {
-    if (count < 1 || count > kMaxGroup) return false;
-    for (int i = 0; i < count; ++i) {
-        if (!matmul_umma_supported(a[i])) return false;
-        if (a[i].kind != a[0].kind || a[i].K != a[0].K || a[i].N != a[0].N) return false;
-    }
-    return true;
-}
-
 // Output tiles are 128 rows x n_tile tokens; K is split across the CTAs of a thread-block cluster while the
 // tiles alone leave SMs idle: a split keeps at least eight steps, a cluster at most 8 CTAs.  Up to 512 tokens,
 // 128-token tiles replace 256-token ones when that doubles the CTAs of the single wave without lengthening a CTA's
@@ -765,8 +756,41 @@ UmmaPlan umma_plan(int kind, uint32_t K, uint32_t N, uint32_t row_tiles, uint32_
     return p;
 }
 
+// The layout of a group's launch; false when its members do not go together.  Whole chunks of 32 tokens are split along K as far
+// as the group's tiles leave SMs idle.  Other counts keep the sums of the single ops, bit for bit: each member's own tile and
+// split have to agree, and the launch takes them.  (A group of its own splits K less, and longer sums lose more: four 2048 x 2048
+// fp16 matrices at 16 tokens 1.25e-6 from float64 against 6.5e-7.)
+static bool group_plan(const MatmulArgs* a, int count, uint32_t num_sms, UmmaPlan* plan) {
+    if (count < 1 || count > kMaxGroup) return false;
+    uint32_t row_tiles = 0;
+    for (int i = 0; i < count; ++i) {
+        if (!matmul_umma_supported(a[i])) return false;
+        if (a[i].kind != a[0].kind || a[i].K != a[0].K || a[i].N != a[0].N) return false;
+        row_tiles += (a[i].M + BM - 1) / BM;
+    }
+    if (a[0].N % 32 == 0) {
+        *plan = umma_plan(a[0].kind, a[0].K, a[0].N, row_tiles, num_sms);
+        return true;
+    }
+    for (int i = 0; i < count; ++i) {
+        if (count > 1 && matmul_small_supported(a[i])) return false;  // alone it takes another kernel
+        const UmmaPlan own = umma_plan(a[i].kind, a[i].K, a[i].N, (a[i].M + BM - 1) / BM, num_sms);
+        if (i == 0) *plan = own;
+        else if (own.n_tile != plan->n_tile || own.splits != plan->splits) return false;
+    }
+    return true;
+}
+
+bool matmul_umma_group_supported(const MatmulArgs* a, int count, int num_sms) {
+    UmmaPlan plan;
+    return group_plan(a, count, (uint32_t)num_sms, &plan);
+}
+
 cudaError_t matmul_umma_group(const MatmulArgs* args, int count, int32_t* status, cudaStream_t stream) {
-    if (!matmul_umma_group_supported(args, count)) return cudaErrorInvalidValue;
+    int sms = 148, device = 0;
+    if (cudaGetDevice(&device) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+    UmmaPlan plan;
+    if (!group_plan(args, count, (uint32_t)sms, &plan)) return cudaErrorInvalidValue;
     const MatmulArgs& a = args[0];
     UmmaGroup g{};
     g.count = (uint32_t)count;
@@ -779,9 +803,6 @@ cudaError_t matmul_umma_group(const MatmulArgs* args, int count, int32_t* status
     g.K = a.K;
     g.N = a.N;
     g.status = status;
-    int sms = 148, device = 0;
-    if (cudaGetDevice(&device) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
-    const UmmaPlan plan = umma_plan(a.kind, a.K, a.N, row_tiles, (uint32_t)sms);
     g.n_tile = plan.n_tile;
     g.acc_cols = plan.acc_cols;
     g.tmem_cols = plan.tmem_cols;

@@ -63,7 +63,7 @@ bool matmul_umma_supported(const MatmulArgs& a);
 cudaError_t matmul_umma(const MatmulArgs& a, int32_t* status, cudaStream_t stream);
 // Up to four matrices of one weight format, K and token count (each with its own activations, output and activation
 // function) as the row tiles of one launch.
-bool matmul_umma_group_supported(const MatmulArgs* a, int count);
+bool matmul_umma_group_supported(const MatmulArgs* a, int count, int num_sms);
 // The tiles, rings and memory of such a launch over `row_tiles` tiles of 128 rows.
 struct UmmaPlan {
     uint32_t n_tile;     // tokens per CTA

@@ -1217,7 +1217,7 @@ int32_t wrk_matrix_matmul_group_op(wrk_matrix* const* matrices, const wrk_view* 
         weights.insert(weights.end(), {m->w, m->m, m->q});
         tensors.insert(tensors.end(), {inputs[i].tensor, outputs[i].tensor});
     }
-    gemm = gemm && k::matmul_umma_group_supported(args, (int)count);
+    gemm = gemm && k::matmul_umma_group_supported(args, (int)count, matrices[0]->w->ctx->num_sms);
     if (gemm) {
         std::vector<k::MatmulArgs> all(args, args + count);
         int32_t* status = args[0].status;

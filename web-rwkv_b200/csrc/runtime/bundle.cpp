@@ -255,12 +255,12 @@ struct GroupItem {
     wrk_view in, out;
     int32_t act;
 };
-// A group with `turbo` asks for the tensor-core kernel, one of up to 8 tokens without it gets a weight-streaming launch.
-// v5 and v7 ask for it from 16 tokens on (9 to 15: a launch per matrix; the tests count the launches of such a job), v6 for
-// whole chunks of 32 only: a group splits K less than its matrices would alone, and the order of the sums shows in the
-// states of a deep v6 model.  Measured: 16 tokens of a 2048-wide fp16 v5 model of twelve layers, 97 GEMM launches of
-// 6.3 us -> 49 of 9.0 us; one token of eight 4096-wide Int8 v7 layers, 111 streaming launches of 7.5 us -> 49 of 13.1 us;
-// 64 tokens of those, the adapters' first matrices 325 us as 31 launches -> 155 us as 8.
+// A group with `turbo` asks for the tensor-core kernel, which takes 16 tokens and more; one of up to 8 tokens without it gets a
+// weight-streaming launch.  v5 and v7 ask for it at every count it takes, v6 for whole chunks of 32 (the others were not
+// measured); at counts that are no multiple of 32 the launch has the sums of the single ops.  Measured: a step of 16
+// sequences of a 2048-wide fp16 v5 model of twelve layers 1417 us in single launches, 1343 in groups; one token of eight
+// 4096-wide Int8 v7 layers, 111 streaming launches of 7.5 us -> 49 of 13.1 us; 64 tokens of those, the adapters' first
+// matrices 325 us as 31 launches -> 155 us as 8.
 int32_t matmul_group(OpList& ops, std::initializer_list<GroupItem> items, bool turbo) {
     wrk_matrix* ms[4];
     wrk_view ins[4], outs[4];
