@@ -295,8 +295,9 @@ int32_t wrk_matrix_matmul_op_sparse(wrk_matrix* m, const wrk_view* input, const 
                                     int32_t turbo, wrk_op** out);
 /* No counterpart in the reference: up to four Matrix::matmul_op of one point of a layer (e.g. key / value / receptance /
  * gate, each with its own input, output and activation) as one op.  Matrices of one format, input width and token count
- * with 16 or more tokens and `turbo` run as the row tiles of a single tensor-core launch; matmuls of the same 1 to 8 tokens, of any formats and widths, share a weight-streaming launch unless one
- * reads what another writes; anything else becomes the list of the single ops.  Results are those of the single ops; the
+ * with 16 or more tokens and `turbo` run as the row tiles of a single tensor-core launch; matmuls of the same 1 to 8
+ * tokens, of any formats and widths, share a weight-streaming launch.  Where one reads or writes what another writes, and
+ * for anything else, the op becomes the list of the single ops, in order.  Results are those of the single ops; the
  * tensor-core launch of a multiple of 32 tokens may sum over K in another order (it splits K less than a single op would). */
 int32_t wrk_matrix_matmul_group_op(wrk_matrix* const* matrices, const wrk_view* inputs, const wrk_view* outputs, const int32_t* acts,
                                    uint32_t count, int32_t turbo, wrk_op** out);

@@ -148,6 +148,16 @@ int32_t stream_op(const char* name, wrk_context* ctx, const k::MatmulArgs* args,
     return WRK_OK;
 }
 
+// Whether two views may share an element: boxes of one tensor are compared axis by axis, other views of one buffer count as sharing.
+bool overlap(const wrk_view& a, const wrk_view& b) {
+    if (a.tensor->buf != b.tensor->buf) return false;
+    for (int i = 0; i < 4; ++i)
+        if (a.stride[i] != b.stride[i]) return true;
+    for (int i = 0; i < 4; ++i)
+        if (a.offset[i] + a.shape[i] <= b.offset[i] || b.offset[i] + b.shape[i] <= a.offset[i]) return false;
+    return true;
+}
+
 // Tokens of one weight-streaming launch over `k` columns: its shared memory holds all their activations.
 uint32_t stream_tokens(uint32_t n, uint32_t k) {
     while (n > 0 && k::fused_gemv_smem(n, k, k, k::PRO_NONE, 2) > 200 * 1024) --n;
@@ -1202,7 +1212,8 @@ int32_t wrk_matrix_matmul_group_op(wrk_matrix* const* matrices, const wrk_view* 
     REQ_NN(matrices, inputs, outputs, acts, out);
     WRK_REQUIRE(count >= 1 && count <= 4, WRK_ERR_INVALID_ARGUMENT, "a group holds 1 to 4 matrices, not %u", count);
     k::MatmulArgs args[4];
-    bool gemm = turbo != 0, stream = true;
+    // The members of one launch run at the same time: none may read, as input or as weights, or write what another writes.
+    bool independent = true, stream = true;
     uint32_t kmax = 0;
     std::vector<wrk_tensor*> weights, tensors;
     for (uint32_t i = 0; i < count; ++i) {
@@ -1212,12 +1223,17 @@ int32_t wrk_matrix_matmul_group_op(wrk_matrix* const* matrices, const wrk_view* 
         WRK_TRY(matmul_args(kind, m->w, m->m, m->q, &inputs[i], &outputs[i], acts[i], &args[i]));
         kmax = std::max(kmax, args[i].K);
         stream = stream && streams(args[i]) && args[i].N == args[0].N;
-        for (uint32_t j = 0; j < i; ++j)
-            stream = stream && inputs[i].tensor->buf != outputs[j].tensor->buf && inputs[j].tensor->buf != outputs[i].tensor->buf;
         weights.insert(weights.end(), {m->w, m->m, m->q});
         tensors.insert(tensors.end(), {inputs[i].tensor, outputs[i].tensor});
     }
-    gemm = gemm && k::matmul_umma_group_supported(args, (int)count, matrices[0]->w->ctx->num_sms);
+    for (uint32_t i = 0; i < count; ++i)
+        for (uint32_t j = 0; j < count; ++j) {
+            if (i == j) continue;
+            independent = independent && !overlap(inputs[i], outputs[j]) && !overlap(outputs[i], outputs[j]);
+            for (const wrk_tensor* w : {matrices[i]->w, matrices[i]->m, matrices[i]->q})
+                independent = independent && (w == nullptr || w->buf != outputs[j].tensor->buf);
+        }
+    const bool gemm = independent && turbo != 0 && k::matmul_umma_group_supported(args, (int)count, matrices[0]->w->ctx->num_sms);
     if (gemm) {
         std::vector<k::MatmulArgs> all(args, args + count);
         int32_t* status = args[0].status;
@@ -1231,11 +1247,11 @@ int32_t wrk_matrix_matmul_group_op(wrk_matrix* const* matrices, const wrk_view* 
         *out = op;
         return WRK_OK;
     }
-    if (stream && stream_tokens(args[0].N, kmax) == args[0].N) {
+    if (independent && stream && stream_tokens(args[0].N, kmax) == args[0].N) {
         WRK_TRY(stream_op("matmul_group", matrices[0]->w->ctx, args, count, 0, args[0].N, weights, tensors, out));
         if (*out != nullptr) return WRK_OK;
     }
-    // shapes the grouped kernel does not take: the same work as a list of single matmuls
+    // what no single launch takes: the same work as a list of single matmuls, in order
     std::vector<wrk_op*> ops;
     int32_t status = WRK_OK;
     for (uint32_t i = 0; i < count && status == WRK_OK; ++i) {
