@@ -42,3 +42,10 @@ def test_stages_fit_the_memories(wrk):
         rings += p["raw"] * 128 * (128 if kind == INT8 else 64) + 8192 if quantized else p["b_stages"] * p["bu"] * 16384
         assert max(rings, p["n_tile"] * 512) + 1024 <= p["smem"] <= 223 * 1024, (case, p)
         assert 1 <= p["splits"] <= 8 and p["splits"] * p["walk"] * (2 if quantized else p["bu"]) * 64 >= k, (case, p)
+
+
+def test_ctas_that_wait_for_each_other_do_not_share_an_sm(wrk):
+    # Split K: a CTA holds its tensor memory until its cluster has met.  Two launches on one SM could then each hold what the
+    # other waits for on the next, unless the SM's shared memory (228 KB, 1 KB of it the system's for each CTA) has room for one.
+    for case, p in _plans(wrk, (FP16, INT8, NF4)):
+        assert p["splits"] == 1 or 2 * (p["smem"] + 1024) > 228 * 1024, (case, p)

@@ -52,6 +52,7 @@ constexpr int kMaxRaw = 8;          // raw weight stages
 constexpr uint32_t kScaleSlots = 8, kScaleAhead = 6;
 constexpr uint32_t SCALE_BYTES = 2 * kScaleSlots * BM * 4;  // two groups of dequantizing warps
 constexpr uint32_t kSpinLimit = 1u << 22;
+constexpr uint32_t kSplitSmem = 114 * 1024;  // half of the 228 KB of an SM; 1 KB more per CTA is the system's
 constexpr uint32_t A_STEP_BYTES = BM * BK * 2;  // fp16 weights: 16 KB of shared memory per step
 constexpr uint32_t A_STEP_COLS = BK / 2;        // quantized weights: 32 TMEM columns of fp16 pairs per step
 
@@ -753,6 +754,10 @@ UmmaPlan umma_plan(int kind, uint32_t K, uint32_t N, uint32_t row_tiles, uint32_
         smem = p.b_stages * stage;
     }
     p.smem = (uint32_t)std::max<size_t>(smem, (size_t)p.n_tile * BM * sizeof(float)) + 1024;  // at the end the f32 tile lies there
+    // A CTA of a cluster keeps its tensor memory until its peers have met it, and an allocation waits without limit.  Were CTAs of
+    // two such launches (of two streams) to share an SM, each could wait on one SM for what the other holds on another.
+    // More than half of an SM's shared memory keeps them apart.  (CTAs that are not split free theirs by themselves.)
+    if (p.splits > 1) p.smem = std::max(p.smem, kSplitSmem);
     return p;
 }
 
