@@ -20,7 +20,8 @@
 // through distributed shared memory.
 // Weights enter the MMA as fp16(fma(q, (max - min) / 255, min)) resp. fp16(table[nib] * absmax), computed in
 // f32 and rounded once; the accumulation is fp32.  Every wait on an mbarrier is bounded: on a timeout the
-// kernel records WRK_ERR_TIMEOUT in the context's status word, stops waiting and still frees its TMEM.
+// kernel records WRK_ERR_TIMEOUT in the context's status word, stops waiting and still frees its TMEM.  A wait whose end
+// depends on the activations comes after griddepcontrol.wait: the limit does not count the kernels in front.
 //
 // What bounds it: at 256 tokens a step is 512 cycles of MMA; it takes about 850, most of it shared-memory and L2 traffic of the
 // activation tile (32 KB per step and CTA).  At 64 tokens and below the dequantizers' instructions (about 250 cycles per
@@ -431,6 +432,7 @@ matmul_umma_kernel(const __grid_constant__ UmmaGroup grp) {
             const uint32_t swz = KIND == MAT_INT8 ? (row & 7) : ((row >> 1) & 3);  // the TMA unit's swizzle of this row
 #pragma unroll 1
             for (uint32_t u = group, i = 0; u < nu; u += 2, ++i) {
+                if (u - a_stages < 2) pdl_wait();  // the group's first pair that has to wait for an MMA
                 fetch_scale(i + kScaleAhead);
                 asm volatile("cp.async.wait_group %0;\n" ::"n"(kScaleAhead) : "memory");
                 const uint32_t sc_word = my_scale[(i % kScaleSlots) * BM];
@@ -480,6 +482,7 @@ matmul_umma_kernel(const __grid_constant__ UmmaGroup grp) {
         }
         // ---- the accumulator to shared memory, [token][128 rows] in f32 (the operand stages are free once every MMA has
         // completed): warp w holds lanes 32 (w % 4) .. and takes half of the columns ----
+        pdl_wait();
         mbar_wait(&done_bar, 0, &abort_flag, status);
         tc_fence_after();
         const uint32_t quad = warp & 3, c_begin = (warp >> 2) * (n_tile / 2), c_end = c_begin + n_tile / 2;
@@ -503,6 +506,7 @@ matmul_umma_kernel(const __grid_constant__ UmmaGroup grp) {
         if (elect_one()) {
             const uint32_t idesc = f16_idesc(BM, n_tile);
             Ring ra, rb;
+            pdl_wait();
             bool have_a = quantized && mbar_test(&a_full[0], 0), have_b = mbar_test(&b_full[0], 0);
             uint32_t accumulate = 0;
             // the stage of shared memory that comes next: its `steps` steps, four MMAs of K = 16 each (32 bytes of K per
@@ -550,6 +554,8 @@ matmul_umma_kernel(const __grid_constant__ UmmaGroup grp) {
             ring.skip(ahead, quantized ? n_raw : b_stages);
 #pragma unroll 1
             for (uint32_t u = ahead; u < nu; ++u) {
+                // a stage that is free only after an MMA: the pair before it in the ring has found no A stage unused
+                if (u - ahead == (quantized ? a_stages : 0)) pdl_wait();
                 if (quantized) {
                     mbar_wait(&raw_empty[ring.stage], ring.phase ^ 1, &abort_flag, status);
                     load_raw(u, ring.stage);
