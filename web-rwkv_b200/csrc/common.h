@@ -121,7 +121,10 @@ struct wrk_op {
     wrk::Launch launch;                              // Atom
     uint32_t num_kernels = 1;                        // kernels one launch() issues
     std::vector<std::shared_ptr<wrk::Buffer>> keep;  // buffers the atom touches
-    std::vector<const wrk::Buffer*> early;           // of those: read before the kernels in front of it have finished (weights)
+    // of those, what the kernel reads before the kernels in front of it have finished: whole buffers that it does not write
+    // (weights, constants), and recurrent states whose rows other than the token-shift rows it reads then and writes later
+    std::vector<const wrk::Buffer*> early, early_state;
+    std::vector<const wrk::Buffer*> shift_rows;      // of `keep`: states of which it touches the token-shift rows alone
     std::vector<wrk_op*> children;                   // List (retained)
     ~wrk_op();
 };

@@ -471,17 +471,22 @@ int32_t wrk_op_num_atoms(const wrk_op* op, uint64_t* count) {
 }
 
 // Which atoms of a list may be launched while the one before them still runs.  Every kernel waits for its predecessors
-// before it touches what they wrote, except that a matmul fetches its first weights (`early`) at once: an atom is chained
-// unless an earlier atom of the list touches one of its weights other than as a weight.  The first atom is not: what
-// precedes it on the stream is not known here.
+// before it touches what they wrote, except for what its op declares as read early: a matmul's first weights, a fused phase's
+// constants, the state of a fused recurrence.  An atom is chained unless an earlier atom of the list touches one of these other
+// than to read it early as well (a state: other than its token-shift rows).  The first atom is not: what precedes it on the
+// stream is not known here.
 static std::vector<char> chain_of(const std::vector<wrk_op*>& atoms) {
     std::vector<char> chained(atoms.size(), 0);
     std::unordered_set<const Buffer*> touched;
     for (size_t i = 0; i < atoms.size(); ++i) {
-        const auto& early = atoms[i]->early;
-        chained[i] = i > 0 && std::none_of(early.begin(), early.end(), [&](const Buffer* b) { return touched.count(b) != 0; });
-        for (const auto& b : atoms[i]->keep)
-            if (std::find(early.begin(), early.end(), b.get()) == early.end()) touched.insert(b.get());
+        const wrk_op& a = *atoms[i];
+        auto free = [&](const std::vector<const Buffer*>& early) {
+            return std::none_of(early.begin(), early.end(), [&](const Buffer* b) { return touched.count(b) != 0; });
+        };
+        auto in = [](const std::vector<const Buffer*>& list, const Buffer* b) { return std::find(list.begin(), list.end(), b) != list.end(); };
+        chained[i] = i > 0 && free(a.early) && free(a.early_state);
+        for (const auto& b : a.keep)
+            if (!in(a.early, b.get()) && !in(a.shift_rows, b.get())) touched.insert(b.get());
     }
     return chained;
 }

@@ -326,8 +326,8 @@ __global__ void __launch_bounds__(4 * S) wkv56_fused_kernel(const Wkv6Args a) {
     }
     if (q == 0) su[j] = a.time_first[c];
     const float gw = __half2float(a.gn_w[c]), gb = __half2float(a.gn_b[c]);
-    // ...nor do the WKV state rows: within a job only this kernel writes them, and every job begins with
-    // launches that are not programmatic dependents, i.e. after the previous job has completed
+    // ...nor do the WKV state rows, which the op declares as read early: a list that touches them in front of it does not chain it,
+    // and no list's first launch is a programmatic dependent, i.e. the previous job has completed
     float st[SI];
 #pragma unroll
     for (int i = 0; i < SI; ++i) st[i] = static_cast<const float*>(a.state.base)[a.state.index(c, 1 + q * SI + i, slot)];

@@ -1,8 +1,9 @@
 // Launching the kernels of a job as a chain (programmatic dependent launch).
 //
 // Inside a job every kernel may be launched while the one before it is still running: it then sets itself up (barriers,
-// tensor memory, its first weights, which no kernel of a job writes) and executes griddepcontrol.wait before it touches
-// anything a kernel before it produced or still reads.  A kernel that lets its successor in early (griddepcontrol.
+// tensor memory, and what its op declares as read early: first weights, constants, the state of a fused recurrence, which
+// chain_of checks against the ops in front) and executes griddepcontrol.wait before it touches anything else that a kernel
+// before it produced or still reads.  A kernel that lets its successor in early (griddepcontrol.
 // launch_dependents) must have taken everything the successor could compete for (tensor memory) by then.
 #pragma once
 

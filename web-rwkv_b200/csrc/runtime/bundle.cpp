@@ -837,8 +837,29 @@ int32_t make_partition(wrk_context* ctx, k::FusedGemvArgs& a, int grid, CachedJo
     return WRK_OK;
 }
 
+// What a fused phase reads before it waits for the phases in front of it (its matrices, the constants of its prologue), and the
+// state of which it touches a token-shift row.
+struct EarlyReads {
+    std::vector<const wrk_tensor*> constants;
+    const wrk_tensor* shift_state = nullptr;
+    EarlyReads(std::initializer_list<wrk_matrix*> matrices, std::initializer_list<const wrk_tensor*> others = {}, const wrk_tensor* shift = nullptr)
+        : constants(others), shift_state(shift) {
+        for (const wrk_matrix* m : matrices) constants.insert(constants.end(), {m->w, m->m, m->q});
+    }
+    void declare(wrk_op* op) const {
+        for (const wrk_tensor* t : constants) {
+            if (t == nullptr) continue;
+            op->keep.push_back(t->buf);
+            op->early.push_back(t->buf.get());
+        }
+        if (shift_state == nullptr) return;
+        op->keep.push_back(shift_state->buf);
+        op->shift_rows.push_back(shift_state->buf.get());
+    }
+};
+
 int32_t add_fused_gemv(wrk_context* ctx, OpList& ops, CachedJob* job, k::FusedGemvArgs a, const char* name,
-                       std::initializer_list<const wrk_tensor*> keep) {
+                       std::initializer_list<const wrk_tensor*> keep, const EarlyReads& early) {
     const int grid = ctx->num_sms;
     a.status = ctx->device_status;
     for (int i = 0; i < a.num_problems; ++i)
@@ -846,6 +867,7 @@ int32_t add_fused_gemv(wrk_context* ctx, OpList& ops, CachedJob* job, k::FusedGe
             return set_error(WRK_ERR_INVALID_ARGUMENT, "NF4 problem without a code book");
     WRK_TRY(make_partition(ctx, a, grid, job));
     ops.ops.push_back(new_atom(name, [a, grid](cudaStream_t s) { return k::fused_gemv(a, grid, s); }, keep));
+    early.declare(ops.ops.back());
     return WRK_OK;
 }
 
@@ -896,8 +918,8 @@ struct FusedSink {
     StepBuilder* step;  // null: one launch per phase
 };
 
-int32_t emit_gemv(FusedSink& sink, k::FusedGemvArgs a, const char* name, std::initializer_list<const wrk_tensor*> keep) {
-    if (sink.step == nullptr) return add_fused_gemv(sink.ctx, *sink.ops, sink.job, a, name, keep);
+int32_t emit_gemv(FusedSink& sink, k::FusedGemvArgs a, const char* name, std::initializer_list<const wrk_tensor*> keep, const EarlyReads& early) {
+    if (sink.step == nullptr) return add_fused_gemv(sink.ctx, *sink.ops, sink.job, a, name, keep, early);
     StepBuilder& sb = *sink.step;
     const int grid = sink.ctx->num_sms;
     a.status = sink.ctx->device_status;
@@ -966,9 +988,10 @@ int32_t layer_v6_fused(wrk_bundle* bd, FusedSink& sink, const Buffers& B, uint32
     const uint32_t* cursors = static_cast<const uint32_t*>(B["cursors"]->ptr());
     const int wide = bd->packed_cursors ? 0 : 1;
     const DView st_att = make_dview(state_att(bd, index, S)), st_ffn = make_dview(state_ffn(bd, index, S));
-    const float* table = nullptr;
+    const wrk_tensor* code_book = nullptr;
     for (wrk_matrix* m : {L.att_w_k.p, L.att_w_o.p, L.ffn_w_k.p})
-        if (m->q) table = static_cast<const float*>(m->q->ptr());
+        if (m->q) code_book = m->q;
+    const float* table = code_book ? static_cast<const float*>(code_book->ptr()) : nullptr;
 
     // A: layer norm + shift(time_mix_x) -> adapter W1 (tanh)
     {
@@ -990,7 +1013,8 @@ int32_t layer_v6_fused(wrk_bundle* bd, FusedSink& sink, const Buffers& B, uint32
         a.p[0] = problem(mat_info(L.time_mix_w1), nullptr, 0, B["time_mix_x"]->ptr(), WRK_F16, WRK_ACT_TANH);
         a.epilogue = k::EPI_STORE;
         a.rescale = 1.0f;
-        WRK_TRY(emit_gemv(sink, a, "fused_ln_shift_adapter", {B["x"], B["att_x"], B["time_mix_x"], L.time_mix_w1.p->w}));
+        WRK_TRY(emit_gemv(sink, a, "fused_ln_shift_adapter", {B["x"], B["att_x"], B["time_mix_x"]},
+                          EarlyReads({L.time_mix_w1.p}, {L.att_ln.w, L.att_ln.b, L.time_mix_x.p}, bd->state[index].p)));
     }
     // B: adapter W2 + static mixes + five-way token shift
     {
@@ -1014,7 +1038,8 @@ int32_t layer_v6_fused(wrk_bundle* bd, FusedSink& sink, const Buffers& B, uint32
             sink.step->phases.push_back(ph);
         } else {
             ops.ops.push_back(new_atom("fused_tmix_shift", [a](cudaStream_t s) { return k::tmix_shift_v6(a, s); },
-                                       {B["time_mix_x"], B["att_x"], B["att_sx"], L.time_mix_w2.p->w, L.time_mix.p}));
+                                       {B["time_mix_x"], B["att_x"], B["att_sx"]}));
+            EarlyReads({L.time_mix_w2.p}, {L.time_mix.p}, bd->state[index].p).declare(ops.ops.back());
         }
     }
     // C: key / value / receptance / gate + decay adapter W1 in one launch
@@ -1035,7 +1060,8 @@ int32_t layer_v6_fused(wrk_bundle* bd, FusedSink& sink, const Buffers& B, uint32
         a.epilogue = k::EPI_STORE;
         a.rescale = 1.0f;
         WRK_TRY(emit_gemv(sink, a, "fused_att_linear",
-                               {B["att_sx"], B["att_k"], B["att_v"], B["att_r"], B["att_g"], B["att_w"]}));
+                               {B["att_sx"], B["att_k"], B["att_v"], B["att_r"], B["att_g"], B["att_w"]},
+                               EarlyReads({L.att_w_k.p, L.att_w_v.p, L.att_w_r.p, L.att_w_g.p, L.time_decay_w1.p}, {code_book})));
     }
     // D: decay adapter W2 + WKV + group norm + gate
     {
@@ -1071,6 +1097,8 @@ int32_t layer_v6_fused(wrk_bundle* bd, FusedSink& sink, const Buffers& B, uint32
             ops.ops.push_back(new_atom("fused_wkv6", [a](cudaStream_t s) { return k::wkv56_fused(a, s); },
                                        {B["att_w"], B["att_k"], B["att_v"], B["att_r"], B["att_g"], B["att_x"], B["att_xx"],
                                         bd->state[index].p}));
+            EarlyReads({L.time_decay_w2.p}, {L.time_decay.p, L.time_first.p, L.gn.w.p, L.gn.b.p}).declare(ops.ops.back());
+            ops.ops.back()->early_state.push_back(bd->state[index].p->buf.get());
         }
     }
     // E: output projection + residual
@@ -1085,7 +1113,7 @@ int32_t layer_v6_fused(wrk_bundle* bd, FusedSink& sink, const Buffers& B, uint32
         a.epilogue = k::EPI_RESIDUAL;
         a.xres = Hm(B["x"]);
         a.rescale = 1.0f;
-        WRK_TRY(emit_gemv(sink, a, "fused_att_out", {B["att_xx"], B["x"]}));
+        WRK_TRY(emit_gemv(sink, a, "fused_att_out", {B["att_xx"], B["x"]}, EarlyReads({L.att_w_o.p}, {code_book})));
     }
     // F: layer norm + two shifts -> ffn key (squared ReLU) and receptance
     {
@@ -1110,7 +1138,8 @@ int32_t layer_v6_fused(wrk_bundle* bd, FusedSink& sink, const Buffers& B, uint32
         a.p[1] = problem(mat_info(L.ffn_w_r), nullptr, 1, B["ffn_r"]->ptr(), WRK_F16, WRK_ACT_NONE);
         a.epilogue = k::EPI_STORE;
         a.rescale = 1.0f;
-        WRK_TRY(emit_gemv(sink, a, "fused_ffn_in", {B["x"], B["ffn_x"], B["ffn_k"], B["ffn_r"]}));
+        WRK_TRY(emit_gemv(sink, a, "fused_ffn_in", {B["x"], B["ffn_x"], B["ffn_k"], B["ffn_r"]},
+                          EarlyReads({L.ffn_w_k.p, L.ffn_w_r.p}, {L.ffn_ln.w, L.ffn_ln.b, L.ffn_time_mix_k.p, L.ffn_time_mix_r.p, code_book}, bd->state[index].p)));
     }
     // G: ffn value + channel mix + residual (+ rescale)
     {
@@ -1129,7 +1158,7 @@ int32_t layer_v6_fused(wrk_bundle* bd, FusedSink& sink, const Buffers& B, uint32
         a.cm_x = H(B["ffn_x"]);
         a.cm_state = st_ffn;
         a.rescale = (index + 1) % bd->model->rescale == 0 ? 0.5f : 1.0f;
-        WRK_TRY(emit_gemv(sink, a, "fused_ffn_out", {B["ffn_k"], B["ffn_r"], B["ffn_x"], B["x"], bd->state[index].p}));
+        WRK_TRY(emit_gemv(sink, a, "fused_ffn_out", {B["ffn_k"], B["ffn_r"], B["ffn_x"], B["x"]}, EarlyReads({L.ffn_w_v.p}, {code_book}, bd->state[index].p)));
     }
     (void)F;
     return WRK_OK;
@@ -1162,7 +1191,7 @@ int32_t build_step_job(wrk_bundle* bd, CachedJob* job, OpList& ops) {
         a.num_problems = 0;
         a.epilogue = k::EPI_STORE;
         a.rescale = 1.0f;
-        WRK_TRY(emit_gemv(sink, a, "step_embed", {}));
+        WRK_TRY(emit_gemv(sink, a, "step_embed", {}, EarlyReads({})));
     }
     for (uint32_t i = 0; i < m->info.num_layer; ++i) WRK_TRY(layer_v6_fused(bd, sink, B, i, T));
     if (NH > 0) {
@@ -1180,7 +1209,7 @@ int32_t build_step_job(wrk_bundle* bd, CachedJob* job, OpList& ops) {
         a.p[0] = problem(mat_info(m->head_w), nullptr, 0, Hd["head_o"]->ptr(), WRK_F32, WRK_ACT_NONE);
         a.epilogue = k::EPI_STORE;
         a.rescale = 1.0f;
-        WRK_TRY(emit_gemv(sink, a, "step_head", {}));
+        WRK_TRY(emit_gemv(sink, a, "step_head", {}, EarlyReads({})));
     }
     auto upload = [&](const void* data, size_t bytes, wrk_tensor** out) -> int32_t {
         const uint32_t shape[4] = {(uint32_t)((bytes + 3) / 4), 1, 1, 1};
@@ -1358,7 +1387,7 @@ int32_t build_job(wrk_bundle* bd, const RnnInfo& info, CachedJob* job) {
         a.p[0] = problem(mat_info(m->head_w), nullptr, 0, Hd["head_o"]->ptr(), WRK_F32, WRK_ACT_NONE);
         a.epilogue = k::EPI_STORE;
         a.rescale = 1.0f;
-        WRK_TRY(add_fused_gemv(m->ctx, ops, job, a, "fused_head", {head_x, Hd["head_o"]}));
+        WRK_TRY(add_fused_gemv(m->ctx, ops, job, a, "fused_head", {head_x, Hd["head_o"]}, EarlyReads({m->head_w}, {m->head_ln.w, m->head_ln.b})));
     } else if (NH > 0 && m->shard.on()) {
         // every rank multiplies its slice of the vocabulary; the slices are gathered and put in order
         HOOK(PRE_HEAD);
