@@ -96,3 +96,39 @@ def test_more_pairs_than_raw_stages(wrk, ctx, kind, k, n):
     got, want = _run(wrk, ctx, kind, k, 500, n, turbo=True, seed=k + n)
     assert_close(got, want, f"{kind} {k} n={n}")
     assert ctx.device_status() == 0
+
+
+@pytest.mark.parametrize("graph", [False, True])
+@pytest.mark.parametrize("n", [4, 64])
+@pytest.mark.parametrize("kind", KINDS)
+def test_a_matmul_waits_for_earlier_ops_that_write_its_parts(wrk, ctx, kind, n, graph):
+    # bytes, scales and code book come from the list itself, from an op that is not the one in front of the matmul; the kernel
+    # between is short, so a matmul that fetched its weights at once would find the zeros that lay there
+    rng = np.random.default_rng(14)
+    K, M = 4096, 1024
+    t_w = ctx.from_numpy((rng.standard_normal((M, K), dtype=np.float32) * 0.02).astype(np.float16))
+    t_x = ctx.from_numpy(rng.standard_normal((n, K), dtype=np.float32).astype(np.float16))
+    small = [ctx.tensor(wrk.F32, [64]) for _ in range(2)]
+    y, want = ctx.tensor(wrk.F32, [M, n]), ctx.tensor(wrk.F32, [M, n])
+    if kind == "fp16":
+        w = ctx.tensor(wrk.F16, [K, M], zeros=True)
+        parts, write = [w], [wrk.blit(t_w, w)]
+        matmul = wrk.matmul_mat_fp16(w, t_x, y)
+        ctx.run(wrk.Matrix.fp16(t_w).matmul_op(t_x, want, turbo=True))
+    elif kind == "int8":
+        w, mm = ctx.tensor(wrk.U8, [K, M], zeros=True), ctx.tensor(wrk.F16, [2 * K * M // 128], zeros=True)
+        parts, write = [w, mm], [wrk.quantize_mat_int8(t_w, mm, w)]
+        matmul = wrk.matmul_mat_int8(w, mm, t_x, y)
+        ctx.run(wrk.Matrix.quant_u8(t_w).matmul_op(t_x, want, turbo=True))
+    else:
+        book, table = ctx.from_numpy(wrk.nf4_table()), ctx.from_numpy(wrk.nf4_table())
+        w, am = ctx.tensor(wrk.U8, [K // 2, M], zeros=True), ctx.tensor(wrk.F16, [K * M // 64], zeros=True)
+        parts, write = [w, am, table], [wrk.quantize_mat_nf4(t_w, book, am, w), wrk.blit(book, table)]
+        matmul = wrk.matmul_mat_nf4(w, table, am, t_x, y)
+        ctx.run(wrk.Matrix.quant_nf4(t_w).matmul_op(t_x, want, turbo=True))
+    commands = ctx.encode(wrk.op_list(write + [wrk.blit(*small), matmul]), use_graph=graph)
+    for _ in range(3):
+        for t in parts:
+            t.load(np.zeros_like(t.numpy()))
+        commands.submit()
+        assert np.array_equal(y.numpy(), want.numpy())
