@@ -1,8 +1,10 @@
 """The layout of a tensor-core launch (`wrk_matmul_plan`), over the sizes it may be asked for.  No GPU is touched."""
 import itertools
 
+import pytest
+
 FP16, INT8, NF4 = 0, 1, 2
-TOKENS = list(range(16, 272, 16)) + [9, 65, 1000]
+TOKENS = list(range(16, 272, 16)) + [17, 65, 1000]
 WIDTHS = [128 * b for b in (1, 2, 3, 4, 5, 6, 7, 8, 10, 12, 13, 16, 20, 21, 32, 40, 70, 112)]
 ROW_TILES = [1, 6, 16, 32, 80, 112, 512]
 
@@ -49,3 +51,10 @@ def test_ctas_that_wait_for_each_other_do_not_share_an_sm(wrk):
     # other waits for on the next, unless the SM's shared memory (228 KB, 1 KB of it the system's for each CTA) has room for one.
     for case, p in _plans(wrk, (FP16, INT8, NF4)):
         assert p["splits"] == 1 or 2 * (p["smem"] + 1024) > 228 * 1024, (case, p)
+
+
+def test_sizes_that_are_no_matmul_are_refused(wrk):
+    for bad in ((3, 256, 16, 1), (INT8, 100, 16, 1), (INT8, 256, 0, 1), (INT8, 256, 16, 0), (INT8, 256, 2 ** 32 - 1, 1)):
+        with pytest.raises(wrk.WrkError):
+            wrk.matmul_plan(*bad)
+    assert wrk.matmul_plan(INT8, 4096, 2 ** 24, 2 ** 24)["splits"] == 1  # no product of them wraps

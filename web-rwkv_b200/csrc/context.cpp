@@ -480,11 +480,11 @@ static std::vector<char> chain_of(const std::vector<wrk_op*>& atoms) {
     std::unordered_set<const Buffer*> touched;
     for (size_t i = 0; i < atoms.size(); ++i) {
         const wrk_op& a = *atoms[i];
-        auto free = [&](const std::vector<const Buffer*>& early) {
+        auto untouched = [&](const std::vector<const Buffer*>& early) {
             return std::none_of(early.begin(), early.end(), [&](const Buffer* b) { return touched.count(b) != 0; });
         };
         auto in = [](const std::vector<const Buffer*>& list, const Buffer* b) { return std::find(list.begin(), list.end(), b) != list.end(); };
-        chained[i] = i > 0 && free(a.early) && free(a.early_state);
+        chained[i] = i > 0 && untouched(a.early) && untouched(a.early_state);
         for (const auto& b : a.keep)
             if (!in(a.early, b.get()) && !in(a.shift_rows, b.get())) touched.insert(b.get());
     }

@@ -708,8 +708,8 @@ UmmaPlan umma_plan(int kind, uint32_t K, uint32_t N, uint32_t row_tiles, uint32_
     const bool quantized = kind != MAT_FP16;
     const uint32_t nk = K / BK;
     auto splits_for = [&](uint32_t n_tile) {
-        const uint32_t tiles = row_tiles * ((N + n_tile - 1) / n_tile);
-        uint32_t want = std::max<uint32_t>(1, num_sms / tiles);
+        const uint64_t tiles = (uint64_t)row_tiles * ((N + n_tile - 1) / n_tile);
+        uint32_t want = std::max<uint32_t>(1, (uint32_t)(num_sms / tiles));
         want = std::min<uint32_t>(want, std::max<uint32_t>(1, nk / 8));
         want = std::min<uint32_t>(want, 8);
         while (nk % 4 == 0 && nk % (4 * want) != 0) --want;  // equal shares where K allows them

@@ -152,7 +152,7 @@ int32_t stream_op(const char* name, wrk_context* ctx, const k::MatmulArgs* args,
 bool overlap(const wrk_view& a, const wrk_view& b) {
     if (a.tensor->buf != b.tensor->buf) return false;
     for (int i = 0; i < 4; ++i)
-        if (a.stride[i] != b.stride[i]) return true;
+        if (a.stride[i] != b.stride[i] || (uint64_t)a.offset[i] + a.shape[i] > a.stride[i] || (uint64_t)b.offset[i] + b.shape[i] > b.stride[i]) return true;
     for (int i = 0; i < 4; ++i)
         if (a.offset[i] + a.shape[i] <= b.offset[i] || b.offset[i] + b.shape[i] <= a.offset[i]) return false;
     return true;
@@ -1199,7 +1199,8 @@ int32_t wrk_matrix_matmul_op_sparse(wrk_matrix* m, const wrk_view* input, const 
 
 int32_t wrk_matmul_plan(int32_t kind, uint32_t k, uint32_t n, uint32_t row_tiles, uint32_t num_sms, uint32_t plan[10]) {
     REQ_NN(plan);
-    WRK_REQUIRE(kind >= 0 && kind <= 2 && k >= 128 && k % 128 == 0 && n > 0 && row_tiles > 0 && num_sms > 0, WRK_ERR_INVALID_ARGUMENT,
+    const uint32_t most = 1u << 24;
+    WRK_REQUIRE(kind >= 0 && kind <= 2 && k >= 128 && k % 128 == 0 && n > 0 && n <= most && row_tiles > 0 && row_tiles <= most && num_sms > 0, WRK_ERR_INVALID_ARGUMENT,
                 "no such matmul: kind %d, k = %u, n = %u, %u row tiles, %u SMs", kind, k, n, row_tiles, num_sms);
     const k::UmmaPlan p = k::umma_plan(kind == 0 ? k::MAT_FP16 : kind == 1 ? k::MAT_INT8 : k::MAT_NF4, k, n, row_tiles, num_sms);
     const uint32_t values[10] = {p.n_tile, p.splits, p.walk, p.bu, p.acc_cols, p.tmem_cols, p.a_stages, p.b_stages, p.raw, p.smem};
