@@ -67,8 +67,8 @@ def test_activation_view_with_row_stride(wrk, ctx):
 @pytest.mark.parametrize("kind", KINDS)
 @pytest.mark.parametrize("k,m,n", [(128, 128, 9), (384, 200, 15), (2688, 768, 33), (8064, 100, 17), (1152, 130, 250), (640, 129, 512)])
 def test_odd_numbers_of_k_blocks_and_few_tokens(wrk, ctx, kind, k, m, n):
-    # 1, 3, 21, 63, 9, 5 blocks of 128: the two dequantizing groups get unequal shares, K splits into unequal parts (4 CTAs of
-    # 5 or 6 blocks, 8 of 7 or 8), fewer blocks than ring stages; 9 tokens are the fewest the kernel takes
+    # 1, 3, 21, 63, 9, 5 blocks of 128: quantized rows of these widths, and 9 or 15 tokens, are with the mma.sync kernel; fp16 from
+    # 17 tokens on splits K into unequal parts (4 CTAs of 5 or 6 blocks, 8 of 7 or 8) and has fewer steps than ring stages
     got, want = _run(wrk, ctx, kind, k, m, n, turbo=True, seed=k + n)
     assert_close(got, want, f"{kind} {k}x{m} n={n}")
     assert ctx.device_status() == 0

@@ -234,6 +234,54 @@ def test_time_first_v7(wrk, ctx, dtype):
     assert_close(t_x.numpy().reshape(T, H, S), ref, "time_first", max_abs=5e-2 if dtype == np.float16 else 2e-2)
 
 
+def _float64_run(r, k, v, w, u=None, sa_in=None, sa_out=None, state=None):
+    """The recurrences in float64.  [T, H, S] operands, state [H, S keys, S values]; v6 with the bonus u, v7 with the vectors
+    whose outer product the state is also multiplied by."""
+    out = []
+    for t in range(r.shape[0]):
+        kv = k[t][:, :, None] * v[t][:, None, :]
+        if u is not None:
+            out.append(np.einsum("hi,hij->hj", r[t], state + u[:, :, None] * kv))
+            state = state * w[t][:, :, None] + kv
+        else:
+            sa = np.einsum("hij,hi->hj", state, sa_in[t])
+            state = state * w[t][:, :, None] + kv + sa_out[t][:, :, None] * sa[:, None, :]
+            out.append(np.einsum("hi,hij->hj", r[t], state))
+    return np.stack(out), state
+
+
+@pytest.mark.parametrize("T", [8, 100])
+@pytest.mark.parametrize("form", ["v6", "blocks", "v7"])
+def test_recurrences_against_float64(wrk, ctx, form, T):
+    """f32 operands, state and sums: outputs and state stay within 2^-22 (a rounding of a result is up to 2^-24; sums of 64
+    products of alternating sign measured 1.0e-7).  Nothing on the way may be held in fewer bits."""
+    rng = np.random.default_rng(T)
+    H, C = 4, 4 * S
+    cursors, _ = _cursors([(0, T)], True)
+    rand = lambda *shape: rng.standard_normal(shape).astype(np.float32)
+    state = rand(1, S + 2, C) * np.float32(0.1)
+    r, k, v, x = rand(T, H, S), rand(T, H, S), rand(T, H, S), rand(T, H, S)
+    start = state[0, 1:S + 1].reshape(S, H, S).swapaxes(0, 1).astype(np.float64)
+    t_state, t_x = ctx.from_numpy(state), ctx.from_numpy(x)
+    rows = t_state.view(y=(0, S + 1))
+    wide = [a.astype(np.float64) for a in (r, k, v)]
+    if form == "v7":
+        w, kk, a = rand(T, H, S), rand(T, H, S), rng.uniform(0, 1, (T, H, S)).astype(np.float32)
+        kk /= np.linalg.norm(kk, axis=-1, keepdims=True)
+        ctx.run(wrk.time_mix_v7(ctx.from_numpy(cursors), rows, ctx.from_numpy(r), ctx.from_numpy(w), ctx.from_numpy(np.stack([k, v, a, kk])), t_x))
+        decay = np.exp(-0.606531 / (1.0 + np.exp(-w.astype(np.float64))))
+        want, end = _float64_run(*wide, decay, sa_in=-kk.astype(np.float64), sa_out=kk.astype(np.float64) * a, state=start)
+    else:
+        u = rng.uniform(-1, 1, (H, S)).astype(np.float32)
+        w = np.exp(-np.exp(rng.uniform(-6, 1, (T, H, S)))).astype(np.float32)
+        args = [ctx.from_numpy(a) for a in (cursors, w, u)] + [rows] + [ctx.from_numpy(a) for a in (k, v, r)] + [t_x]
+        ctx.run(wrk.time_mix_blocks(True, *args) if form == "blocks" else wrk.time_mix_v6(*args))
+        want, end = _float64_run(*wide, w.astype(np.float64), u=u.astype(np.float64), state=start)
+    got_end = t_state.numpy().reshape(S + 2, C)[1:S + 1].reshape(S, H, S).swapaxes(0, 1)
+    for got, ref in ((t_x.numpy().reshape(T, H, S), want), (got_end, end)):
+        assert np.linalg.norm(got - ref) <= 2.0 ** -22 * np.linalg.norm(ref)
+
+
 def test_shape_errors(wrk, ctx):
     H, T = 2, 3
     f = lambda *s: ctx.tensor(wrk.F32, list(s))

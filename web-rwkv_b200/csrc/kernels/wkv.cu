@@ -234,14 +234,15 @@ __global__ void __launch_bounds__((S / 4) * (NC / 4)) time_mix_v56_kernel(const 
 // Every product of decays is taken forwards (no division, nothing can overflow; what underflows is a contribution that
 // has decayed to nothing).  The work of a block is then three small matrix products - [16 x 64][64 x 64] for the state's
 // share of y, [16 x 16][16 x 64] for the block's own tokens and [64 x 16][16 x 64] for the new state - in which no
-// element waits for another: 4 x 4 register tiles in fp32 on the CUDA cores, operands from shared memory.  The serial
-// kernel above spends about 650 cycles on a token's chain of dependent steps; this one about 130 per token.
+// element waits for another: 4 x 4 register tiles in fp32 on the CUDA cores, operands from shared memory.
 // Two CTAs of 256 threads per (head of 64 channels, batch slot), each with 32 of the state's columns, which do not depend on one
 // another (both form A and the decay products); the state tile of a thread stays in registers from block to block; the
 // tokens' rows are staged a block ahead as in the serial kernel.  Every element is summed in the order that one CTA per head
-// took, so its bits are the same.  256 tokens of 64 heads: 76 -> 68 us, and 53 with the loads of a block in flight together.
-// The serial kernel above is faster (35 us), but it sums in another order, and what that changes in the last bit of a
-// state grows through the layers of a deep model (24 layers of random weights: to 1e-2 of the last layer's state).
+// took, so its bits are the same.  256 tokens of 64 heads: 76 -> 68 us, and 53 (0.21 per token) with the loads of a block in flight
+// together.  The serial kernel above has become the faster one (35 us, 0.14 per token); it sums in another order, and what that
+// changes in the last bit of a state grows through the layers of a deep model (24 layers of random weights: to 1e-2 of the last
+// layer's state).  It is also no further from float64 (256 tokens: outputs 8.8e-8 against 9.5e-8 here, states 5.3e-8 against
+// 5.9e-8); jobs of more than 8 tokens have not been moved to it.
 constexpr int kBlockTokens = 16;
 constexpr int kQtStride = 20;  // row stride of Qt in floats: 16-byte rows whose vector stores do not collide
 constexpr int kBlockCols = 32;  // columns of a CTA
