@@ -20,7 +20,8 @@
 // through distributed shared memory.
 // Weights enter the MMA as fp16(fma(q, (max - min) / 255, min)) resp. fp16(table[nib] * absmax), computed in
 // f32 and rounded once; the accumulation is fp32.  Every wait on an mbarrier is bounded: on a timeout the
-// kernel records WRK_ERR_TIMEOUT in the context's status word, stops waiting and still frees its TMEM.  A wait whose end
+// kernel records WRK_ERR_TIMEOUT in the context's status word, stops waiting and copying, lets the copies and MMAs in flight
+// end (with a limit again) and still frees its TMEM.  A wait whose end
 // depends on the activations comes after griddepcontrol.wait: the limit does not count the kernels in front.
 //
 // What bounds it: at 256 tokens a step is 512 cycles of MMA; it takes about 850, most of it shared-memory and L2 traffic of the
@@ -53,6 +54,7 @@ constexpr int kMaxRaw = 8;          // raw weight stages
 constexpr uint32_t kScaleSlots = 8, kScaleAhead = 6;
 constexpr uint32_t SCALE_BYTES = 2 * kScaleSlots * BM * 4;  // two groups of dequantizing warps
 constexpr uint32_t kSpinLimit = 1u << 22;
+constexpr uint32_t kDrainLimit = 1u << 16;
 constexpr uint32_t kSplitSmem = 114 * 1024;  // half of the 228 KB of an SM; 1 KB more per CTA is the system's
 constexpr uint32_t A_STEP_BYTES = BM * BK * 2;  // fp16 weights: 16 KB of shared memory per step
 constexpr uint32_t A_STEP_COLS = BK / 2;        // quantized weights: 32 TMEM columns of fp16 pairs per step
@@ -166,16 +168,17 @@ __device__ __forceinline__ bool mbar_try(uint64_t* bar, uint32_t parity) {
         : "memory");
     return ok != 0;
 }
-// Waits for it; gives up after kSpinLimit polls (or at once when another wait of this CTA has already given up) and
+// Waits for it; gives up (false) after kSpinLimit polls (or at once when another wait of this CTA has already given up) and
 // reports it.
-__device__ __forceinline__ void mbar_wait(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int32_t* status) {
+__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int32_t* status) {
 #pragma unroll 1
     for (uint32_t i = 0; i < kSpinLimit; ++i) {
-        if (mbar_try(bar, parity)) return;
-        if (*abort_flag) return;
+        if (mbar_try(bar, parity)) return true;
+        if (*abort_flag) return false;
     }
     *abort_flag = 1;
     if (status != nullptr) atomicExch(status, (int32_t)WRK_ERR_TIMEOUT);
+    return false;
 }
 
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory"); }
@@ -359,6 +362,7 @@ matmul_umma_kernel(const __grid_constant__ UmmaGroup grp) {
         tma_load_3d(w_base + stage * bu * A_STEP_BYTES, &map_w, 0, m0, (u_begin + u) * bu, &b_full[stage]);
     };
     const uint32_t ahead = min(nu, quantized ? n_raw : b_stages);
+    uint32_t copies = 0;  // of a TMA thread: issued so far, in the order of its ring
     if (warp == kWeightTmaWarp) {
         if (elect_one()) {
             if (quantized) {
@@ -375,6 +379,7 @@ matmul_umma_kernel(const __grid_constant__ UmmaGroup grp) {
                 if (quantized) load_raw(u, u);
                 else load_weights(u, u);
             }
+            copies = ahead;
         }
         __syncwarp();
     } else if (warp == kMmaWarp) {
@@ -557,14 +562,15 @@ matmul_umma_kernel(const __grid_constant__ UmmaGroup grp) {
                 // a stage that is free only after an MMA: the pair before it in the ring has found no A stage unused
                 if (u - ahead == (quantized ? a_stages : 0)) pdl_wait();
                 if (quantized) {
-                    mbar_wait(&raw_empty[ring.stage], ring.phase ^ 1, &abort_flag, status);
+                    if (!mbar_wait(&raw_empty[ring.stage], ring.phase ^ 1, &abort_flag, status)) break;
                     load_raw(u, ring.stage);
                     ring.next(n_raw);
                 } else {
-                    mbar_wait(&b_empty[ring.stage], ring.phase ^ 1, &abort_flag, status);
+                    if (!mbar_wait(&b_empty[ring.stage], ring.phase ^ 1, &abort_flag, status)) break;
                     load_weights(u, ring.stage);
                     ring.next(b_stages);
                 }
+                copies = u + 1;
             }
         }
         __syncwarp();
@@ -575,13 +581,17 @@ matmul_umma_kernel(const __grid_constant__ UmmaGroup grp) {
 #pragma unroll 1
             for (uint32_t u = 0; u < nu; ++u) {
                 const uint32_t first = (u_begin + u) * unit;
+                bool ok = true;
 #pragma unroll 1
                 for (uint32_t d = 0; d < unit; d += bu) {
-                    mbar_wait(&b_empty[ring.stage], ring.phase ^ 1, &abort_flag, status);
+                    ok = mbar_wait(&b_empty[ring.stage], ring.phase ^ 1, &abort_flag, status);
+                    if (!ok) break;
                     mbar_expect_tx(&b_full[ring.stage], b_bytes);
                     tma_load_3d(b_base + ring.stage * b_bytes, &map_x, 0, n0, first + d, &b_full[ring.stage]);
                     ring.next(b_stages);
+                    ++copies;
                 }
+                if (!ok) break;
             }
         }
         __syncwarp();
@@ -589,7 +599,23 @@ matmul_umma_kernel(const __grid_constant__ UmmaGroup grp) {
     tc_fence_before();
     if (splits > 1) cluster_sync();  // a hardware barrier that every thread reaches, also after a wait above has given up
     else __syncthreads();
+    if (copies != 0 && abort_flag != 0) {  // nobody has waited for the last copies: a thread of this CTA stays until they have landed
+        const bool packed = quantized && warp == kWeightTmaWarp;
+        uint64_t* const full = packed ? raw_full : b_full;
+        const uint32_t stages = packed ? n_raw : b_stages;
+#pragma unroll 1
+        for (uint32_t j = copies - min(copies, stages); j < copies; ++j)
+#pragma unroll 1
+            for (uint32_t i = 0; i < kDrainLimit && !mbar_try(&full[j % stages], j / stages & 1); ++i) {
+            }
+    }
     if (warp == kMmaWarp) {
+        if (abort_flag != 0) {  // nor for the last MMAs
+#pragma unroll 1
+            for (uint32_t i = 0; i < kDrainLimit && !mbar_try(&done_bar, 0); ++i) {
+            }
+            __syncwarp();
+        }
         tc_fence_after();
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem_d), "r"(grp.tmem_cols) : "memory");
     }
